@@ -46,6 +46,7 @@ SIGNATURES = {
 
 _lock = threading.Lock()
 _lib = None
+_binding = None
 
 
 class NvllmError(RuntimeError):
@@ -70,6 +71,18 @@ def load() -> ctypes.CDLL:
                 fn.argtypes = args
             _lib = lib
     return _lib
+
+
+def binding():
+    """The native host path of the torch operators (csrc/torch_binding.cpp), bound to the loaded library."""
+    global _binding
+    if _binding is None:
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        lib = load()
+        from . import _torch_binding
+        _torch_binding.bind({name: _c.cast(getattr(lib, name), _vp).value for name in SIGNATURES}, check)
+        _binding = _torch_binding
+    return _binding
 
 
 def check(code: int) -> None:

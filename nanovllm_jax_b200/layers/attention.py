@@ -27,7 +27,7 @@ from typing import NamedTuple
 
 import torch
 
-from .. import ops
+from .. import _lib, ops
 from ..utils.context import AttentionContext
 
 # The reference exports this flag from its Pallas module (layers/attention.py:21-28); callers test it before
@@ -121,9 +121,9 @@ class Attention:
         if not context.is_prefill and self.k_cache is not None and self.v_cache is not None:
             # decode: the scatter of the step's K/V rows and the attention over the pages go down as one C call
             # (same result as the two calls of the reference, :465-467 then :476-478)
-            return ops.decode_step(q.to(self.k_cache.dtype).contiguous(), k.contiguous(), v.contiguous(),
-                                   self.k_cache, self.v_cache, context.slot_mapping, context.block_tables,
-                                   context.context_lens, self.scale, self.block_size)
+            return _lib.binding().decode_step(q, k, v, self.k_cache, self.v_cache, context.slot_mapping,
+                                              context.block_tables, context.context_lens, self.scale, self.block_size,
+                                              None, True)
         if self.k_cache is not None and self.v_cache is not None:
             num_blocks = self.k_cache.shape[0]
             flat = (num_blocks * self.block_size, self.num_kv_heads, self.head_dim)

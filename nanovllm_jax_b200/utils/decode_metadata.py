@@ -24,6 +24,7 @@ from typing import Sequence
 import numpy as np
 import torch
 
+from .. import _lib
 from .context import AttentionContext, create_decode_context
 from .staging import packed_like
 
@@ -36,16 +37,19 @@ def compiled_batch_sizes(max_num_seqs: int) -> list[int]:
 
 def bucket_batch(n: int, max_num_seqs: int) -> int:
     """Smallest compiled batch size >= n (n itself beyond the list: the reference would compile it on the fly)."""
-    for b in compiled_batch_sizes(max_num_seqs):
-        if b >= n:
-            return b
-    return n
+    largest = min(max(int(max_num_seqs), 1), 512)
+    b = next((b for b in (1, 2, 4, 8) if b >= n), -(-n // 16) * 16)
+    return b if b <= (largest if largest < 16 else largest // 16 * 16) else n
 
 
 def bucket_blocks(n: int, min_blocks: int = 1) -> int:
     """Block-table width rounded up to a power of two."""
     n = max(int(n), min_blocks, 1)
     return 1 << (n - 1).bit_length()
+
+
+def _int_list(x):
+    return x if type(x) in (list, tuple) else np.asarray(x, dtype=np.int32).tolist()
 
 
 class DecodeMetadata:
@@ -68,6 +72,7 @@ class DecodeMetadata:
         self._dev_flat, dv = packed_like(like, self.device)
         self.h_ids, self.h_pos, self.h_slots, self.h_ctx, self.h_tables = hv
         self.input_ids, self.positions, self.slot_mapping, self.context_lens, self.block_tables = dv
+        self._host_ptrs = [t.data_ptr() for t in hv]
         self._host_flat.zero_()
         self.h_slots.fill_(-1)
         self.h_tables.fill_(-1)
@@ -80,30 +85,20 @@ class DecodeMetadata:
                context_lens: Sequence[int], block_tables: Sequence[Sequence[int]], max_num_seqs: int | None = None):
         """One step's metadata, as engine/model_runner.py:340-374 computes it, into the fixed buffers.
         Returns (padded_batch, width): the bucket a captured step is keyed by."""
+        lists = [_int_list(x) for x in (input_ids, positions, slot_mapping, context_lens)]
+        tables = [_int_list(t) for t in block_tables]
         n = len(input_ids)
         if not (len(positions) == len(slot_mapping) == len(context_lens) == len(block_tables) == n):
             raise ValueError("per-sequence lists differ in length")
         if n > self.max_batch:
             raise ValueError(f"{n} sequences exceed the buffers' {self.max_batch}")
-        longest = max((len(t) for t in block_tables), default=1)
+        longest = max(map(len, tables), default=1)
         if longest > self.max_blocks:
             raise ValueError(f"a block table of {longest} pages exceeds the buffers' {self.max_blocks}")
         nb = min(bucket_batch(max(n, 1), max_num_seqs if max_num_seqs is not None else self.max_batch), self.max_batch)
         nb = max(nb, n)
-        self.h_ids[:n] = torch.as_tensor(np.asarray(input_ids, dtype=np.int32))
-        self.h_pos[:n] = torch.as_tensor(np.asarray(positions, dtype=np.int32))
-        self.h_slots[:n] = torch.as_tensor(np.asarray(slot_mapping, dtype=np.int32))
-        self.h_ctx[:n] = torch.as_tensor(np.asarray(context_lens, dtype=np.int32))
         # rows that were live in an earlier, larger batch become padding again
-        hi = max(self.padded_batch, nb)
-        self.h_ids[n:hi] = 0
-        self.h_pos[n:hi] = 0
-        self.h_slots[n:hi] = -1
-        self.h_ctx[n:hi] = 0
-        self.h_tables[:hi].fill_(-1)
-        for i, t in enumerate(block_tables):
-            if len(t):
-                self.h_tables[i, :len(t)] = torch.as_tensor(np.asarray(t, dtype=np.int32))
+        _lib.binding().fill_decode_metadata(*lists, tables, *self._host_ptrs, self.max_blocks, max(self.padded_batch, nb))
         self._dev_flat.copy_(self._host_flat, non_blocking=True)  # the step's single host -> device copy
         self.batch, self.padded_batch, self.width = n, nb, bucket_blocks(longest)
         return nb, self.width
