@@ -7,32 +7,41 @@
 //
 //  * Work unit = one 64-token tile of one (sequence, kv head).  All tiles of
 //    one kv head are laid end to end (sequence after sequence) and cut into
-//    `num_groups` contiguous ranges of equal COST ("stream-K" partition): a tile
-//    costs one unit and every sequence four more in front of its tiles (the
+//    `num_groups` contiguous chunks of equal COST ("stream-K" partition): a tile
+//    costs one unit and every sequence three more in front of its tiles (the
 //    time a CTA loses at a sequence boundary -- q load, page lookup, the
-//    cross-warp combine, and the partial results at the ends of a range).  So every CTA
+//    cross-warp combine, and the partial results at the ends of a chunk).  So every CTA
 //    finishes at the same time no matter how skewed the context lengths are or
-//    how many short sequences fall into its range.  CTA c serves kv head c % KVH of group c / KVH; the KVH CTAs of a
-//    group walk the same tokens at the same pace, so the 256-byte per-head rows
-//    they fetch are neighbours in DRAM.
+//    how many short sequences fall into its chunk.  CTA c serves kv head c % KVH of chunk c / KVH; the KVH CTAs of a
+//    chunk walk the same tokens at the same pace, so the 256-byte per-head rows
+//    they fetch are neighbours in DRAM.  Small batches use fewer, longer chunks (make_cut).
 //  * Persistent CTAs, 2 per SM: one producer warp issues TMA tile loads
-//    (cp.async.bulk.tensor, 128-byte swizzle, no multicast) into a 3-stage
-//    mbarrier ring and runs ahead across sequence boundaries; four consumer
-//    warps each own 16 tokens of a tile.
-//  * The G = H/KVH query heads that share a kv head are packed into the 16-row
-//    M dimension of mma.sync.m16n8k16 (bf16 in, fp32 accumulate) for both
-//    q.K^T and P.V; the online softmax (exp2 domain) lives in registers with
-//    warp-shuffle row reductions.
-//  * A range that ends inside a sequence leaves an fp32 partial (m, l, O) in
+//    (cp.async.bulk.tensor, 128-byte swizzle, no multicast, one load per 16 KB tile) into a ring of two
+//    or three stages (ring_stages) and runs ahead across sequence boundaries; what a tile is (live tokens, first or last
+//    of its sequence, where its result goes) travels beside it in the ring, so only the producer walks the
+//    sequences.  Four consumer warps each own 16 tokens of a tile.
+//  * The G = H/KVH query heads that share a kv head are the 8 columns of
+//    mma.sync.m16n8k16 (bf16 in, fp32 accumulate), tokens and dims its 16 rows: S^T = K Q^T, O^T += V^T P^T (the heads as
+//    half-empty rows took twice the instructions and cost 3-5 % of the whole kernel).  The online softmax (exp2
+//    domain) lives in registers; the running maximum may be stale by 2^8, so the lanes vote on it instead of
+//    reducing it for every tile.
+//  * A chunk that ends inside a sequence leaves an fp32 partial (m, l, O) in
 //    the caller's workspace and takes a ticket for that (sequence, kv head); the
 //    CTA that draws the last ticket combines all partials of the sequence, in
-//    group order (bitwise reproducible whichever CTA arrives last), and writes
+//    chunk order (bitwise reproducible whichever CTA arrives last), and writes
 //    the rows -- all G rows at once, every load of a batch of four partials in
 //    flight together, so the combine costs about one round trip to L2 per four
-//    partials.  Nobody waits for another CTA.  Sequences wholly inside one range are
+//    partials.  Nobody waits for another CTA.  Sequences wholly inside one chunk are
 //    written directly.  The tickets are cleared by the small kernel that runs
 //    before this one (decode_prepare_kernel, which in the fused decode step
 //    also scatters the step's new K/V rows into the cache).
+//  * The first tiles are requested before that kernel has finished, unless they hold a slot that it writes.
+//
+// Measured on a B200 (per call, CUDA-graph replay, before -> after the transposed products, the two-stage ring, the
+// early requests and the native walk): one sequence of 300 tokens, 16 / 8 heads, 12.6 -> 7.3 us; Qwen3-8B shapes, batch
+// 64, 1.14 GB: 177 -> 163 us (7.0 TB/s); Qwen3-32B shapes, batch 256, 4.51 GB: 668 -> 621 us (7.26 TB/s).  What bounds it:
+// the stream itself runs at about 7.25 TB/s (a build without the math is not faster); about 3.5 us pass before the first
+// tile is under way and 3.5 us after the last one has landed.
 //
 // No spin-wait is unbounded: every mbarrier wait gives up after a poll limit,
 // raises a device error flag (readable through nvllm_b200_device_status) and
@@ -52,18 +61,22 @@ constexpr int kD = 128;                        // head_dim
 constexpr int kConsumerWarps = 4;
 constexpr int kWarps = kConsumerWarps + 1;     // consumers, TMA producer
 constexpr int kThreads = kWarps * 32;
-constexpr int kStages = 3;
+constexpr int kStages = 3;                     // ring stages; long streams use two of them (see ring_stages)
 constexpr int kMaxG = 8;                       // query heads per kv head packed in one CTA
-constexpr int kItemCostDefault = 4;            // cost of a sequence boundary in tile units (stream-K weights)
+constexpr int kItemCostDefault = 3;            // cost of a sequence boundary in tile units (stream-K weights)
 constexpr int kPanelBytes = kTile * 128;       // 64 tokens x 64 dims bf16, 128B-swizzled
 constexpr int kTileBytes = 2 * kPanelBytes;    // one K or V tile
 constexpr int kQBytes = kMaxG * kD * 2;        // 2 KiB
 constexpr int kStageBytes = 2 * kTileBytes + kQBytes;  // 34816
-constexpr int kOsStride = kD + 8;              // padded row of the cross-warp merge buffers (bank spread)
-constexpr int kOsBytes = 2 * kMaxG * kOsStride * 4;  // two buffers [8][136] fp32
-constexpr int kMiscBytes = 1024;
-constexpr int kSmemBytes = kStages * kStageBytes + kOsBytes + kMiscBytes + 1024;  // + alignment slack
+constexpr int kOsStride = kD + 4;              // padded row of the cross-warp merge buffers (bank spread)
+constexpr int kOsBytes = 2 * kMaxG * kOsStride * 4;  // two buffers [8][132] fp32
+constexpr int kMiscBytes = 768 + kThreads * 8;
+constexpr int kSmemBytes = kStages * kStageBytes + kOsBytes + kMiscBytes;
+static_assert(kSmemBytes + 1024 <= 228 * 1024 / 2, "two CTAs per SM");
 constexpr int kCtasPerSm = 2;
+constexpr float kStale = 8.f;                  // log2 units by which scores may exceed the running maximum
+constexpr int kMergeBatch = 4;                 // partial results the combine has in flight
+constexpr int kEarlySlots = 8;                 // slots per producer lane: batches up to 256 request tiles ahead of the wait
 
 // Per-partial record in the workspace: O[G][128] fp32, then m[8], l[8].
 __host__ __device__ inline size_t partial_floats(int G) { return (size_t)G * kD + 2 * kMaxG; }
@@ -74,8 +87,10 @@ struct Params {
     const __nv_bfloat16* q;
     const int32_t* block_tables;
     const int32_t* context_lens;
+    const int32_t* slot_mapping;  // [B] slots that the kernel just before this one writes, or null: it writes none
+    int q_in_flight;              // that kernel writes q too
     __nv_bfloat16* out;
-    float* partials;        // [grid][2][partial_floats]
+    float* partials;        // [chunks][KVH][2][partial_floats]
     unsigned int* tickets;  // [B*KVH] partials delivered so far per (sequence, kv head); zero when the kernel starts
     int B, H, KVH, G, NB, block_size, MB;
     int num_groups;
@@ -86,44 +101,88 @@ struct Params {
 __device__ __forceinline__ int clamp_ctx(int c, int max_ctx) { return c < 0 ? 0 : (c > max_ctx ? max_ctx : c); }
 __device__ __forceinline__ int tiles_of(int ctx) { return (ctx + kTile - 1) / kTile; }
 
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
 }
-__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(addr));
 }
-// D(16x8,f32) += A(16x16,bf16,row) * B(16x8,bf16,col); rows 8..15 of A are zero here.
-__device__ __forceinline__ void mma_lo(float (&c)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-    const uint32_t z = 0u;
+// D(16x8,f32) += A(16x16,bf16,row) * B(16x8,bf16,col)
+__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(z), "r"(a2), "r"(z), "r"(b0), "r"(b1));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
 }
 
+// ------------------------------------------------------------------------------------------
+// the cut of the work
+// ------------------------------------------------------------------------------------------
 // The cost line: sequence b with tb > 0 tiles occupies tb + item_cost units, the first item_cost of them standing
 // for its boundary overhead, the rest for its tiles 0 .. tb-1; empty sequences occupy nothing.
 __device__ __forceinline__ int units_of(int tb, int item_cost) { return tb > 0 ? tb + item_cost : 0; }
 
+// The line of one kv head (`total` units) is cut into `groups` contiguous chunks, one per CTA: the first `rem` of
+// `len + 1` units, the others of `len`.  The cut depends on the lengths alone: the results are bitwise reproducible.
+// (Handing the last eighth of the line out dynamically in ever smaller chunks was measured: the CTAs then finish
+// together, but at the same time as before -- the stream is bound by DRAM, not by its slowest CTA -- and the many small
+// partial results of a long sequence cost up to 15 us to combine.)
+struct Cut {
+    int groups;
+    long long len, rem;
+
+    __device__ __forceinline__ long long bound(int chunk) const { return chunk * len + (chunk < rem ? chunk : rem); }
+    // chunk that holds unit u
+    __device__ __forceinline__ int chunk_of(long long u) const {
+        const long long head = rem * (len + 1);
+        return u < head ? (int)div(u, len + 1) : (int)(rem + div(u - head, len));
+    }
+    // 64-bit divisions are slow and only lines of more than 2^31 units need them
+    static __device__ __forceinline__ long long div(long long a, long long b) {
+        return ((a | b) >> 31) == 0 ? (long long)((uint32_t)a / (uint32_t)b) : a / b;
+    }
+};
+
+// Less than kMinChunk units per CTA: chunks of kMinChunk units and fewer CTAs.  Five tiles take about as long as splitting
+// them further would cost (partial, ticket, combine: 2.5 us).
+constexpr int kMinChunk = 5;
+__device__ __forceinline__ Cut make_cut(long long total, int num_groups) {
+    Cut c;
+    c.groups = num_groups;
+    if (total < (long long)kMinChunk * num_groups) c.groups = max(1, (int)total / kMinChunk);
+    c.len = Cut::div(total, c.groups);
+    c.rem = total - c.len * c.groups;
+    return c;
+}
+
+// Stages of the ring in use.  A short chunk wants its first tiles requested at once; a long stream is faster with less in
+// flight: 128 KB per SM keep DRAM busy, and with 192 KB the requests of all SMs get in each other's way (Qwen3-32B
+// shapes, batch 256: 664 us with three stages, 640 with two).
+__device__ __forceinline__ uint32_t ring_stages(const Cut& cut) { return cut.len > 16 ? 2u : 3u; }
+
 struct Walk {
     int b;             // next sequence to look at
     long long fv;      // unit at which sequence b starts
-    long long x0, x1;  // this CTA's range of units
+    long long x0, x1;  // the chunk's range of units
 };
 struct Item {
-    int b, t0, n;      // sequence, first tile and number of tiles this CTA serves of it
+    int b, t0, n;      // sequence, first tile and number of tiles this chunk holds of it
     int ctx, tb;       // its context length and total tiles
     long long fv;      // unit at which the sequence starts (its tile 0 sits at fv + item_cost)
 };
 
-// Advance to the next sequence of which this CTA serves at least one tile; false when the range is exhausted.
+// Advance to the next sequence of which the chunk holds at least one tile; false when the chunk is exhausted.
 // (hint_b, hint_ctx): a context length the caller has fetched ahead of time (hint_b < 0: none).
-__device__ __forceinline__ bool next_item(Walk& w, const Params& p, int max_ctx, Item& it, int hint_b = -1,
-                                          int hint_ctx = 0) {
+__device__ __forceinline__ bool next_item(Walk& w, const Params& p, int max_ctx, Item& it, int hint_b, int hint_ctx) {
     while (w.b < p.B && w.fv < w.x1) {
         const int ctx = clamp_ctx(w.b == hint_b ? hint_ctx : __ldg(p.context_lens + w.b), max_ctx);
         const int tb = tiles_of(ctx);
@@ -136,7 +195,7 @@ __device__ __forceinline__ bool next_item(Walk& w, const Params& p, int max_ctx,
         const long long lo = w.x0 - t_base, hi = w.x1 - t_base;
         const int t0 = (int)(lo < 0 ? 0 : (lo > tb ? tb : lo));
         const int t1 = (int)(hi < 0 ? 0 : (hi > tb ? tb : hi));
-        if (t0 >= t1) continue;  // only boundary units of this sequence fall into the range
+        if (t0 >= t1) continue;  // only boundary units of this sequence fall into the chunk
         it.t0 = t0;
         it.n = t1 - t0;
         it.ctx = ctx;
@@ -146,45 +205,51 @@ __device__ __forceinline__ bool next_item(Walk& w, const Params& p, int max_ctx,
     return false;
 }
 
-// Combine the partials of sequence b (its tiles occupy units [first, first + tb) of the cost line) for kv head kvh and
-// write its G output rows.  Called by the 128 consumer threads: thread t owns row t / 16 and dims 8 (t % 16) ..
-// 8 (t % 16) + 7.  Partials are taken in group order, four at a time (all loads of a batch are independent), so the
-// result does not depend on which CTA runs this.
-__device__ __forceinline__ void merge_sequence(const Params& p, int b, int kvh, long long first, int tb,
-                                               long long total, int ctid) {
+// What the producer tells the consumers about a tile, beside the tile in the ring.
+struct TileMeta {
+    int valid;   // live tokens from this tile's first token on
+    int flags;   // kFirst | kLast | kWhole | kDone
+    int b;       // sequence
+    int part;    // record of the partial result (an item that is not a whole sequence)
+    int gf, gl;  // first and last chunk that hold tiles of the sequence
+    int pad[2];
+};
+constexpr int kFirst = 1, kLast = 2, kWhole = 4, kDone = 8;
+
+// Combine the partials of sequence b (chunks gf .. gl) for kv head kvh and write its G output rows.  Called by the 128
+// consumer threads: thread t owns row t / 16 and dims 8 (t % 16) .. 8 (t % 16) + 7.  Partials are taken in chunk order,
+// kMergeBatch at a time (all loads of a batch are in flight together), so the result does not depend on which CTA runs this.
+__device__ __forceinline__ void merge_sequence(const Params& p, int b, int kvh, int gf, int gl, int ctid) {
     const int r = ctid >> 4, c8 = (ctid & 15) * 8;
     if (r >= p.G) return;
-    const int ng = p.num_groups;
-    long long gf = ((first + 1) * ng - 1) / total;
-    long long gl = ((first + tb) * ng - 1) / total;
-    if (gf > ng - 1) gf = ng - 1;
-    if (gl > ng - 1) gl = ng - 1;
     const size_t pf = partial_floats(p.G);
     float mt = -INFINITY, lt = 0.f;
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    for (long long g0 = gf; g0 <= gl; g0 += 4) {
-        float mv[4], lv[4];
-        float4 oa[4], ob[4];
+    for (int g0 = gf; g0 <= gl; g0 += kMergeBatch) {
+        float mv[kMergeBatch], lv[kMergeBatch];
+        float4 oa[kMergeBatch], ob[kMergeBatch];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const long long g = g0 + u;
-            const bool live = g <= gl && (g * total / ng < (g + 1) * total / ng);  // empty groups wrote nothing
+        for (int u = 0; u < kMergeBatch; ++u) {
+            const int g = g0 + u;
+            const bool live = g <= gl;
             const float* part = p.partials + ((size_t)(g * p.KVH + kvh) * 2 + (g == gf ? 1 : 0)) * pf;
             mv[u] = live ? __ldcg(part + p.G * kD + r) : -INFINITY;
             lv[u] = live ? __ldcg(part + p.G * kD + kMaxG + r) : 0.f;
             oa[u] = live ? __ldcg(reinterpret_cast<const float4*>(part + r * kD + c8)) : make_float4(0.f, 0.f, 0.f, 0.f);
             ob[u] = live ? __ldcg(reinterpret_cast<const float4*>(part + r * kD + c8) + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        const float mnew = fmaxf(fmaxf(mt, fmaxf(mv[0], mv[1])), fmaxf(mv[2], mv[3]));
+        float mnew = mt;
+#pragma unroll
+        for (int u = 0; u < kMergeBatch; ++u) mnew = fmaxf(mnew, mv[u]);
         if (mnew == -INFINITY) continue;
         const float sc = (mt == -INFINITY) ? 0.f : fast_exp2(mt - mnew);
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] *= sc;
         lt *= sc;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < kMergeBatch; ++u) {
             const float f = (mv[u] == -INFINITY) ? 0.f : fast_exp2(mv[u] - mnew);
             acc[0] += oa[u].x * f;
             acc[1] += oa[u].y * f;
@@ -207,34 +272,55 @@ __device__ __forceinline__ void merge_sequence(const Params& p, int b, int kvh, 
     *reinterpret_cast<uint4*>(p.out + ((size_t)b * p.H + (size_t)kvh * p.G + r) * kD + c8) = w;
 }
 
-__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+__device__ __forceinline__ unsigned int atomic_add_acq_rel(unsigned int* addr, unsigned int v) {
+    unsigned int old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(addr), "r"(v) : "memory");
+    return old;
+}
+
+__device__ __forceinline__ bool wait_or_abort(volatile int* abort, uint64_t* bar, uint32_t parity) {
+    return mbar_try_wait(bar, parity) || (!*abort && mbar_wait(bar, parity));
+}
+
+// The G query rows of (sequence b, kv head kvh), behind the tile in its ring stage.
+__device__ __forceinline__ void load_q(const Params& p, uint8_t* stage, uint64_t* bar, int b, int kvh) {
+    bulk_load(stage + 2 * kTileBytes, p.q + ((size_t)b * p.H + (size_t)kvh * p.G) * kD, (uint32_t)p.G * kD * 2, bar);
+}
+
+// Two CTAs fit an SM (shared memory).  The registers of a third are left free: the blocks of the kernel behind this one on
+// the stream (128 or 256 threads) then start, and wait, beside this kernel's CTAs instead of after them, and this kernel's
+// CTAs beside the blocks of the kernel in front.
+__global__ void __launch_bounds__(kThreads, kCtasPerSm + 1)
 paged_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                     const Params p) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    extern __shared__ __align__(1024) uint8_t smem[];
     float* Os = reinterpret_cast<float*>(smem + kStages * kStageBytes);
     uint8_t* misc = smem + kStages * kStageBytes + kOsBytes;
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(misc);            // [kStages]
     uint64_t* empty_bar = full_bar + kStages;                          // [kStages]
-    int* sm_i = reinterpret_cast<int*>(misc + 64);                     // scan scratch [8] + start [2] + abort [1]
+    int* sm_i = reinterpret_cast<int*>(misc + 64);                     // scan scratch [8], ticket [1], abort [1]
     volatile int* sm_abort = sm_i + 12;
-    long long* sm_fv = reinterpret_cast<long long*>(sm_i + 14);       // unit at which the CTA's first sequence starts
     float* sm_ml = reinterpret_cast<float*>(misc + 128);               // [2 parities][m|l][4 warps][8 rows]
+    TileMeta* sm_meta = reinterpret_cast<TileMeta*>(misc + 640);       // [kStages]
+    long long* sm_seg = reinterpret_cast<long long*>(misc + 768);      // [kThreads] unit at which a thread's sequences start
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
     const int kvh = blockIdx.x % p.KVH;
-    const int group = blockIdx.x / p.KVH;
+    const int chunk = blockIdx.x / p.KVH;
     const int max_ctx = p.MB * p.block_size;
 
+    if (smem_u32(smem) & 1023) {  // the swizzled tiles need it; the alignment above asks for it
+        if (tid == 0) atomicOr(&g_error_flag, 1);
+        griddep_wait();
+        return;
+    }
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_bar + s, 1);
             mbar_init(empty_bar + s, kConsumerWarps);
         }
         fence_mbar_init();
-        sm_i[10] = -1;
-        sm_i[11] = 0;
         *sm_abort = 0;
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
@@ -244,321 +330,384 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
 
     // Programmatic dependent launch: this grid starts while the kernel launched just before it on the stream
     // (decode_prepare_kernel: ticket clear, and in the fused step the scatter / rotation of the step's rows) is
-    // still running.  That kernel writes tickets, cache rows and (fused step) q -- never context_lens or
-    // block_tables -- and everything launched before IT has completed by the time this grid starts (its own
-    // blocks passed their griddepcontrol.wait before they let this grid go).  So the scan below and the first
-    // page lookup read only settled memory and run ahead of the wait; the wait sits right before the first
-    // access to anything the preparing kernel writes.
+    // still running.  That kernel writes tickets, the cache rows of the step's slots and (fused step) q -- never
+    // context_lens, block_tables or slot_mapping -- and everything launched before IT has completed by the time this
+    // grid starts (its own blocks passed their griddepcontrol.wait before they let this grid go).  So the scan below,
+    // the page lookups and the K/V rows of all other slots are settled memory: the producer requests the CTA's first
+    // tiles ahead of the wait unless they hold a slot that this step writes, and waits only then.
 
-    // ---- prologue: total cost units per head and the sequence this CTA's range starts in ----
+    // The step's slots, for that check (one load latency, in parallel with the scan's).
+    int my_slots[kEarlySlots];
+    const bool early = p.slot_mapping == nullptr || p.B <= 32 * kEarlySlots;
+    if (warp == kConsumerWarps && p.slot_mapping != nullptr && early) {
+#pragma unroll
+        for (int i = 0; i < kEarlySlots; ++i)
+            my_slots[i] = lane + 32 * i < p.B ? __ldg(p.slot_mapping + lane + 32 * i) : -1;
+    }
+
+    // ---- prologue: total cost units per head, and where on the line every thread's share of the sequences starts ----
     // Every CTA scans context_lens itself (B / 160 values per thread and one warp scan): that is one global
     // load latency, paid in parallel by all CTAs, and cheaper than fetching the result of a serial plan.
     const int per = (p.B + kThreads - 1) / kThreads;
-    const int b_lo = min(p.B, tid * per), b_hi = min(p.B, b_lo + per);
-    int mine = 0;
-    for (int b = b_lo; b < b_hi; ++b) {
-        const int tb = tiles_of(clamp_ctx(__ldg(p.context_lens + b), max_ctx));
-        mine += units_of(tb, p.item_cost);
-        if (tb == 0 && b % p.num_groups == group) {
-            // an empty sequence attends to nothing: its rows are zeros (one CTA per kv head writes them)
-            uint4* orow = reinterpret_cast<uint4*>(p.out + ((size_t)b * p.H + (size_t)kvh * p.G) * kD);
-            for (int i = 0; i < p.G * (kD * 2 / 16); ++i) orow[i] = make_uint4(0, 0, 0, 0);
-        }
-    }
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) sm_i[warp] = incl;
-    __syncthreads();
-    long long total = 0;
-    int warp_off = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-        const int v = sm_i[w];
-        if (w < warp) warp_off += v;
-        total += v;
-    }
-    const long long x0 = (long long)group * total / p.num_groups;
-    const long long x1 = (long long)(group + 1) * total / p.num_groups;
     {
-        long long run = warp_off + incl - mine;
+        const int b_lo = min(p.B, tid * per), b_hi = min(p.B, b_lo + per);
+        int mine = 0;
         for (int b = b_lo; b < b_hi; ++b) {
-            const int ub = units_of(tiles_of(clamp_ctx(__ldg(p.context_lens + b), max_ctx)), p.item_cost);
-            if (ub > 0 && run <= x0 && x0 < run + ub) {
-                sm_i[10] = b;
-                *sm_fv = run;
+            const int tb = tiles_of(clamp_ctx(__ldg(p.context_lens + b), max_ctx));
+            mine += units_of(tb, p.item_cost);
+            if (tb == 0 && b % (int)gridDim.x == (int)blockIdx.x) {
+                // an empty sequence attends to nothing: its rows are zeros (one CTA writes them)
+                uint4* orow = reinterpret_cast<uint4*>(p.out + (size_t)b * p.H * kD);
+                for (int i = 0; i < p.H * (kD * 2 / 16); ++i) orow[i] = make_uint4(0, 0, 0, 0);
             }
-            run += ub;
         }
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) sm_i[warp] = incl;
+        __syncthreads();
+        long long warp_off = 0;
+        for (int w = 0; w < warp; ++w) warp_off += sm_i[w];
+        sm_seg[tid] = warp_off + incl - mine;
+        __syncthreads();
     }
-    __syncthreads();
-    if (x0 >= x1 || sm_i[10] < 0) return;  // nothing to do (uniform across the CTA)
+    long long total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) total += sm_i[w];
+    const Cut cut = make_cut(total, p.num_groups);
+    if (total == 0 || chunk >= cut.groups) {  // less work than CTAs (uniform across the CTA)
+        griddep_wait();  // this grid must not be complete before the kernel in front of it is
+        return;
+    }
 
-    Walk walk;
-    walk.b = sm_i[10];
-    walk.fv = *sm_fv;
-    walk.x0 = x0;
-    walk.x1 = x1;
-    // page of the first tile, fetched ahead of the wait (block_tables is settled memory, see above)
-    int first_phys = 0;
-    if (warp == kConsumerWarps && lane == 0) {
-        Walk peek = walk;
-        Item first;
-        if (next_item(peek, p, max_ctx, first))
-            first_phys = __ldg(p.block_tables + (size_t)first.b * p.MB + (first.t0 * kTile) / p.block_size);
-    }
-    griddep_wait();
+    const uint32_t stages = ring_stages(cut);
 
     if (warp == kConsumerWarps) {
         // =========================== producer warp ===========================
-        if (lane == 0) {
-            const uint64_t pol = policy_evict_first();
-            uint32_t it = 0;
-            Item item;
-            bool ok = true;
-            // Metadata of the sequence after the current one is fetched one item ahead (its length and its first
-            // page: every item but a CTA's first starts at tile 0), so that a sequence boundary does not put two
-            // dependent global-load latencies between two tile requests.
-            int pf_b = -1, pf_ctx = 0, pf_phys = 0;
-            while (ok && next_item(walk, p, max_ctx, item, pf_b, pf_ctx)) {
-                const int32_t* bt = p.block_tables + (size_t)item.b * p.MB;
-                for (int i = 0; i < item.n; ++i, ++it) {
-                    const int stage = it % kStages;
-                    const uint32_t parity = ((it / kStages) & 1u) ^ 1u;
-                    if (*sm_abort || !mbar_wait(empty_bar + stage, parity)) {
-                        ok = false;
-                        break;
-                    }
-                    const int tok0 = (item.t0 + i) * kTile;
-                    const int bi = tok0 / p.block_size;
-                    int phys = it == 0 ? first_phys : ((i == 0 && item.b == pf_b && bi == 0) ? pf_phys : __ldg(bt + bi));
-                    phys = phys < 0 ? 0 : (phys >= p.NB ? p.NB - 1 : phys);
-                    const int slot = phys * p.block_size + (tok0 - bi * p.block_size);
-                    uint8_t* st = smem + stage * kStageBytes;
-                    uint64_t* bar = full_bar + stage;
-                    const uint32_t qbytes = (i == 0) ? (uint32_t)p.G * kD * 2 : 0u;
-                    mbar_expect_tx(bar, 2 * kTileBytes + qbytes);
-                    tma_load_3d_hint(st, &tm_k, bar, 0, kvh, slot, pol);
-                    tma_load_3d_hint(st + kPanelBytes, &tm_k, bar, 64, kvh, slot, pol);
-                    tma_load_3d_hint(st + kTileBytes, &tm_v, bar, 0, kvh, slot, pol);
-                    tma_load_3d_hint(st + kTileBytes + kPanelBytes, &tm_v, bar, 64, kvh, slot, pol);
-                    if (i == 0) {
-                        bulk_load(st + 2 * kTileBytes, p.q + ((size_t)item.b * p.H + (size_t)kvh * p.G) * kD, qbytes,
-                                  bar);
-                        if (walk.b < p.B) {  // the loads are issued now and first used at the next boundary
-                            pf_b = walk.b;
-                            pf_ctx = __ldg(p.context_lens + walk.b);
-                            pf_phys = __ldg(p.block_tables + (size_t)walk.b * p.MB);
-                        }
+        const uint64_t pol = policy_evict_first();
+        Walk walk;
+        walk.x0 = cut.bound(chunk);
+        walk.x1 = cut.bound(chunk + 1);
+        {
+            int s = -1;  // last segment that starts at or before x0
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) s += __popc(__ballot_sync(0xffffffffu, sm_seg[32 * w + lane] <= walk.x0));
+            walk.b = s * per;
+            walk.fv = sm_seg[s];
+        }
+        // Lane 0 walks the CTA's tiles; the other lanes help only to compare a tile with the step's slots, until the
+        // wait for the kernel in front has been passed.
+        Item item;
+        int left = 0;             // tiles left of `item`
+        int valid = 0;            // live tokens from the next tile on
+        int bi = 0, off = 0;      // its page and the offset in the page
+        int phys = 0, next = 0;   // that page's block and the following page's (requested one page ahead)
+        const int32_t* bt = p.block_tables;
+        // Metadata of the sequence after the current one is fetched one item ahead (its length and its first
+        // page: every item but a CTA's first starts at tile 0), so that a sequence boundary does not put two
+        // dependent global-load latencies between two tile requests.
+        int pf_b = -1, pf_ctx = 0, pf_phys = 0;
+        bool waited = false, ok = true;
+        uint32_t it = 0, stage = 0, parity = 1;  // parity of the stage's "empty" phase: its first filling need not wait
+#pragma unroll 1
+        while (true) {
+            int slot = -1, flags = 0;
+            if (lane == 0) {
+                if (left == 0 && next_item(walk, p, max_ctx, item, pf_b, pf_ctx)) {
+                    left = item.n;
+                    flags = kFirst;
+                    valid = item.ctx - item.t0 * kTile;
+                    bi = item.t0 == 0 ? 0 : item.t0 * kTile / p.block_size;
+                    off = item.t0 * kTile - bi * p.block_size;
+                    bt = p.block_tables + (size_t)item.b * p.MB;
+                    phys = item.b == pf_b && bi == 0 ? pf_phys : __ldg(bt + bi);
+                    next = bi + 1 < p.MB ? __ldg(bt + bi + 1) : 0;
+                    if (walk.b < p.B) {  // the loads are issued now and first used at the next boundary
+                        pf_b = walk.b;
+                        pf_ctx = __ldg(p.context_lens + walk.b);
+                        pf_phys = __ldg(p.block_tables + (size_t)walk.b * p.MB);
                     }
                 }
+                if (left > 0) {
+                    slot = (phys < 0 ? 0 : (phys >= p.NB ? p.NB - 1 : phys)) * p.block_size + off;
+                    if (--left == 0) flags |= item.n == item.tb ? kLast | kWhole : kLast;
+                }
             }
-            if (!ok) {
-                *sm_abort = 1;
-                atomicOr(&g_error_flag, 1);
-                // Let loads already issued land before the CTA's shared memory is released.
-                for (uint32_t j = (it >= kStages ? it - kStages : 0); j < it; ++j)
-                    (void)mbar_wait(full_bar + (j % kStages), (j / kStages) & 1u, 1u << 16);
+            if (!waited) {
+                const int first_slot = __shfl_sync(0xffffffffu, slot, 0);
+                bool stop = !early || first_slot < 0 || it == (p.q_in_flight ? stages : 2 * stages);
+                if (p.slot_mapping != nullptr) {
+#pragma unroll
+                    for (int i = 0; i < kEarlySlots; ++i) {
+                        if (32 * i >= p.B) break;
+                        stop |= (uint32_t)(my_slots[i] - first_slot) < (uint32_t)kTile;
+                    }
+                }
+                if (__any_sync(0xffffffffu, stop)) {
+                    griddep_wait();
+                    waited = true;
+                    if (lane != 0) return;
+                    for (uint32_t e = 0; p.q_in_flight && e < it; ++e)
+                        if (sm_meta[e].flags & kFirst) load_q(p, smem + e * kStageBytes, full_bar + e, sm_meta[e].b, kvh);
+                }
             }
+            if (lane == 0) {
+                uint8_t* st = smem + stage * kStageBytes;
+                uint64_t* bar = full_bar + stage;
+                if (it >= stages && !wait_or_abort(sm_abort, empty_bar + stage, parity)) {
+                    ok = false;
+                    break;
+                }
+                if (slot < 0) {
+                    sm_meta[stage].flags = kDone;
+                    mbar_arrive(bar);
+                    break;
+                }
+                sm_meta[stage].valid = valid;
+                sm_meta[stage].flags = flags;
+                sm_meta[stage].b = item.b;
+                if ((flags & (kLast | kWhole)) == kLast) {
+                    const long long first = item.fv + p.item_cost;  // unit of the sequence's tile 0
+                    sm_meta[stage].part = (chunk * p.KVH + kvh) * 2 + (item.t0 == 0 ? 1 : 0);
+                    sm_meta[stage].gf = item.t0 == 0 ? chunk : cut.chunk_of(first);
+                    sm_meta[stage].gl = item.t0 + item.n == item.tb ? chunk : cut.chunk_of(first + item.tb - 1);
+                }
+                mbar_expect_tx(bar, 2 * kTileBytes + ((flags & kFirst) ? (uint32_t)p.G * kD * 2 : 0u));
+                tma_load_4d_hint(st, &tm_k, bar, 0, slot, 0, kvh, pol);
+                tma_load_4d_hint(st + kTileBytes, &tm_v, bar, 0, slot, 0, kvh, pol);
+                if ((waited || !p.q_in_flight) && (flags & kFirst)) load_q(p, st, bar, item.b, kvh);
+                valid -= kTile;
+                off += kTile;
+                if (off == p.block_size) {
+                    off = 0;
+                    phys = next;
+                    ++bi;
+                    next = bi + 1 < p.MB ? __ldg(bt + bi + 1) : 0;
+                }
+            }
+            ++it;
+            if (++stage == stages) stage = 0, parity ^= 1u;
+        }
+        if (!ok) {
+            *sm_abort = 1;
+            atomicOr(&g_error_flag, 1);
+            // Let loads already issued land before the CTA's shared memory is released.
+            for (uint32_t j = (it >= stages ? it - stages : 0); j < it; ++j)
+                (void)mbar_wait(full_bar + (j % stages), (j / stages) & 1u, 1u << 16);
         }
         return;
     }
 
     // ============================= consumer warps =============================
-    const int row = lane >> 2;       // query head within the group (valid if < G)
+    // Both products are computed transposed, tokens or dims as the 16 rows and the query heads as the 8 columns of
+    // mma.m16n8k16: S^T = K Q^T and O^T += V^T P^T.  Lane l holds tokens (dims) l / 4 and l / 4 + 8 of heads 2 (l % 4) and
+    // 2 (l % 4) + 1.
+    const int grp = lane >> 2;
     const int quad = lane & 3;
     const int mi = lane >> 3;        // which 8x8 matrix this lane addresses in ldmatrix.x4
     const int r8 = lane & 7;
     const int tok_base = warp * 16;
     const int ctid = tid;            // 0..127 among consumers
-    uint32_t it = 0, item = 0;
-    Item cur;
-    bool ok = true;
+    uint32_t item = 0;
+    uint32_t qb[8][2];               // Q^T: dims 16 ks + 2 quad (+1), + 8 of head grp
+    float o[8][4];                   // O^T: dims 16 j + grp and + 8 of the lane's two heads
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;  // per head; the sums are this lane's tokens only
+    bool waited = false;             // for the kernel in front, which clears the tickets
 
-    for (; ok && next_item(walk, p, max_ctx, cur); ++item) {
-        const int n = cur.n, ctx = cur.ctx, tb = cur.tb;
-        const bool full_item = (cur.t0 == 0 && n == tb);
+    for (uint32_t next = 0, parity = 0;;) {
+        const uint32_t stage = next;
+        if (!wait_or_abort(sm_abort, full_bar + stage, parity)) {
+            *sm_abort = 1;
+            atomicOr(&g_error_flag, 2);
+            break;
+        }
+        if (++next == stages) next = 0, parity ^= 1u;
+        uint8_t* st = smem + stage * kStageBytes;
+        const int2 head = *reinterpret_cast<const int2*>(sm_meta + stage);
+        const int flags = head.y;
+        if (flags & kDone) break;
+        if (flags & kFirst) {
+            const uint32_t* qs = reinterpret_cast<const uint32_t*>(st + 2 * kTileBytes);
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+                qb[ks][0] = grp < p.G ? qs[grp * 64 + ks * 8 + quad] : 0u;
+                qb[ks][1] = grp < p.G ? qs[grp * 64 + ks * 8 + 4 + quad] : 0u;
+            }
+            m0 = m1 = -INFINITY;
+            l0 = l1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+        }
+        const int valid = head.x - tok_base;  // live tokens in this warp's 16-token slice
+        if (valid > 0) {
+            const uint32_t kbase = smem_u32(st);
+            const uint32_t vbase = kbase + kTileBytes;
+            if (valid < 16) {
+                // Rows past the context end may hold anything (even NaN bit patterns): zero the V rows so
+                // that 0 * garbage cannot reach the accumulators.  Each row is 2 panels x 8 chunks of 16 B.
+                for (int idx = lane; idx < (16 - valid) * 16; idx += 32) {
+                    const int r = tok_base + valid + (idx >> 4);
+                    const int c = idx & 15;
+                    uint8_t* dst = st + kTileBytes + (c >> 3) * kPanelBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+                    *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+                }
+                fence_proxy_async_smem();  // order these generic writes before the stage's next TMA refill
+                __syncwarp();
+            }
+            // ---- S^T = K Q^T for 16 tokens, in two accumulators (half the chain) ----
+            float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+            {
+                const uint32_t krow = kbase + (tok_base + (mi & 1) * 8 + r8) * 128;
+#pragma unroll
+                for (int ks = 0; ks < 8; ++ks) {
+                    const int chunk = ks * 2 + (mi >> 1);
+                    uint32_t a[4];
+                    ldsm_x4(krow + (chunk >> 3) * kPanelBytes + (((chunk & 7) ^ r8) << 4), a);
+                    mma_16816(ks & 1 ? sb : sa, a, qb[ks][0], qb[ks][1]);
+                }
+            }
+            // ---- online softmax (log2 domain), against a maximum that may be stale by up to 2^kStale: it cancels in
+            // the final division, and as long as no score exceeds it by more the lanes need not agree on a new one ----
+            const float s00 = sa[0] + sb[0], s01 = sa[1] + sb[1], s10 = sa[2] + sb[2], s11 = sa[3] + sb[3];
+            const bool in0 = grp < valid, in1 = grp + 8 < valid;
+            float x00 = in0 ? fmaf(s00, p.scale_log2, -m0) : -INFINITY, x01 = in0 ? fmaf(s01, p.scale_log2, -m1) : -INFINITY;
+            float x10 = in1 ? fmaf(s10, p.scale_log2, -m0) : -INFINITY, x11 = in1 ? fmaf(s11, p.scale_log2, -m1) : -INFINITY;
+            if (__any_sync(0xffffffffu, fmaxf(fmaxf(x00, x01), fmaxf(x10, x11)) > kStale)) {
+                float r0 = fmaxf(in0 ? s00 * p.scale_log2 : -INFINITY, in1 ? s10 * p.scale_log2 : -INFINITY);
+                float r1 = fmaxf(in0 ? s01 * p.scale_log2 : -INFINITY, in1 ? s11 * p.scale_log2 : -INFINITY);
+#pragma unroll
+                for (int step = 4; step < 32; step <<= 1) {
+                    r0 = fmaxf(r0, __shfl_xor_sync(0xffffffffu, r0, step));
+                    r1 = fmaxf(r1, __shfl_xor_sync(0xffffffffu, r1, step));
+                }
+                r0 = fmaxf(m0, r0), r1 = fmaxf(m1, r1);
+                const float f0 = fast_exp2(m0 - r0), f1 = fast_exp2(m1 - r1);
+                m0 = r0, m1 = r1;
+                l0 *= f0, l1 *= f1;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j][0] *= f0, o[j][1] *= f1, o[j][2] *= f0, o[j][3] *= f1;
+                x00 = in0 ? fmaf(s00, p.scale_log2, -m0) : -INFINITY, x01 = in0 ? fmaf(s01, p.scale_log2, -m1) : -INFINITY;
+                x10 = in1 ? fmaf(s10, p.scale_log2, -m0) : -INFINITY, x11 = in1 ? fmaf(s11, p.scale_log2, -m1) : -INFINITY;
+            }
+            x00 = fast_exp2(x00), x01 = fast_exp2(x01), x10 = fast_exp2(x10), x11 = fast_exp2(x11);
+            l0 += x00 + x10;
+            l1 += x01 + x11;
+            // P^T as the B operand: tokens along k, head grp as the column
+            const uint32_t p0 = transpose_8x8(pack_bf16(x00, x01)), p1 = transpose_8x8(pack_bf16(x10, x11));
+            // ---- O^T += V^T P^T: 8 row tiles of 16 dims ----
+            {
+                const uint32_t vrow = vbase + (tok_base + (mi >> 1) * 8 + r8) * 128;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int chunk = j * 2 + (mi & 1);
+                    uint32_t a[4];
+                    ldsm_x4_t(vrow + (chunk >> 3) * kPanelBytes + (((chunk & 7) ^ r8) << 4), a);
+                    mma_16816(o[j], a, p0, p1);
+                }
+            }
+        }
+        TileMeta tm;
+        if (flags & kLast) tm = sm_meta[stage];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty_bar + stage);
+        if (!(flags & kLast)) continue;
+
+        // ---- merge the four warps' (m, l, O) and emit the item ----
         // (m, l) exchange buffers alternate between consecutive items so that a warp that races ahead
         // into the next item cannot overwrite values a slower warp is still reading.
         float* sm_m = sm_ml + (item & 1u) * (2 * kConsumerWarps * kMaxG);
         float* sm_l = sm_m + kConsumerWarps * kMaxG;
-        uint32_t qa[8][2];
-        float o[16][4];
-        float m = -INFINITY, l = 0.f;
+        ++item;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-
-        for (int i = 0; i < n; ++i, ++it) {
-            const int stage = it % kStages;
-            if (*sm_abort || !mbar_wait(full_bar + stage, (it / kStages) & 1u)) {
-                ok = false;
-                break;
-            }
-            uint8_t* st = smem + stage * kStageBytes;
-            if (i == 0) {
-                const uint32_t* qs = reinterpret_cast<const uint32_t*>(st + 2 * kTileBytes);
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    qa[ks][0] = row < p.G ? qs[row * 64 + ks * 8 + quad] : 0u;
-                    qa[ks][1] = row < p.G ? qs[row * 64 + ks * 8 + 4 + quad] : 0u;
-                }
-            }
-            const int valid = ctx - ((cur.t0 + i) * kTile + tok_base);  // live tokens in this warp's 16-token slice
-            if (valid > 0) {
-                const uint32_t kbase = smem_u32(st);
-                const uint32_t vbase = kbase + kTileBytes;
-                if (valid < 16) {
-                    // Rows past the context end may hold anything (even NaN bit patterns): zero the V rows so
-                    // that 0 * garbage cannot reach the accumulators.  Each row is 2 panels x 8 chunks of 16 B.
-                    for (int idx = lane; idx < (16 - valid) * 16; idx += 32) {
-                        const int r = tok_base + valid + (idx >> 4);
-                        const int c = idx & 15;
-                        uint8_t* dst = st + kTileBytes + (c >> 3) * kPanelBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4);
-                        *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-                    }
-                    fence_proxy_async_smem();  // order these generic writes before the stage's next TMA refill
-                    __syncwarp();
-                }
-                // ---- S = Q K^T for 16 tokens: two n-tiles of 8 tokens ----
-                float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-                {
-                    const int tok = tok_base + (mi >> 1) * 8 + r8;
-#pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) {
-                        const int chunk = ks * 2 + (mi & 1);
-                        const uint32_t addr =
-                            kbase + (chunk >> 3) * kPanelBytes + tok * 128 + (((chunk & 7) ^ r8) << 4);
-                        uint32_t b0, b1, b2, b3;
-                        ldsm_x4(addr, b0, b1, b2, b3);
-                        mma_lo(s0, qa[ks][0], qa[ks][1], b0, b1);
-                        mma_lo(s1, qa[ks][0], qa[ks][1], b2, b3);
-                    }
-                }
-                // ---- online softmax (log2 domain) ----
-                const int c0 = 2 * quad;
-                float v00 = (c0 < valid) ? s0[0] * p.scale_log2 : -INFINITY;
-                float v01 = (c0 + 1 < valid) ? s0[1] * p.scale_log2 : -INFINITY;
-                float v10 = (c0 + 8 < valid) ? s1[0] * p.scale_log2 : -INFINITY;
-                float v11 = (c0 + 9 < valid) ? s1[1] * p.scale_log2 : -INFINITY;
-                float rmax = fmaxf(fmaxf(v00, v01), fmaxf(v10, v11));
-                rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 1));
-                rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, 2));
-                const float m_new = fmaxf(m, rmax);
-                const float alpha = fast_exp2(m - m_new);
-                v00 = fast_exp2(v00 - m_new);
-                v01 = fast_exp2(v01 - m_new);
-                v10 = fast_exp2(v10 - m_new);
-                v11 = fast_exp2(v11 - m_new);
-                l = l * alpha + ((v00 + v01) + (v10 + v11));
-                m = m_new;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    o[j][0] *= alpha;
-                    o[j][1] *= alpha;
-                }
-                const uint32_t pa0 = pack_bf16(v00, v01), pa2 = pack_bf16(v10, v11);
-                // ---- O += P V: 16 n-tiles of 8 dims, two per ldmatrix.x4.trans ----
-                {
-                    const int tok = tok_base + (mi & 1) * 8 + r8;
-#pragma unroll
-                    for (int np = 0; np < 8; ++np) {
-                        const int chunk = np * 2 + (mi >> 1);
-                        const uint32_t addr =
-                            vbase + (chunk >> 3) * kPanelBytes + tok * 128 + (((chunk & 7) ^ r8) << 4);
-                        uint32_t b0, b1, b2, b3;
-                        ldsm_x4_t(addr, b0, b1, b2, b3);
-                        mma_lo(o[2 * np], pa0, pa2, b0, b1);
-                        mma_lo(o[2 * np + 1], pa0, pa2, b2, b3);
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty_bar + stage);
+        for (int step = 4; step < 32; step <<= 1) {
+            l0 += __shfl_xor_sync(0xffffffffu, l0, step);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, step);
         }
-        if (!ok) break;
-
-        // ---- merge the four warps' (m, l, O) and emit the item ----
-        l += __shfl_xor_sync(0xffffffffu, l, 1);
-        l += __shfl_xor_sync(0xffffffffu, l, 2);
-        if (quad == 0) {
-            sm_m[warp * kMaxG + row] = m;
-            sm_l[warp * kMaxG + row] = l;
+        if (grp == 0) {
+            *reinterpret_cast<float2*>(sm_m + warp * kMaxG + 2 * quad) = make_float2(m0, m1);
+            *reinterpret_cast<float2*>(sm_l + warp * kMaxG + 2 * quad) = make_float2(l0, l1);
         }
         named_barrier_sync(1, kConsumerWarps * 32);
         {
             // Fixed-order reduction (bitwise reproducible): warps 0,1 store, warps 2,3 add, readers sum the two.
-            float mt = -INFINITY;
+            float t0 = -INFINITY, t1 = -INFINITY;
 #pragma unroll
-            for (int w = 0; w < kConsumerWarps; ++w) mt = fmaxf(mt, sm_m[w * kMaxG + row]);
-            const float f = (m == -INFINITY) ? 0.f : fast_exp2(m - mt);
-            float* dst = Os + (warp & 1) * (kMaxG * kOsStride) + row * kOsStride + 2 * quad;
+            for (int w = 0; w < kConsumerWarps; ++w) {
+                const float2 v = *reinterpret_cast<const float2*>(sm_m + w * kMaxG + 2 * quad);
+                t0 = fmaxf(t0, v.x), t1 = fmaxf(t1, v.y);
+            }
+            const float f0 = (m0 == -INFINITY) ? 0.f : fast_exp2(m0 - t0), f1 = (m1 == -INFINITY) ? 0.f : fast_exp2(m1 - t1);
+            float* d0 = Os + (warp & 1) * (kMaxG * kOsStride) + 2 * quad * kOsStride + grp;
+            float* d1 = d0 + kOsStride;
             if (warp < 2) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    *reinterpret_cast<float2*>(dst + j * 8) = make_float2(o[j][0] * f, o[j][1] * f);
+                for (int j = 0; j < 8; ++j) {
+                    d0[16 * j] = o[j][0] * f0, d1[16 * j] = o[j][1] * f1;
+                    d0[16 * j + 8] = o[j][2] * f0, d1[16 * j + 8] = o[j][3] * f1;
+                }
             }
             named_barrier_sync(1, kConsumerWarps * 32);
             if (warp >= 2) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    float2 cur = *reinterpret_cast<float2*>(dst + j * 8);
-                    cur.x += o[j][0] * f;
-                    cur.y += o[j][1] * f;
-                    *reinterpret_cast<float2*>(dst + j * 8) = cur;
+                for (int j = 0; j < 8; ++j) {
+                    d0[16 * j] += o[j][0] * f0, d1[16 * j] += o[j][1] * f1;
+                    d0[16 * j + 8] += o[j][2] * f0, d1[16 * j + 8] += o[j][3] * f1;
                 }
             }
         }
         named_barrier_sync(1, kConsumerWarps * 32);
-        {
-            float* part = nullptr;
-            if (!full_item)
-                part = p.partials + ((size_t)blockIdx.x * 2 + (cur.t0 == 0 ? 1 : 0)) * partial_floats(p.G);
-            for (int r = 0; r < p.G; ++r) {
-                float mt = -INFINITY;
+        // thread t finishes row t / 16, dims 8 (t % 16) .. + 7
+        const int r = ctid >> 4, c8 = (ctid & 15) * 8;
+        if (r < p.G) {
+            float mt = -INFINITY;
 #pragma unroll
-                for (int w = 0; w < kConsumerWarps; ++w) mt = fmaxf(mt, sm_m[w * kMaxG + r]);
-                float lt = 0.f;
+            for (int w = 0; w < kConsumerWarps; ++w) mt = fmaxf(mt, sm_m[w * kMaxG + r]);
+            float lt = 0.f;
 #pragma unroll
-                for (int w = 0; w < kConsumerWarps; ++w) {
-                    const float mw = sm_m[w * kMaxG + r];
-                    if (mw != -INFINITY) lt += sm_l[w * kMaxG + r] * fast_exp2(mw - mt);
-                }
-                const float acc = Os[r * kOsStride + ctid] + Os[(kMaxG + r) * kOsStride + ctid];
-                if (full_item) {
-                    p.out[((size_t)cur.b * p.H + (size_t)kvh * p.G + r) * kD + ctid] =
-                        __float2bfloat16_rn(acc / (lt + 1e-9f));
-                } else {
-                    part[r * kD + ctid] = acc;
-                    if (ctid == 0) {
-                        part[p.G * kD + r] = mt;
-                        part[p.G * kD + kMaxG + r] = lt;
-                    }
-                }
+            for (int w = 0; w < kConsumerWarps; ++w) {
+                const float mw = sm_m[w * kMaxG + r];
+                if (mw != -INFINITY) lt += sm_l[w * kMaxG + r] * fast_exp2(mw - mt);
             }
-            if (!full_item) {
-                // Publish the partial, then take a ticket for this (sequence, kv head).  Whoever draws the last
-                // ticket finds every partial of the sequence visible and combines them; nobody waits.
-                __threadfence();
-                named_barrier_sync(1, kConsumerWarps * 32);
-                if (ctid == 0) sm_i[9] = (int)atomicAdd(p.tickets + (size_t)cur.b * p.KVH + kvh, 1u);
-                named_barrier_sync(1, kConsumerWarps * 32);
-                const long long first = cur.fv + p.item_cost;  // unit of the sequence's tile 0 on the cost line
-                long long parts = tb;  // fewer units than groups: every non-empty group holds exactly one unit
-                if (total >= p.num_groups)
-                    parts = ((first + tb) * p.num_groups - 1) / total - ((first + 1) * p.num_groups - 1) / total + 1;
-                if ((long long)sm_i[9] == parts - 1) {
-                    __threadfence();
-                    merge_sequence(p, cur.b, kvh, first, tb, total, ctid);
+            const float* s0 = Os + r * kOsStride + c8;
+            const float* s1 = s0 + kMaxG * kOsStride;
+            const float4 x0 = *reinterpret_cast<const float4*>(s0), x1 = *reinterpret_cast<const float4*>(s0 + 4);
+            const float4 y0 = *reinterpret_cast<const float4*>(s1), y1 = *reinterpret_cast<const float4*>(s1 + 4);
+            float4 a = make_float4(x0.x + y0.x, x0.y + y0.y, x0.z + y0.z, x0.w + y0.w);
+            float4 b = make_float4(x1.x + y1.x, x1.y + y1.y, x1.z + y1.z, x1.w + y1.w);
+            if (tm.flags & kWhole) {
+                const float den = lt + 1e-9f;
+                uint4 w;
+                w.x = pack_bf16(a.x / den, a.y / den);
+                w.y = pack_bf16(a.z / den, a.w / den);
+                w.z = pack_bf16(b.x / den, b.y / den);
+                w.w = pack_bf16(b.z / den, b.w / den);
+                *reinterpret_cast<uint4*>(p.out + ((size_t)tm.b * p.H + (size_t)kvh * p.G + r) * kD + c8) = w;
+            } else {
+                float* part = p.partials + (size_t)tm.part * partial_floats(p.G);
+                *reinterpret_cast<float4*>(part + r * kD + c8) = a;
+                *reinterpret_cast<float4*>(part + r * kD + c8 + 4) = b;
+                if (c8 == 0) {
+                    part[p.G * kD + r] = mt;
+                    part[p.G * kD + kMaxG + r] = lt;
                 }
             }
         }
-    }
-    if (!ok) {
-        *sm_abort = 1;
-        atomicOr(&g_error_flag, 2);
+        if (!(tm.flags & kWhole)) {
+            if (!waited) griddep_wait();
+            waited = true;
+            // Publish the partial, then take a ticket for this (sequence, kv head).  Whoever draws the last
+            // ticket finds every partial of the sequence visible and combines them; nobody waits.
+            named_barrier_sync(1, kConsumerWarps * 32);
+            if (ctid == 0) {
+                // release: the other threads' stores too, which the barrier orders before it
+                sm_i[9] = (int)atomic_add_acq_rel(p.tickets + (size_t)tm.b * p.KVH + kvh, 1u);
+            }
+            named_barrier_sync(1, kConsumerWarps * 32);
+            if (sm_i[9] == tm.gl - tm.gf) merge_sequence(p, tm.b, kvh, tm.gf, tm.gl, ctid);
+        }
     }
 }
 
@@ -574,7 +723,7 @@ decode_prepare_kernel(unsigned int* __restrict__ tickets, int num_tickets, int s
     griddep_wait();  // the previous kernel may still be reading these tickets or the cache rows written below
     griddep_launch_dependents();
     if ((int)blockIdx.x < store_blocks) {
-        store_block<SrcT>(blockIdx.x, k, v, k_cache, v_cache, slot_mapping, total_chunks, row_chunks, num_slots);
+        store_block<SrcT, 1>(blockIdx.x, k, v, k_cache, v_cache, slot_mapping, total_chunks, row_chunks, num_slots);
     } else {
         const int i = ((int)blockIdx.x - store_blocks) * kStoreThreads + threadIdx.x;
         if (i < num_tickets) tickets[i] = 0u;
@@ -643,11 +792,13 @@ static int cached_cache_map(CUtensorMap* map, const void* base, int64_t num_slot
     }
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return fail(NVLLM_B200_EDRIVER, "cuTensorMapEncodeTiled entry point not available");
-    cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)KVH, (cuuint64_t)num_slots};
-    cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)KVH * kD * 2};
-    cuuint32_t box[3] = {64, 1, (cuuint32_t)kTile};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+    // The head dimension is seen as two halves of 64 (the widest row a 128-byte swizzle takes) with the half as an outer
+    // dimension: one load then brings the tile in as the two 64-dim panels.
+    cuuint64_t dims[4] = {64, (cuuint64_t)num_slots, 2, (cuuint64_t)KVH};
+    cuuint64_t strides[3] = {(cuuint64_t)KVH * kD * 2, 64 * 2, (cuuint64_t)kD * 2};
+    cuuint32_t box[4] = {64, (cuuint32_t)kTile, 2, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(NVLLM_B200_EDRIVER, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
@@ -729,6 +880,8 @@ static int launch_decode(const char* who, const DecodeArgs& a, const StepArgs* s
     p.q = (const __nv_bfloat16*)a.q;
     p.block_tables = a.block_tables;
     p.context_lens = a.context_lens;
+    p.q_in_flight = pre != nullptr;
+    p.slot_mapping = pre ? pre->slot_mapping : (step ? step->slot_mapping : nullptr);
     p.out = (__nv_bfloat16*)a.out;
     p.tickets = tickets;
     p.partials = partials;
@@ -755,7 +908,7 @@ static int launch_decode(const char* who, const DecodeArgs& a, const StepArgs* s
     const int clear_blocks = (num_tickets + kStoreThreads - 1) / kStoreThreads;
     const int row_chunks = a.KVH * kD / 8;
     const int64_t total_chunks = step ? (int64_t)a.B * row_chunks : 0;
-    const int64_t store_blocks = step ? store_blocks_for(total_chunks) : 0;
+    const int64_t store_blocks = step ? store_blocks_for(total_chunks, 1) : 0;
     if (store_blocks + clear_blocks > 0x7fffffffLL) return fail(NVLLM_B200_EUNSUPPORTED, "%s: batch too large", who);
     cfg.gridDim = dim3((unsigned)(store_blocks + clear_blocks));
     cfg.blockDim = dim3(kStoreThreads);

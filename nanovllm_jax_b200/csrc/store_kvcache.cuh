@@ -29,18 +29,18 @@ __device__ __forceinline__ uint4 load_chunk_as_bf16(const float* src, int64_t ch
     return r;
 }
 
-// The share of store block `block` (of kStoreThreads threads): chunks [block*kStoreThreads*kStoreUnroll, +that).
+// The share of store block `block` (of kStoreThreads threads): chunks [block*kStoreThreads*kUnroll, +that).
 // A slot < 0 is skipped, a slot >= num_slots dropped.
-template <typename SrcT>
+template <typename SrcT, int kUnroll = kStoreUnroll>
 __device__ __forceinline__ void store_block(int64_t block, const SrcT* __restrict__ k, const SrcT* __restrict__ v,
                                             __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                                             const int32_t* __restrict__ slot_mapping, int64_t total_chunks,
                                             int row_chunks, int64_t num_slots) {
-    const int64_t base = block * (kStoreThreads * kStoreUnroll) + threadIdx.x;
-    uint4 kv[kStoreUnroll], vv[kStoreUnroll];
-    int64_t dst[kStoreUnroll];
+    const int64_t base = block * (kStoreThreads * kUnroll) + threadIdx.x;
+    uint4 kv[kUnroll], vv[kUnroll];
+    int64_t dst[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kStoreUnroll; ++u) {
+    for (int u = 0; u < kUnroll; ++u) {
         const int64_t i = base + (int64_t)u * kStoreThreads;
         dst[u] = -1;
         if (i < total_chunks) {
@@ -55,7 +55,7 @@ __device__ __forceinline__ void store_block(int64_t block, const SrcT* __restric
         }
     }
 #pragma unroll
-    for (int u = 0; u < kStoreUnroll; ++u) {
+    for (int u = 0; u < kUnroll; ++u) {
         if (dst[u] >= 0) {
             reinterpret_cast<uint4*>(k_cache)[dst[u]] = kv[u];
             reinterpret_cast<uint4*>(v_cache)[dst[u]] = vv[u];
@@ -63,8 +63,8 @@ __device__ __forceinline__ void store_block(int64_t block, const SrcT* __restric
     }
 }
 
-inline int64_t store_blocks_for(int64_t total_chunks) {
-    const int64_t per_block = (int64_t)kStoreThreads * kStoreUnroll;
+inline int64_t store_blocks_for(int64_t total_chunks, int unroll = kStoreUnroll) {
+    const int64_t per_block = (int64_t)kStoreThreads * unroll;
     return (total_chunks + per_block - 1) / per_block;
 }
 

@@ -113,7 +113,7 @@ struct Workspace {
     uint64_t used;
     at::Tensor buf;
 };
-constexpr size_t kMaxWorkspaces = 256;
+constexpr size_t kMaxWorkspaces = 64;
 std::vector<Workspace>& workspaces() {
     static auto* list = new std::vector<Workspace>();  // never destroyed: the allocator may be gone at exit
     return *list;
