@@ -732,6 +732,7 @@ decode_prepare_kernel(unsigned int* __restrict__ tickets, int num_tickets, int s
 
 // The same with the whole pre-attention step in front: blocks [0, pre_blocks) normalise and rotate the step's q and
 // k rows and scatter the k and v rows (pre_attention.cuh), the rest clear the tickets.
+// Small blocks: three of them fit an SM beside two CTAs of the attention kernel (registers).
 __global__ void __launch_bounds__(preattn::kThreads)
 decode_prepare_fused_kernel(unsigned int* __restrict__ tickets, int num_tickets, int pre_blocks, const preattn::Params pp) {
     griddep_wait();
@@ -915,7 +916,7 @@ static int launch_decode(const char* who, const DecodeArgs& a, const StepArgs* s
     cfg.dynamicSmemBytes = 0;
     if (pre) {
         const int64_t pre_blocks = preattn::blocks_for(pre->T, pre->H, pre->KVH);
-        cfg.gridDim = dim3((unsigned)(pre_blocks + clear_blocks));
+        cfg.gridDim = dim3((unsigned)(pre_blocks + (num_tickets + preattn::kThreads - 1) / preattn::kThreads));
         cfg.blockDim = dim3(preattn::kThreads);
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, decode_prepare_fused_kernel, tickets, num_tickets, (int)pre_blocks, *pre));
     } else if (step && step->src_dtype == NVLLM_B200_DTYPE_F32) {
@@ -1018,7 +1019,7 @@ extern "C" int nvllm_b200_fused_decode_step(void* q, void* k, const void* v, con
                           stream};
     const preattn::Params pp{(__nv_bfloat16*)q, (__nv_bfloat16*)k, (const __nv_bfloat16*)v, q_weight, k_weight,
                              cos_sin_cache, positions, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, slot_mapping,
-                             (int64_t)B, H, KVH, num_slots, max_pos, eps};
+                             (int64_t)B, H, KVH, num_slots, max_pos, eps, 1.0f};
     return decode_with_workspace("fused_decode_step", a, nullptr, workspace, workspace_bytes, &pp);
 }
 

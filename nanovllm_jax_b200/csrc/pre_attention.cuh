@@ -11,7 +11,8 @@
 // HBM-bound: per token (H + 2 KVH) rows of 256 B are read once, the q and k rows written back, the k and v rows
 // written to the cache.  Four lanes per row, four 16-byte chunks per lane (chunks q, q+4, q+8, q+12 of the row's sixteen:
 // a dim and its rotation partner 64 dims further sit in the same lane, and three quarters of the per-row scalar work --
-// the divide and the square root -- that sixteen lanes per row repeated is gone).
+// the divide and the square root -- that sixteen lanes per row repeated is gone).  The math runs on packed pairs of
+// neighbouring dims (.f32x2: two IEEE operations per instruction).
 //
 // Arithmetic is pinned so that a host restatement reproduces the bf16 results bit for bit: every fp32 operation
 // is a separate IEEE round-to-nearest multiply / add / divide / square root (no fused multiply-add, no approximate
@@ -25,8 +26,7 @@ namespace nvllm {
 namespace preattn {
 
 constexpr int kD = 128;
-constexpr int kThreads = 256;
-constexpr int kRowsPerBlock = kThreads / 4;  // four lanes per 256-byte row
+constexpr int kThreads = 64;  // of a block that works row by row: small, so that it fits beside other kernels' CTAs
 
 struct Params {
     __nv_bfloat16* q;
@@ -43,31 +43,45 @@ struct Params {
     int H, KVH;
     int64_t num_slots, max_pos;
     float eps;
+    float one;  // 1.0f
 };
 
-__device__ __forceinline__ void unpack8(const uint4& w, float (&f)[8]) {
-    const uint32_t u[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float(u[i] << 16);
-        f[2 * i + 1] = __uint_as_float(u[i] & 0xFFFF0000u);
-    }
+// Packed pairs of fp32: every operation is two separate IEEE round-to-nearest operations.
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
 }
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-    uint4 w;
-    w.x = pack_bf16(f[0], f[1]);
-    w.y = pack_bf16(f[2], f[3]);
-    w.z = pack_bf16(f[4], f[5]);
-    w.w = pack_bf16(f[6], f[7]);
-    return w;
+__device__ __forceinline__ void split(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
-__device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-
-constexpr int kRowsInFlight = 2;  // rows a thread of the stand-alone kernel has loads in flight for
+// Sums are written a * one + b, with a `one` (or minus one) that reaches the kernel as an argument: the assembler contracts
+// a packed add or subtract behind a packed multiply into one fused operation, explicit rounding or not -- it also sees
+// through a constant one -- and the result then differs in the last bit.
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t unpack_bf16(uint32_t u) {
+    return pair(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+}
+__device__ __forceinline__ uint32_t pack_pair(uint64_t v) {
+    float a, b;
+    split(v, a, b);
+    return pack_bf16(a, b);
+}
+// eight consecutive floats as four pairs
+__device__ __forceinline__ void load_pairs(const float* src, uint64_t (&f)[4]) {
+    const float4 a = *reinterpret_cast<const float4*>(src), b = *(reinterpret_cast<const float4*>(src) + 1);
+    f[0] = pair(a.x, a.y), f[1] = pair(a.z, a.w), f[2] = pair(b.x, b.y), f[3] = pair(b.z, b.w);
+}
 
 inline int64_t blocks_for(int64_t T, int H, int KVH) {
-    const int64_t rows = T * (H + 2 * KVH);
-    return (rows + kRowsPerBlock - 1) / kRowsPerBlock;
+    return (T * (H + 2 * KVH) * 4 + kThreads - 1) / kThreads;
 }
 
 // A quarter of one row as a thread holds it between its loads and its math: lane q (0..3) of the row's four lanes owns
@@ -102,86 +116,97 @@ __device__ __forceinline__ Part load_part(int64_t row, const int q, const Params
     return c;
 }
 
-__device__ __forceinline__ void load8(const float* src, float (&f)[8]) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
-    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
-}
-
-// Norm, rotation and stores of one part.  Every lane of the warp must call this together (full-warp shuffles; the
-// eight rows of a warp may be of different kinds): v rows and dead rows simply do not use the result of the math.
+// RMSNorm and rotation of one row over its four lanes, in place.  Lane q holds chunks q, q+4, q+8 and q+12 in w; `weight`
+// points at dim 8q of the norm's weights, c and s hold the cosines and sines of chunks q and q + 4.  Every lane of the
+// warp must call this together (shuffles).
 //
 // The sum of squares keeps one fixed order whatever the lane layout: sixteen partial sums, one per chunk, each taken
 // front to back, then the butterfly p[c] + p[c ^ 8], + [c ^ 4], + [c ^ 2], + [c ^ 1].  With chunks q, q+4, q+8, q+12
 // in one lane the first two levels are local and the last two are shuffles over the row's four lanes.
-__device__ __forceinline__ void finish_part(const Part& ch, const int q, const Params& p) {
-    const int kind = ch.r < p.H ? 0 : (ch.r < p.H + p.KVH ? 1 : 2);
-    const int head = kind == 0 ? ch.r : (kind == 1 ? ch.r - p.H : ch.r - p.H - p.KVH);
-    uint4 out[4];
+__device__ __forceinline__ void norm_rope(uint4 (&w)[4], const float* weight, const uint64_t (&c)[2][4],
+                                          const uint64_t (&s)[2][4], float eps, float one) {
+    uint64_t x[4][4];
+    float pp[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) out[i] = ch.w[i];
-    // a warp whose eight rows are all v rows (or past the end) has nothing to compute: the rows are copied
-    if (!__all_sync(0xffffffffu, kind == 2 || !ch.live)) {
-        float x[4][8], pp[4];
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t u[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+        float ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            unpack8(ch.w[i], x[i]);
-            float ss = __fmul_rn(x[i][0], x[i][0]);
-#pragma unroll
-            for (int e = 1; e < 8; ++e) ss = __fadd_rn(ss, __fmul_rn(x[i][e], x[i][e]));
-            pp[i] = ss;
+        for (int e = 0; e < 4; ++e) {
+            x[i][e] = unpack_bf16(u[e]);
+            float a, b;
+            split(x[i][e], a, b);
+            ss = e == 0 ? __fmul_rn(a, a) : __fadd_rn(ss, __fmul_rn(a, a));
+            ss = __fadd_rn(ss, __fmul_rn(b, b));
         }
-        float ss = __fadd_rn(__fadd_rn(pp[0], pp[2]), __fadd_rn(pp[1], pp[3]));  // levels c ^ 8 and c ^ 4
-        ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, 2));                  // level c ^ 2
-        ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, 1));                  // level c ^ 1
-        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(ss, 1.0f / kD), p.eps)));
-        const float* wgt = kind == 1 ? p.k_weight : p.q_weight;
-        float y[4][8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float ws[8];
-            load8(wgt + (q + 4 * i) * 8, ws);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) y[i][e] = round_bf16(__fmul_rn(__fmul_rn(x[i][e], inv), ws[e]));  // the norm returns bf16
-        }
-        int64_t pos = ch.pos;
-        if (pos < 0) pos = 0;
-        if (pos >= p.max_pos) pos = p.max_pos - 1;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {  // chunk q + 4i holds dims d < 64, its rotation partner d + 64 is chunk q + 4i + 8
-            float c[8], sn[8], lo[8], hi[8];
-            const float* cs = p.cos_sin + pos * kD + (q + 4 * i) * 8;
-            load8(cs, c);
-            load8(cs + 64, sn);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                lo[e] = __fsub_rn(__fmul_rn(y[i][e], c[e]), __fmul_rn(y[i + 2][e], sn[e]));  // x1 cos - x2 sin
-                hi[e] = __fadd_rn(__fmul_rn(y[i + 2][e], c[e]), __fmul_rn(y[i][e], sn[e]));  // x2 cos + x1 sin
-            }
-            out[i] = pack8(lo);
-            out[i + 2] = pack8(hi);
-        }
-        if (kind == 2) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) out[i] = ch.w[i];
-        }
+        pp[i] = ss;
     }
-    if (ch.live && kind != 2) {
-        __nv_bfloat16* dst = kind == 0 ? p.q + (ch.t * p.H + head) * kD : p.k + (ch.t * p.KVH + head) * kD;
+    float ss = __fadd_rn(__fadd_rn(pp[0], pp[2]), __fadd_rn(pp[1], pp[3]));  // levels c ^ 8 and c ^ 4
+    ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, 2));                  // level c ^ 2
+    ss = __fadd_rn(ss, __shfl_xor_sync(0xffffffffu, ss, 1));                  // level c ^ 1
+    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fmul_rn(ss, 1.0f / kD), eps)));
+    const uint64_t inv2 = pair(inv, inv);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(dst + (q + 4 * i) * 8) = out[i];
+    for (int i = 0; i < 4; ++i) {
+        uint64_t ws[4];
+        load_pairs(weight + 32 * i, ws);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[i][e] = unpack_bf16(pack_pair(mul2(mul2(x[i][e], inv2), ws[e])));  // the norm returns bf16
     }
-    if (ch.live && kind != 0 && ch.slot >= 0 && ch.slot < p.num_slots) {
-        __nv_bfloat16* cache = (kind == 1 ? p.k_cache : p.v_cache) + (ch.slot * p.KVH + head) * kD;
+    const uint64_t plus = pair(one, one), minus = pair(-one, -one);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(cache + (q + 4 * i) * 8) = out[i];
+    for (int i = 0; i < 2; ++i) {  // chunk q + 4i holds dims d < 64, its rotation partner d + 64 is chunk q + 4i + 8
+        uint32_t lo[4], hi[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            lo[e] = pack_pair(fma2(mul2(x[i + 2][e], s[i][e]), minus, mul2(x[i][e], c[i][e])));  // x1 cos - x2 sin
+            hi[e] = pack_pair(fma2(mul2(x[i][e], s[i][e]), plus, mul2(x[i + 2][e], c[i][e])));        // x2 cos + x1 sin
+        }
+        w[i] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        w[i + 2] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     }
 }
 
-// The share of block `block` (kThreads threads): rows [block * 64, block * 64 + 64) of the T * (H + 2 KVH) rows, four
-// lanes per row, 64 bytes per lane.
+// Cosines and sines of chunks q and q + 4 at a position (clamped to the table).
+__device__ __forceinline__ void load_rotation(const Params& p, int64_t pos, int q, uint64_t (&c)[2][4], uint64_t (&s)[2][4]) {
+    if (pos < 0) pos = 0;
+    if (pos >= p.max_pos) pos = p.max_pos - 1;
+    const float* cs = p.cos_sin + pos * kD + q * 8;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        load_pairs(cs + 32 * i, c[i]);
+        load_pairs(cs + 32 * i + 64, s[i]);
+    }
+}
+
+// Norm, rotation and stores of one part.  Every lane of the warp must call this together (full-warp shuffles; the
+// eight rows of a warp may be of different kinds): v rows and dead rows simply do not use the result of the math.
+__device__ __forceinline__ void finish_part(const Part& ch, const int q, const Params& p) {
+    const int kind = ch.r < p.H ? 0 : (ch.r < p.H + p.KVH ? 1 : 2);
+    const int head = kind == 0 ? ch.r : (kind == 1 ? ch.r - p.H : ch.r - p.H - p.KVH);
+    uint4 w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = ch.w[i];
+    auto store = [&](__nv_bfloat16* dst) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(dst + (q + 4 * i) * 8) = w[i];
+    };
+    const bool cached = ch.live && kind != 0 && ch.slot >= 0 && ch.slot < p.num_slots;
+    if (kind == 2 && cached) store(p.v_cache + (ch.slot * p.KVH + head) * kD);
+    // a warp whose eight rows are all v rows (or past the end) has nothing to compute
+    if (__all_sync(0xffffffffu, kind == 2 || !ch.live)) return;
+    uint64_t c[2][4], s[2][4];
+    load_rotation(p, ch.pos, q, c, s);
+    norm_rope(w, (kind == 1 ? p.k_weight : p.q_weight) + q * 8, c, s, p.eps, p.one);
+    if (ch.live && kind != 2) store(kind == 0 ? p.q + (ch.t * p.H + head) * kD : p.k + (ch.t * p.KVH + head) * kD);
+    if (kind == 1 && cached) store(p.k_cache + (ch.slot * p.KVH + head) * kD);
+}
+
+// The share of block `block`: kThreads / 4 of the T * (H + 2 KVH) rows, four lanes per row, 64 bytes
+// per lane.
 __device__ __forceinline__ void pre_attention_block(int64_t block, const Params& p) {
     const int q = threadIdx.x & 3;
-    const Part c = load_part(block * kRowsPerBlock + (threadIdx.x >> 2), q, p);
+    const Part c = load_part((block * kThreads + threadIdx.x) >> 2, q, p);
     finish_part(c, q, p);
 }
 
