@@ -237,6 +237,25 @@ int nvllm_b200_paged_prefill(const void* q, const void* k_cache, const void* v_c
                              int NB, int block_size, int MB, float scale, void* stream);
 
 /*
+ * prefill_step: one prefill step of one layer, what Attention.__call__ does with a
+ * prefill context (layers/attention.py:465-480): scatter the step's K/V rows by
+ * slot_mapping (as nvllm_b200_store_kvcache, bf16 rows), then attend -- over the
+ * packed k / v (as nvllm_b200_varlen_prefill, max_seqlen_q >= any length) when
+ * block_tables is NULL, over the pages (as nvllm_b200_paged_prefill) otherwise.
+ * Same results as the two calls.  One call lets the scatter run beside the
+ * attention of packed keys, which does not read the cache.
+ *
+ *   k_cache, v_cache [NB, block_size, KVH, D] bf16;  MB is the width of block_tables
+ */
+int nvllm_b200_prefill_step(const void* q, const void* k, const void* v, void* k_cache,
+                            void* v_cache, const int32_t* slot_mapping,
+                            const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
+                            const int32_t* block_tables, const int32_t* cu_seqlens_q_host,
+                            void* out, void* workspace, size_t workspace_bytes,
+                            int64_t T, int B, int max_seqlen_q, int H, int KVH, int D,
+                            int NB, int block_size, int MB, float scale, void* stream);
+
+/*
  * qk_norm_rope_store: the step a Qwen3 layer runs between its QKV projection and
  * attention, fused into one pass over q, k, v (models/qwen3.py:157-166):
  *     q = q_norm(q); k = k_norm(k)          layers/layernorm.py:31-48 (RMSNorm over head_dim)

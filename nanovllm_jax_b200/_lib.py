@@ -32,6 +32,7 @@ SIGNATURES = {
     "nvllm_b200_varlen_prefill_workspace_bytes": (_sz, [_i64, _i32, _i32, _i32, _i32]),
     "nvllm_b200_varlen_prefill": (_i32, [_vp] * 8 + [_sz, _i64, _i32, _i32, _i32, _i32, _i32, _f32, _vp]),
     "nvllm_b200_paged_prefill": (_i32, [_vp] * 9 + [_sz, _i64] + [_i32] * 8 + [_f32, _vp]),
+    "nvllm_b200_prefill_step": (_i32, [_vp] * 12 + [_sz, _i64] + [_i32] * 8 + [_f32, _vp]),
     "nvllm_b200_device_status_reset": (_i32, []),
     "nvllm_b200_comm_buffer_bytes": (_sz, [_sz]),
     "nvllm_b200_comm_alloc": (_i32, [_sz, _c.POINTER(_vp), _vp]),

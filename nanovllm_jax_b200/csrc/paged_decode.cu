@@ -723,7 +723,7 @@ decode_prepare_kernel(unsigned int* __restrict__ tickets, int num_tickets, int s
     griddep_wait();  // the previous kernel may still be reading these tickets or the cache rows written below
     griddep_launch_dependents();
     if ((int)blockIdx.x < store_blocks) {
-        store_block<SrcT, 1>(blockIdx.x, k, v, k_cache, v_cache, slot_mapping, total_chunks, row_chunks, num_slots);
+        store_block<SrcT, 1>(blockIdx.x, threadIdx.x, k, v, k_cache, v_cache, slot_mapping, total_chunks, row_chunks, num_slots);
     } else {
         const int i = ((int)blockIdx.x - store_blocks) * kStoreThreads + threadIdx.x;
         if (i < num_tickets) tickets[i] = 0u;

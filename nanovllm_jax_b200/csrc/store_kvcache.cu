@@ -15,7 +15,7 @@ store_kvcache_kernel(const SrcT* __restrict__ k, const SrcT* __restrict__ v, __n
                      int row_chunks, int64_t num_slots) {
     griddep_wait();  // k, v and slot_mapping may come from the kernel just before this one
     griddep_launch_dependents();
-    store_block<SrcT>(blockIdx.x, k, v, k_cache, v_cache, slot_mapping, total_chunks, row_chunks, num_slots);
+    store_block<SrcT>(blockIdx.x, threadIdx.x, k, v, k_cache, v_cache, slot_mapping, total_chunks, row_chunks, num_slots);
 }
 
 }  // namespace nvllm

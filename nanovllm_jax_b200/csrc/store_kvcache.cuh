@@ -29,14 +29,14 @@ __device__ __forceinline__ uint4 load_chunk_as_bf16(const float* src, int64_t ch
     return r;
 }
 
-// The share of store block `block` (of kStoreThreads threads): chunks [block*kStoreThreads*kUnroll, +that).
+// The share of thread `tid` of store block `block` (kStoreThreads threads): of chunks [block*kStoreThreads*kUnroll, +that).
 // A slot < 0 is skipped, a slot >= num_slots dropped.
 template <typename SrcT, int kUnroll = kStoreUnroll>
-__device__ __forceinline__ void store_block(int64_t block, const SrcT* __restrict__ k, const SrcT* __restrict__ v,
+__device__ __forceinline__ void store_block(int64_t block, int tid, const SrcT* __restrict__ k, const SrcT* __restrict__ v,
                                             __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                                             const int32_t* __restrict__ slot_mapping, int64_t total_chunks,
                                             int row_chunks, int64_t num_slots) {
-    const int64_t base = block * (kStoreThreads * kUnroll) + threadIdx.x;
+    const int64_t base = block * (kStoreThreads * kUnroll) + tid;
     uint4 kv[kUnroll], vv[kUnroll];
     int64_t dst[kUnroll];
 #pragma unroll
@@ -62,6 +62,16 @@ __device__ __forceinline__ void store_block(int64_t block, const SrcT* __restric
         }
     }
 }
+
+// The K/V scatter of a prefill step as the prefill kernels carry it: bf16 rows, 16-byte chunks.
+struct Scatter {
+    const __nv_bfloat16 *k, *v;
+    __nv_bfloat16 *k_cache, *v_cache;
+    const int32_t* slot_mapping;
+    int64_t chunks;  // T * row_chunks
+    int row_chunks;
+    int64_t num_slots;
+};
 
 inline int64_t store_blocks_for(int64_t total_chunks, int unroll = kStoreUnroll) {
     const int64_t per_block = (int64_t)kStoreThreads * unroll;

@@ -30,6 +30,7 @@ struct Api {
     decltype(&nvllm_b200_varlen_prefill_workspace_bytes) prefill_workspace_bytes;
     decltype(&nvllm_b200_varlen_prefill) varlen_prefill;
     decltype(&nvllm_b200_paged_prefill) paged_prefill;
+    decltype(&nvllm_b200_prefill_step) prefill_step;
     decltype(&nvllm_b200_qk_norm_rope_store) qk_norm_rope_store;
     decltype(&nvllm_b200_fused_decode_step) fused_decode_step;
 } api = {};
@@ -415,6 +416,65 @@ PyObject* paged_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// prefill_step(q, key, value, k_cache, v_cache, slot_mapping, block_tables, cu_seqlens_q, cu_seqlens_k, max_seqlen, scale,
+//              block_size, num_heads, num_kv_heads, cu_seqlens_host)
+// The attention layer's prefill: q comes in the cache's dtype where the keys are read from the pages, and q, key, value are
+// made contiguous.  Returns None, and does nothing, for sources or caches of another kind than bf16 [NB, block, KVH, D].
+PyObject* prefill_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return entry("prefill_step", n, 15, [&]() -> PyObject* {
+        at::Tensor q = tensor(a[0], "q"), key = tensor(a[1], "key"), value = tensor(a[2], "value");
+        const at::Tensor &kc = tensor(a[3], "k_cache"), &vc = tensor(a[4], "v_cache");
+        const bool paged = a[6] != Py_None;
+        const int block_size = to_int(a[11]);
+        if (key.scalar_type() != at::kBFloat16 || kc.scalar_type() != at::kBFloat16 || kc.dim() != 4 || key.dim() != 3 ||
+            kc.size(1) != block_size || kc.size(2) != key.size(1) || kc.size(3) != key.size(2))
+            Py_RETURN_NONE;
+        if (paged && q.scalar_type() != at::kBFloat16) q = q.to(at::kBFloat16);
+        if (!q.is_contiguous()) q = q.contiguous();
+        if (!key.is_contiguous()) key = key.contiguous();
+        if (!value.is_contiguous()) value = value.contiguous();
+        need(q, "q", at::kBFloat16, 3);
+        need(key, "k", at::kBFloat16, 3);
+        need(value, "v", at::kBFloat16, 3);
+        need(kc, "k_cache", at::kBFloat16, 4);
+        need(vc, "v_cache", at::kBFloat16, 4);
+        const at::Tensor& slots = need(a[5], "slot_mapping", at::kInt, 1);
+        const at::Tensor& cu = need(a[7], "cu_seqlens_q", at::kInt, 1);
+        const at::Tensor& cu_k = need(a[8], "cu_seqlens_k", at::kInt, 1);
+        const int max_seqlen = to_int(a[9]);
+        const float scale = to_float(a[10]);
+        const Cache c = paged_cache(kc, vc, q, block_size);
+        const int64_t t = q.size(0);
+        const int h = (int)q.size(1), b = (int)cu.size(0) - 1;
+        if (value.sizes() != key.sizes() || key.size(0) != t)
+            raise(PyExc_ValueError, "k/v shape " + shape_text(key) + " inconsistent with q " + shape_text(q));
+        if ((!paged && h != to_int(a[12])) || c.kvh != to_int(a[13])) raise(PyExc_ValueError, "head counts do not match the tensors");
+        if (slots.size(0) != t)
+            raise(PyExc_ValueError, "slot_mapping has " + std::to_string(slots.size(0)) + " entries for " + std::to_string(t) +
+                                        " tokens");
+        const int32_t* tables = nullptr;
+        int mb = 0;
+        if (paged) {
+            const at::Tensor& bt = need(a[6], "block_tables", at::kInt, 2);
+            if (bt.size(0) != b) raise(PyExc_ValueError, "cu_seqlens_k / block_tables batch mismatch");
+            tables = iptr(bt);
+            mb = (int)bt.size(1);
+        }
+        if (cu_k.size(0) != b + 1) raise(PyExc_ValueError, "cu_seqlens_k / cu_seqlens_q batch mismatch");
+        const HostLengths host(a[14], b + 1);
+        const Site site(q);
+        const at::Tensor out = at::empty_like(q);
+        zero_uncovered(host, b, out, t);
+        const at::Tensor ws = site.scratch(std::max<size_t>(api.prefill_workspace_bytes(t, b, h, c.kvh, c.d), 256));
+        call([&] {
+            return api.prefill_step(ptr(q), ptr(key), ptr(value), mptr(kc), mptr(vc), iptr(slots), iptr(cu), iptr(cu_k), tables,
+                                    host.data, mptr(out), mptr(ws), ws.nbytes(), t, b, max_seqlen, h, c.kvh, c.d, c.nb, c.block,
+                                    mb, scale, site.stream);
+        });
+        return THPVariable_Wrap(out);
+    });
+}
+
 struct PreAttention {
     const at::Tensor &q, &key, &value, &q_weight, &k_weight, &cos_sin, &positions, &slots;
     int64_t t, h, kvh, d;
@@ -562,6 +622,7 @@ PyObject* bind(PyObject*, PyObject* args) {
         {"nvllm_b200_varlen_prefill_workspace_bytes", (void**)&api.prefill_workspace_bytes},
         {"nvllm_b200_varlen_prefill", (void**)&api.varlen_prefill},
         {"nvllm_b200_paged_prefill", (void**)&api.paged_prefill},
+        {"nvllm_b200_prefill_step", (void**)&api.prefill_step},
         {"nvllm_b200_qk_norm_rope_store", (void**)&api.qk_norm_rope_store},
         {"nvllm_b200_fused_decode_step", (void**)&api.fused_decode_step},
     };
@@ -584,6 +645,7 @@ PyMethodDef methods[] = {
     FAST("decode_step", decode_step),
     FAST("varlen_prefill", varlen_prefill),
     FAST("paged_prefill", paged_prefill),
+    FAST("prefill_step", prefill_step),
     FAST("qk_norm_rope_store", qk_norm_rope_store),
     FAST("fused_decode_step", fused_decode_step),
     FAST("workspace", py_workspace),

@@ -9,17 +9,17 @@
 // prefix = len_k - len_q; the model runner attaches the tables on a prefix hit,
 // engine/model_runner.py:311-314).
 //
-// Work item = two 128-row Q tiles (A and B) that share every K/V tile they read.  When
-// the GQA group size is even the two tiles are the same 128 query rows of two q heads of
-// one kv head: both see the same keys, run the same number of K/V tiles and finish
-// together.  Otherwise they are two consecutive row blocks of one head (B then sees one
+// Work item = two 128-row Q tiles (A and B) that share every K/V tile they read: the same 128
+// query rows of two q heads of one kv head -- both see the same keys, run the same number of K/V tiles and finish
+// together -- or, for the last head of an odd group, two consecutive row blocks of it (B then sees one
 // K/V tile more than A).  A tiny plan kernel turns cu_seqlens into the list of
 // (sequence, row block) pairs, longest causal span first; one persistent CTA per SM
-// takes items round-robin from that list (heavy ones first, so the CTAs finish
+// starts on the item of its number and claims the others one by one (heavy ones first, so the CTAs finish
 // together), and the heads of one (sequence, row block) are neighbours in the list so
 // that the G heads of a kv head find each other's K/V tiles in L2.  Tensor memory and
 // barriers are set up once per CTA; the loads of the next item are already in flight
-// while the current one drains.
+// while the current one drains.  A list of at most one item per SM that the host knows travels with the launch instead
+// (ShortParams), and the step's K/V scatter runs on the SMs it leaves.
 //
 // Per CTA (12 warps = 3 warpgroups; the first gives registers away with setmaxnreg, the softmax
 // warpgroups take them):
@@ -35,13 +35,14 @@
 //               issued and all commits of the pair follow the Q.K^T(j+1) MMAs, so nothing
 //               is polled between the two groups of MMAs.  Warp 1 also owns the tensor-
 //               memory allocation (512 columns: S_A S_B O_A O_B).
+//   warp 3      claims the CTA's items and writes their records ahead into shared memory.
 //   warps 4-7   softmax of tile A, warps 8-11 of tile B: one thread per query row holds
 //               its S row (128 scores) in registers, keeps the running max / sum (packed
 //               f32x2 math, 3-input max), writes bf16 P back over S in two halves (each
 //               releases four P.V k-steps) and rescales O only when the max grew by more
 //               than 2^8 (exact: the stale max is carried into the final normalisation).
-//               Tiles strictly above the diagonal are skipped, the diagonal tile is
-//               masked element-wise.  The exponentials of the two tiles take turns
+//               Tiles strictly above the diagonal are skipped; of a diagonal tile each warp
+//               masks the one chunk of 32 keys that its rows' limits fall into and skips the chunks behind it.  The exponentials of the two tiles take turns
 //               (A(0) B(0) A(1) ...): they share the four MUFU pipes, which bound the
 //               kernel, and alternating keeps one tile's MMAs, score loads and row max
 //               running under the other tile's exponentials.
@@ -50,8 +51,9 @@
 // alone together with the poll-free MMA issue order.
 // Every mbarrier wait is bounded; on timeout the CTA raises a device error flag,
 // stops issuing work, and still releases its tensor memory before it exits.
-#include "common.cuh"
+#include "store_kvcache.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -64,29 +66,54 @@ __device__ int g_error_flag = 0;
 
 constexpr int kD = 128;
 constexpr int kTileQ = 128;            // rows per Q tile
-constexpr int kBlockQ = 2 * kTileQ;    // rows per work item when its two Q tiles are row blocks of one head
 constexpr int kTileKV = 128;
 constexpr int kThreads = 384;            // 3 warpgroups: {TMA, MMA, 2 idle warps} | softmax A | softmax B
 constexpr int kPanelBytes = 128 * 128;  // 128 rows x 64 dims bf16, 128B-swizzled
 constexpr int kTileBytes = 2 * kPanelBytes;
 constexpr int kSlots = 5;                // one ring for K and V tiles, filled in the order K0 V0 K1 V1 ...
 constexpr int kSmemTiles = (2 + kSlots) * kTileBytes;  // Q_A Q_B | K/V ring  (224 KB)
-constexpr int kSmemBytes = kSmemTiles + 512 + 1024;
-constexpr int kMaxLevels = 2048;       // row blocks per sequence the plan kernel can rank
+constexpr int kSmemBytes = kSmemTiles + 512 + 1024;  // barriers and item records, alignment slack
+constexpr int kMaxLevels = 4096;       // row blocks per sequence the plan kernel can rank
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
+constexpr int kInlineRecords = 32;     // (sequence, row block) pairs that travel as a kernel argument
+
+// A (sequence, row block) pair, longest causal span first: {first query token of the sequence, its query length, first
+// row of the block, sequence index} and {first key token (packed keys), key length, 0, 0}.
+struct Record {
+    int4 q, k;
+};
+
 struct Params {
-    const int4* items;  // record 0: {number of (sequence, row block) pairs, 0, 0, 0}; then two records per pair, longest
-                        // causal span first: {first query token of the sequence, its query length, first row of the
-                        // block, sequence index} and {first key token (packed keys), key length, 0, 0}
+    const int4* items;  // record 0: {number of pairs, items claimed, 0, 0}; then the two halves of every Record
     const int32_t* block_tables;  // [B, MB] page ids, or nullptr for packed keys/values
     int MB, block_size;
     __nv_bfloat16* out;
     int H, G;
-    int pair_heads;  // 1: an item is 128 rows of heads (2h, 2h+1); 0: 256 rows of one head
+    int per_pair;  // items per (sequence, row block): two heads of one kv head each, a lone head where G is odd
+    int wide;      // out is aligned to 32 bytes
     float scale_log2;
 };
+
+// A short launch (at most one item per SM) carries its records (sorted by the host) and the step's K/V scatter with it: no other kernel runs in front.
+// A kernel of its own, because reading the records from the arguments costs the long launches 3 %.
+struct ShortParams : Params {
+    Record records[kInlineRecords];
+    int pairs;
+    int item_ctas;    // CTAs that take items; the others carry the scatter
+    Scatter scatter;  // chunks = 0: none
+};
+__device__ __forceinline__ Record record_of(const Params& p, int pair) {
+    return Record{__ldg(p.items + 1 + 2 * pair), __ldg(p.items + 2 + 2 * pair)};
+}
+__device__ __forceinline__ Record record_of(const ShortParams& p, int pair) { return p.records[pair]; }
+__device__ __forceinline__ int claim_item(const Params& p) {
+    return (int)gridDim.x + atomicAdd(&const_cast<int4*>(p.items)->y, 1);
+}
+__device__ __forceinline__ int claim_item(const ShortParams& p) { return 0x7fffffff; }  // an item per CTA at most
+__device__ __forceinline__ int pairs_of(const Params& p) { return p.items[0].x; }
+__device__ __forceinline__ int pairs_of(const ShortParams& p) { return p.pairs; }
 
 // ------------------------------------------------------------------------------------------
 // tcgen05 wrappers
@@ -229,11 +256,11 @@ constexpr uint32_t kIdescPV = kIdescQK | (1u << 16);  // B operand MN-major
 // ------------------------------------------------------------------------------------------
 // plan kernel: (sequence, row block) pairs sorted by causal span, largest first
 // ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) prefill_plan_kernel(const int32_t* __restrict__ cu_seqlens,
-                                                            const int32_t* __restrict__ cu_k, int paged, int B,
-                                                            int4* __restrict__ items, int capacity, int bq) {
-    // bq = query rows per block (256, or 128 when an item is two heads).  A row block's weight is its causal span in
-    // bq-key units: level = prefix / bq + block index.
+constexpr int kPlanThreads = 1024;
+__global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_t* __restrict__ cu_seqlens,
+                                                                    const int32_t* __restrict__ cu_k, int paged, int B,
+                                                                    int4* __restrict__ items, int capacity) {
+    // A row block's weight is its causal span in blocks of 128 keys: level = prefix / 128 + block index.
     __shared__ int hist[kMaxLevels];
     __shared__ int base[kMaxLevels];
     __shared__ int max_level, bad;
@@ -242,22 +269,22 @@ __global__ void __launch_bounds__(1024) prefill_plan_kernel(const int32_t* __res
     for (int i = threadIdx.x; i < kMaxLevels; i += blockDim.x) hist[i] = 0;
     if (threadIdx.x == 0) max_level = 0, bad = 0;
     __syncthreads();
-    for (int b = threadIdx.x; b < B; b += blockDim.x) {
+    // few sequences: a warp each, its lanes take the row blocks; many: a thread each
+    const bool by_warp = B <= 256;
+    const int b0 = by_warp ? threadIdx.x >> 5 : threadIdx.x, db = by_warp ? kPlanThreads / 32 : kPlanThreads;
+    const int l0 = by_warp ? threadIdx.x & 31 : 0, dl = by_warp ? 32 : 1;
+    for (int b = b0; b < B; b += db) {
         const int len = cu_seqlens[b + 1] - cu_seqlens[b];
         const int len_k = cu_k[b + 1] - cu_k[b];
         // keys can never be fewer than queries; packed keys sit beside the queries, so the counts must be equal
         if (len > 0 && (len_k < len || (!paged && (len_k != len || cu_k[b] != cu_seqlens[b])))) bad = 1;
-        const int lvl0 = len_k > len ? (len_k - len) / bq : 0;
-        const int n = len > 0 ? (len + bq - 1) / bq : 0;
-        for (int l = 0; l < n; ++l) {
-            int lvl = lvl0 + l;
-            if (lvl >= kMaxLevels) {
-                lvl = kMaxLevels - 1;
-                atomicOr(&g_error_flag, 16);
-            }
-            atomicAdd(&hist[lvl], 1);
-            atomicMax(&max_level, lvl + 1);
+        const int lvl0 = len_k > len ? (len_k - len) / kTileQ : 0;
+        const int n = len > 0 ? (len + kTileQ - 1) / kTileQ : 0;
+        if (n > 0 && l0 == 0) {
+            atomicMax(&max_level, min(lvl0 + n, kMaxLevels));
+            if (lvl0 + n > kMaxLevels) atomicOr(&g_error_flag, 16);
         }
+        for (int l = l0; l < n; l += dl) atomicAdd(&hist[min(lvl0 + l, kMaxLevels - 1)], 1);
     }
     __syncthreads();
     if (bad) {  // uniform: publish an empty list so that the main kernel computes nothing
@@ -267,26 +294,33 @@ __global__ void __launch_bounds__(1024) prefill_plan_kernel(const int32_t* __res
         }
         return;
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {  // base[l] = number of pairs of higher levels: a warp scan from the top, 32 levels at a time
         int run = 0;
-        for (int l = max_level - 1; l >= 0; --l) {
-            base[l] = run;
-            run += hist[l];
+        for (int top = max_level - 1; top >= 0; top -= 32) {
+            const int l = top - (int)threadIdx.x;
+            const int h = l >= 0 ? hist[l] : 0;
+            int incl = h;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)threadIdx.x >= o) incl += v;
+            }
+            if (l >= 0) base[l] = run + incl - h;
+            run += __shfl_sync(0xffffffffu, incl, 31);
         }
-        items[0] = make_int4(run < capacity ? run : capacity, 0, 0, 0);
+        if (threadIdx.x == 0) items[0] = make_int4(run < capacity ? run : capacity, 0, 0, 0);
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < B; b += blockDim.x) {
+    for (int b = b0; b < B; b += db) {
         const int start = cu_seqlens[b];
         const int len = cu_seqlens[b + 1] - start;
         const int len_k = cu_k[b + 1] - cu_k[b];
-        const int lvl0 = len_k > len ? (len_k - len) / bq : 0;
-        const int n = len > 0 ? (len + bq - 1) / bq : 0;
-        for (int l = 0; l < n; ++l) {
-            const int lvl = min(lvl0 + l, kMaxLevels - 1);
-            const int slot = atomicAdd(&base[lvl], 1);
+        const int lvl0 = len_k > len ? (len_k - len) / kTileQ : 0;
+        const int n = len > 0 ? (len + kTileQ - 1) / kTileQ : 0;
+        for (int l = l0; l < n; l += dl) {
+            const int slot = atomicAdd(&base[min(lvl0 + l, kMaxLevels - 1)], 1);
             if (slot < capacity) {
-                items[1 + 2 * slot] = make_int4(start, len, l * bq, b);
+                items[1 + 2 * slot] = make_int4(start, len, l * kTileQ, b);
                 items[2 + 2 * slot] = make_int4(cu_k[b], len_k, 0, 0);
             }
         }
@@ -296,7 +330,19 @@ __global__ void __launch_bounds__(1024) prefill_plan_kernel(const int32_t* __res
 // ------------------------------------------------------------------------------------------
 // main kernel
 // ------------------------------------------------------------------------------------------
+struct Item {
+    int seq_start, len, q0, head;      // first query token of the sequence, query length, first row of the block, first head
+    int k_start, len_k, prefix, kvh;   // first key token (packed keys), key length, len_k - len, kv head
+    int n_a, n_b, n_kv, b;             // KV tiles seen by Q tile A, by Q tile B (0: no such rows; else n_a or n_a + 1), the
+                                       // larger (0: nothing to do; -1: no more items), sequence
+    int dq, dh, ragged, pad;           // Q tile B = rows + dq of head + dh; the last KV tile reaches past the last key
+};
+constexpr int kItemRing = 2;
+constexpr int kItemReaders = 3 + 8;    // TMA producer, two MMA issuers, eight softmax warps
+
 struct Shared {
+    Item items[kItemRing];  // the items of this CTA, written ahead by an otherwise idle warp
+    uint64_t item_full[kItemRing], item_empty[kItemRing];
     uint64_t q_full, q_empty;
     uint64_t kv_full[kSlots], kv_empty[kSlots];
     uint64_t s_full[2], p_full[2][2], o_full[2], o_empty[2];
@@ -304,6 +350,8 @@ struct Shared {
     uint32_t tmem_base;
     volatile int abort_flag;
 };
+
+static_assert(sizeof(Shared) <= 512, "see kSmemBytes");
 
 __device__ __forceinline__ bool wait_or_abort(Shared* sh, uint64_t* bar, uint32_t parity) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -314,38 +362,46 @@ __device__ __forceinline__ bool wait_or_abort(Shared* sh, uint64_t* bar, uint32_
     return false;
 }
 
-struct Item {
-    int seq_start, len, q0, head, b;  // first query token of the sequence, query length, first row of the block
-    int k_start, len_k, prefix;       // first key token (packed keys), key length, len_k - len
-    int dq, dh;          // Q tile B = rows + dq of head + dh
-    int n_a, n_b, n_kv;  // KV tiles seen by Q tile A, by Q tile B (0: no such rows; else n_a or n_a + 1), and the larger
-    bool ragged;         // the last KV tile reaches past the sequence's last key
-};
-
-__device__ __forceinline__ Item load_item(const Params& p, int idx) {
+template <class P>
+__device__ __forceinline__ Item load_item(const P& p, int idx) {
     Item it;
-    const int per_pair = p.pair_heads ? p.H >> 1 : p.H;
-    const int pair = idx / per_pair;
-    it.head = (idx - pair * per_pair) << p.pair_heads;
-    it.dq = p.pair_heads ? 0 : kTileQ;
-    it.dh = p.pair_heads;
-    const int4 r = __ldg(p.items + 1 + 2 * pair), rk = __ldg(p.items + 2 + 2 * pair);
-    it.seq_start = r.x;
-    it.len = r.y;
-    it.q0 = r.z;
-    it.b = r.w;
-    it.k_start = rk.x;
-    it.len_k = rk.y;
+    const int pair = idx / p.per_pair;
+    const int r = idx - pair * p.per_pair;
+    const int per_kv = (p.G + 1) >> 1;      // items per kv head
+    it.kvh = r / per_kv;
+    const int h2 = 2 * (r - it.kvh * per_kv);  // first of the item's heads within the kv head
+    const bool two = h2 + 1 < p.G;
+    it.head = it.kvh * p.G + h2;
+    it.dq = two ? 0 : kTileQ;
+    it.dh = two ? 1 : 0;
+    const Record rec = record_of(p, pair);
+    const int4 q = rec.q, k = rec.k;
+    it.seq_start = q.x;
+    it.len = q.y;
+    it.q0 = q.z;
+    it.b = q.w;
+    it.k_start = k.x;
+    it.len_k = k.y;
     it.prefix = it.len_k - it.len;  // >= 0: the plan kernel publishes no items otherwise
-    const int rows = min(p.pair_heads ? kTileQ : kBlockQ, it.len - it.q0);
     const int nk_total = (it.len_k + kTileKV - 1) / kTileKV;
     // the last row of Q tile x sees keys 0 .. prefix + q0 + 128 x + 127
     it.n_a = min(nk_total, (it.prefix + it.q0 + kTileQ - 1) / kTileKV + 1);
-    it.n_b = p.pair_heads ? it.n_a
-                          : (rows > kTileQ ? min(nk_total, (it.prefix + it.q0 + 2 * kTileQ - 1) / kTileKV + 1) : 0);
+    it.n_b = two ? it.n_a
+                 : (it.len - it.q0 > kTileQ ? min(nk_total, (it.prefix + it.q0 + 2 * kTileQ - 1) / kTileKV + 1) : 0);
+    // a lone head takes two row blocks at a time, on the even ones
+    if (!two && ((it.q0 / kTileQ) & 1)) it.n_a = it.n_b = 0;
     it.n_kv = max(it.n_a, it.n_b);
     it.ragged = it.n_kv * kTileKV > it.len_k;
     return it;
+}
+
+// The next item from the ring (k-th of this CTA).  The readers arrive on the slot once they have their copy, the softmax
+// warps once they are done with the item.
+__device__ __forceinline__ bool next_item(Shared* sh, uint32_t k, Item& it) {
+    const uint32_t slot = k % kItemRing;
+    if (!wait_or_abort(sh, &sh->item_full[slot], (k / kItemRing) & 1u)) return false;
+    it = sh->items[slot];
+    return it.n_kv >= 0;
 }
 
 // First token (row of the k / v tensor map) of KV tile j of the item's sequence.
@@ -355,6 +411,12 @@ __device__ __forceinline__ int kv_tile_token(const Params& p, const Item& it, in
     int page = __ldg(p.block_tables + (size_t)it.b * p.MB + off / p.block_size);
     if (page < 0) page = 0;  // a padding entry: never reached for keys below len_k
     return page * p.block_size + off % p.block_size;  // block_size is a multiple of the tile: a tile never straddles pages
+}
+
+__device__ __forceinline__ void store_32bytes(void* dst, const uint32_t (&w)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
 }
 
 // One 128-column S row -> running max, optional O rescale, bf16 P in two halves.  DIAG: key column c of this tile is
@@ -374,15 +436,19 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
     tmem_ld32(t_s + 96, v[3]);
     tmem_wait_ld();
     float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+    const int warp_lim = lim - (int)(threadIdx.x & 31);  // limit of the warp's first row; the others' follow one by one
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
+        if (DIAG) {
+            if (32 * c > warp_lim + 31) continue;  // nothing of this chunk is visible to any row of the warp
+            if (32 * c + 31 > warp_lim) {          // mask in place so that the second pass needs no select
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    if (c * 32 + i > lim) v[c][i] = 0xFF800000u;
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 32; i += 8) {
-            if (DIAG) {  // mask in place so that the second pass needs no select
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (c * 32 + i + u > lim) v[c][i + u] = 0xFF800000u;
-            }
             mx0 = max3(mx0, __uint_as_float(v[c][i]), __uint_as_float(v[c][i + 1]));
             mx1 = max3(mx1, __uint_as_float(v[c][i + 2]), __uint_as_float(v[c][i + 3]));
             mx2 = max3(mx2, __uint_as_float(v[c][i + 4]), __uint_as_float(v[c][i + 5]));
@@ -421,6 +487,10 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
     uint64_t acc_a = pack2(0.f, 0.f), acc_b = pack2(0.f, 0.f);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
+        if (DIAG && 32 * c > warp_lim + 31) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[c][i] = 0u;
+        } else {
 #pragma unroll
         for (int i = 0; i < 16; i += 2) {
             float x0, x1, x2, x3;
@@ -433,6 +503,7 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
             acc_b = add2(acc_b, pack2(e2, e3));
             v[c][i] = pack_bf16(e0, e1);  // in place: word i <= 2i has been consumed
             v[c][i + 1] = pack_bf16(e2, e3);
+        }
         }
         tmem_st16(t_s + c * 16, v[c]);
         if (c == 3 && turn_out != nullptr) {
@@ -453,9 +524,10 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
     return true;
 }
 
+template <class P>
 __global__ void __launch_bounds__(kThreads, 1)
 varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                      const __grid_constant__ CUtensorMap tm_v, const Params p) {
+                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ P p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sQ = smem;                                   // [2][tile]
@@ -464,7 +536,24 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+    int item_ctas = gridDim.x;
+    if constexpr (std::is_same<P, ShortParams>::value) {
+        item_ctas = p.item_ctas;
+        if ((int)blockIdx.x >= item_ctas) {  // a CTA that only scatters
+            griddep_wait();
+            const Scatter& sc = p.scatter;
+            const int first = (blockIdx.x - item_ctas) * (kThreads / kStoreThreads) + tid / kStoreThreads;
+            if (tid < kThreads / kStoreThreads * kStoreThreads)
+                store_block<__nv_bfloat16>(first, tid % kStoreThreads, sc.k, sc.v, sc.k_cache, sc.v_cache, sc.slot_mapping,
+                                           sc.chunks, sc.row_chunks, sc.num_slots);
+            return;
+        }
+    }
     if (tid == 0) {
+        for (int s = 0; s < kItemRing; ++s) {
+            mbar_init(&sh->item_full[s], 1);
+            mbar_init(&sh->item_empty[s], kItemReaders);
+        }
         mbar_init(&sh->q_full, 1);
         mbar_init(&sh->q_empty, 2);   // both MMA issuers
         for (int s = 0; s < kSlots; ++s) {
@@ -500,20 +589,19 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
     // Register budget: the TMA / MMA warpgroup keeps 96 registers per thread, the two softmax warpgroups take 200
     // (96*128 + 200*256 <= 64K), enough to hold a whole 128-column score row.
-    const int total = (tmem != 0xFFFFFFFFu) ? p.items[0].x * (p.pair_heads ? p.H >> 1 : p.H) : 0;
-    const int first_idx = blockIdx.x, stride = gridDim.x;
+    const int total = (tmem != 0xFFFFFFFFu) ? pairs_of(p) * p.per_pair : 0;
 
     if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
     if (warp == 0) {
         // =============================== TMA producer ===============================
         if (lane == 0) {
-            uint32_t kt = 0;
-            int i = 0;
+            uint32_t kt = 0, i = 0;
             bool ok = true;
-            for (int idx = first_idx; ok && idx < total; idx += stride, ++i) {
-                const Item it = load_item(p, idx);
-                const int kvh = it.head / p.G;
+            Item it;
+            while (ok && next_item(sh, i, it)) {
+                mbar_arrive(&sh->item_empty[i % kItemRing]);
+                const int kvh = it.kvh;
                 const int tok_q = it.seq_start + it.q0;
                 if (i > 0 && !(ok = wait_or_abort(sh, &sh->q_empty, (i - 1) & 1u))) break;
                 mbar_expect_tx(&sh->q_full, (it.n_b > 0 ? 2 : 1) * kTileBytes);
@@ -537,6 +625,32 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     }
                     if (!ok) break;
                 }
+                ++i;
+            }
+        }
+    } else if (warp == 3) {
+        // ============================== item records ================================
+        // The readers would each spend two dependent loads and a division per item between two items.  The first item of a
+        // CTA is fixed, the others are claimed from a counter when the softmax warps start on the item before: with the
+        // heaviest items first the CTAs finish together (dealt round-robin, the CTAs with the heaviest items of every round
+        // also got the ones left over: 257 us for the last of 148, 209 for the median one).
+        if (lane == 0) {
+            uint32_t k = 0;
+            int idx = blockIdx.x;
+            while (true) {
+                const uint32_t slot = k % kItemRing;
+                if (!wait_or_abort(sh, &sh->item_empty[slot], ((k / kItemRing) & 1u) ^ 1u)) break;
+                Item it;
+                do {
+                    if (k > 0 || idx != (int)blockIdx.x) idx = claim_item(p);
+                    it.n_kv = -1;
+                    if (idx < total) it = load_item(p, idx);
+                    if (it.n_kv == 0) idx = total;  // nothing to do there: claim another one
+                } while (it.n_kv == 0);
+                sh->items[slot] = it;
+                mbar_arrive(&sh->item_full[slot]);
+                if (it.n_kv < 0) break;
+                ++k;
             }
         }
     } else if (warp == 1 || warp == 2) {
@@ -558,7 +672,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             uint32_t kt = 0;     // K/V tiles consumed before this item
             uint32_t tiles = 0;  // tiles finished by this Q tile, over all items (barrier phases)
             uint32_t used = 0;   // items in which this Q tile was active (o_empty phases)
-            int i = 0;
+            uint32_t i = 0;      // items
             bool ok = true;
 
             auto issue_qk = [&](uint64_t kd) {
@@ -585,8 +699,9 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             // the slot holding ring position pos: K(j) sits at 2j, V(j) at 2j+1
             auto slot_full = [&](uint32_t pos) { return wait_or_abort(sh, &sh->kv_full[pos % kSlots], (pos / kSlots) & 1u); };
 
-            for (int idx = first_idx; ok && idx < total; idx += stride, ++i) {
-                const Item it = load_item(p, idx);
+            Item it;
+            while (ok && next_item(sh, i, it)) {
+                mbar_arrive(&sh->item_empty[i % kItemRing]);
                 const int n_x = x == 0 ? it.n_a : it.n_b;
                 if (!(ok = wait_or_abort(sh, &sh->q_full, i & 1u))) break;
                 if (n_x == 0) mbar_arrive(&sh->q_empty);  // this tile never reads the Q buffer of this item
@@ -629,6 +744,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 }
                 used += n_x > 0 ? 1 : 0;
                 kt += it.n_kv;
+                ++i;
             }
         }
     }
@@ -650,12 +766,16 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         uint32_t turns_seen = 0;  // completions of the other tile's turn barrier this warp has consumed
         uint32_t kt = 0;          // K/V tiles of the items before this one (ring positions)
         bool ok = true;
-        for (int idx = first_idx; ok && idx < total; idx += stride) {
-            const Item it = load_item(p, idx);
+        Item it;
+        for (uint32_t k = 0; ok && next_item(sh, k, it); ++k) {
             const int n_x = x == 0 ? it.n_a : it.n_b;
             const uint32_t kt0 = kt;
             kt += it.n_kv;
-            if (n_x == 0) continue;
+            if (n_x == 0) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh->item_empty[k % kItemRing]);
+                continue;
+            }
             const bool both = it.n_b > 0;
             const int q_pos = it.q0 + x * it.dq + row;             // row of the sequence's query block
             const int first_lim = it.prefix + it.q0 + x * it.dq;  // last key visible to the first row of this Q tile
@@ -720,7 +840,16 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 uint32_t ov[32];
                 tmem_ld32(t_o + c * 32, ov);
                 tmem_wait_ld();
-                if (q_pos < it.len) {
+                if (q_pos < it.len && p.wide) {  // whole sectors: half the store instructions
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        uint32_t w[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            w[e] = pack_bf16(__uint_as_float(ov[16 * i + 2 * e]) * inv, __uint_as_float(ov[16 * i + 2 * e + 1]) * inv);
+                        store_32bytes(orow + c * 32 + i * 16, w);
+                    }
+                } else if (q_pos < it.len) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         uint4 w;
@@ -734,7 +863,10 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->o_empty[x]);
+            if (lane == 0) {
+                mbar_arrive(&sh->o_empty[x]);
+                mbar_arrive(&sh->item_empty[k % kItemRing]);  // only now: the next claim waits for it
+            }
         }
     }
 
@@ -753,6 +885,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 static int make_map(CUtensorMap* map, const void* base, int heads, int64_t tokens) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return fail(NVLLM_B200_EDRIVER, "cuTensorMapEncodeTiled entry point not available");
+    // a panel of 64 dims per load: both panels in one load (the half as a fourth dimension) were 1 % slower
     cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)heads, (cuuint64_t)tokens};
     cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)heads * kD * 2};
     cuuint32_t box[3] = {64, 1, 128};
@@ -771,20 +904,30 @@ static int ensure_attr() {
     NVLLM_CUDA_OK(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(mu);
     if (dev >= 0 && dev < 64 && !done[dev]) {
-        NVLLM_CUDA_OK(
-            cudaFuncSetAttribute(varlen_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        NVLLM_CUDA_OK(cudaFuncSetAttribute(varlen_prefill_kernel<Params>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kSmemBytes));
+        NVLLM_CUDA_OK(cudaFuncSetAttribute(varlen_prefill_kernel<ShortParams>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         done[dev] = true;
     }
     return NVLLM_B200_OK;
 }
 
-static int64_t item_capacity(int64_t T, int B) { return T / kTileQ + B + 1; }  // covers 128-row blocks
+static int check_pages(const char* who, int NB, int block_size) {
+    if (block_size <= 0 || block_size % kTileKV != 0)
+        return fail(NVLLM_B200_EUNSUPPORTED, "%s: block_size %d (must be a multiple of %d)", who, block_size, kTileKV);
+    if (NB <= 0) return fail(NVLLM_B200_EINVAL, "%s: NB must be positive", who);
+    return NVLLM_B200_OK;
+}
+
+static int64_t item_capacity(int64_t T, int B) { return T / kTileQ + B + 1; }
 
 // Common launcher.  kv_tokens: extent of the token axis of k / v (T for packed tensors, the slot count of the cache).
+// sc (may be null): the step's K/V scatter.
 static int launch(const char* who, const void* q, const void* k, const void* v, int64_t kv_tokens,
                   const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, const int32_t* block_tables, int MB,
                   int block_size, const int32_t* cu_seqlens_host, void* out, void* workspace, size_t workspace_bytes,
-                  int64_t T, int B, int max_seqlen, int H, int KVH, int D, float scale, void* stream) {
+                  int64_t T, int B, int max_seqlen, int H, int KVH, int D, float scale, const Scatter* sc, void* stream) {
     if (T < 0 || B < 0 || H <= 0 || KVH <= 0)
         return fail(NVLLM_B200_EINVAL, "%s: bad size (T=%lld B=%d H=%d KVH=%d)", who, (long long)T, B, H, KVH);
     if (D != kD) return fail(NVLLM_B200_EUNSUPPORTED, "%s: head_dim %d (only 128)", who, D);
@@ -793,7 +936,14 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     if (T > 0x7fffffffLL || kv_tokens > 0x7fffffffLL)
         return fail(NVLLM_B200_EUNSUPPORTED, "%s: more than 2^31-1 tokens", who);
     if (!(scale > 0.f)) return fail(NVLLM_B200_EINVAL, "%s: scale must be positive", who);
-    if (T == 0 || B == 0) return NVLLM_B200_OK;
+    if (T == 0) return NVLLM_B200_OK;
+    const bool scatter = sc && sc->chunks > 0 && sc->num_slots > 0;
+    auto scatter_only = [&]() -> int {  // no sequence to attend to: the rows are stored all the same
+        return !scatter ? NVLLM_B200_OK
+                        : nvllm_b200_store_kvcache(sc->k, sc->v, sc->k_cache, sc->v_cache, sc->slot_mapping, T, KVH, D,
+                                                   sc->num_slots, NVLLM_B200_DTYPE_BF16, stream);
+    };
+    if (B == 0) return scatter_only();
     if (!q || !k || !v || !cu_seqlens_q || !cu_seqlens_k || !out) return fail(NVLLM_B200_EINVAL, "%s: null pointer", who);
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15)
         return fail(NVLLM_B200_EINVAL, "%s: q/k/v/out must be 16-byte aligned", who);
@@ -802,33 +952,33 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
         return fail(NVLLM_B200_EWORKSPACE, "%s: workspace of %zu bytes required, got %zu", who, need,
                     workspace ? workspace_bytes : (size_t)0);
 
-    // Two q heads of one kv head make an item when there are such pairs: both Q tiles then see the same number of K/V
-    // tiles and finish together.  Otherwise an item is 256 rows of one head.
-    const int pair_heads = ((H / KVH) % 2 == 0) ? 1 : 0;
-    const int bq = pair_heads ? kTileQ : kBlockQ;
-    const int per_pair = pair_heads ? H / 2 : H;
+    ShortParams p;
     // Upper bound of (sequence, row block) pairs: exact from the host copy of cu_seqlens, else from max_seqlen.
-    int64_t pairs = 0;
     const int64_t cap = item_capacity(T, B);
+    int64_t pairs = 0;
     if (cu_seqlens_host) {
         for (int b = 0; b < B; ++b) {
             const int64_t len = (int64_t)cu_seqlens_host[b + 1] - cu_seqlens_host[b];
             if (len < 0 || cu_seqlens_host[b + 1] > T)
                 return fail(NVLLM_B200_EINVAL, "%s: cu_seqlens_host is not a non-decreasing prefix of T", who);
-            if (len > (int64_t)kMaxLevels * bq)
+            if (len > (int64_t)kMaxLevels * kTileQ)
                 return fail(NVLLM_B200_EUNSUPPORTED, "%s: sequence of %lld tokens (max %d)", who, (long long)len,
-                            kMaxLevels * bq);
-            pairs += (len + bq - 1) / bq;
+                            kMaxLevels * kTileQ);
+            pairs += (len + kTileQ - 1) / kTileQ;
         }
     } else {
         if (max_seqlen <= 0) return fail(NVLLM_B200_EINVAL, "%s: max_seqlen must be positive", who);
-        if (max_seqlen > kMaxLevels * bq)
-            return fail(NVLLM_B200_EUNSUPPORTED, "%s: max_seqlen %d (max %d)", who, max_seqlen, kMaxLevels * bq);
-        pairs = (int64_t)B * ((max_seqlen + bq - 1) / bq);
+        if (max_seqlen > kMaxLevels * kTileQ)
+            return fail(NVLLM_B200_EUNSUPPORTED, "%s: max_seqlen %d (max %d)", who, max_seqlen, kMaxLevels * kTileQ);
+        pairs = (int64_t)B * ((max_seqlen + kTileQ - 1) / kTileQ);
     }
     if (pairs > cap) pairs = cap;
-    if (pairs == 0) return NVLLM_B200_OK;
-    if (pairs * per_pair > 0x7fffffffLL) return fail(NVLLM_B200_EUNSUPPORTED, "%s: grid too large", who);
+    if (pairs == 0) return scatter_only();
+    const int G = H / KVH;
+    // Two q heads of one kv head make an item: both Q tiles then see the same number of K/V tiles and finish together.  Where
+    // the group size is odd its last head goes alone, 256 rows at a time.
+    p.per_pair = KVH * ((G + 1) / 2);
+    if (pairs * p.per_pair > 0x7fffffffLL) return fail(NVLLM_B200_EUNSUPPORTED, "%s: grid too large", who);
 
     int rc = ensure_attr();
     if (rc) return rc;
@@ -837,34 +987,64 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     if ((rc = make_map(&tm_k, k, KVH, kv_tokens))) return rc;
     if ((rc = make_map(&tm_v, v, KVH, kv_tokens))) return rc;
 
-    Params p;
     p.items = (const int4*)workspace;
+    p.pairs = 0;
     p.block_tables = block_tables;
     p.MB = MB;
     p.block_size = block_size;
     p.out = (__nv_bfloat16*)out;
     p.H = H;
-    p.G = H / KVH;
-    p.pair_heads = pair_heads;
+    p.G = G;
+    p.wide = ((uintptr_t)out & 31) == 0;
     p.scale_log2 = scale * 1.4426950408889634f;
+    p.scatter = Scatter{};
+    const int sms = sm_count();
+    int ctas = p.item_ctas = (int)std::min<int64_t>(pairs * p.per_pair, sms);
+
+    // A short list known to the host (and nothing for the plan kernel to check on the device) travels with the launch, and
+    // the scatter, where SMs are left, with it.  Elsewhere the scatter is a launch of its own: on the idle warp of the
+    // attention CTAs it slowed them by as much as it took (power and issue slots).
+    const bool brief = cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q && pairs <= kInlineRecords &&
+                       pairs * p.per_pair <= sms;
+    if (brief) {
+        for (int b = 0; b < B; ++b) {
+            const int start = cu_seqlens_host[b], len = cu_seqlens_host[b + 1] - start;
+            for (int l = 0; l < len; l += kTileQ)
+                p.records[p.pairs++] = Record{make_int4(start, len, l, b), make_int4(start, len, 0, 0)};
+        }
+        std::stable_sort(p.records, p.records + p.pairs, [](const Record& a, const Record& b) { return a.q.z > b.q.z; });
+    }
+    if (scatter) {
+        const int64_t blocks = (store_blocks_for(sc->chunks) + kThreads / kStoreThreads - 1) / (kThreads / kStoreThreads);
+        if (brief && ctas + blocks <= sms) {
+            p.scatter = *sc;
+            ctas += (int)blocks;
+        } else if ((rc = scatter_only())) {
+            return rc;
+        }
+    }
 
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1);
-    cfg.blockDim = dim3(1024);
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, prefill_plan_kernel, cu_seqlens_q, cu_seqlens_k, block_tables ? 1 : 0, B,
-                                     (int4*)workspace, (int)cap, bq));
-    const int64_t ctas = pairs * per_pair < (int64_t)sm_count() ? pairs * per_pair : (int64_t)sm_count();
+    if (!brief) {
+        cfg.gridDim = dim3(1);
+        cfg.blockDim = dim3(kPlanThreads);
+        NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, prefill_plan_kernel, cu_seqlens_q, cu_seqlens_k, block_tables ? 1 : 0, B,
+                                         (int4*)workspace, (int)cap));
+    }
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
-    NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, varlen_prefill_kernel, tm_q, tm_k, tm_v, p));
+    if (brief)
+        NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, varlen_prefill_kernel<ShortParams>, tm_q, tm_k, tm_v, p));
+    else
+        NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, varlen_prefill_kernel<Params>, tm_q, tm_k, tm_v, (const Params&)p));
     return NVLLM_B200_OK;
 }
 
@@ -898,7 +1078,7 @@ extern "C" int nvllm_b200_varlen_prefill(const void* q, const void* k, const voi
     // cu_seqlens_q, which the plan kernel checks on the device
     return nvllm::prefill::launch("varlen_prefill", q, k, v, T, cu_seqlens_q, cu_seqlens_k, nullptr, 0, 0,
                                   cu_seqlens_host, out, workspace, workspace_bytes, T, B, max_seqlen, H, KVH, D, scale,
-                                  stream);
+                                  nullptr, stream);
 }
 
 extern "C" int nvllm_b200_paged_prefill(const void* q, const void* k_cache, const void* v_cache,
@@ -909,11 +1089,36 @@ extern "C" int nvllm_b200_paged_prefill(const void* q, const void* k_cache, cons
                                         void* stream) {
     using namespace nvllm;
     if (!block_tables || MB <= 0) return fail(NVLLM_B200_EINVAL, "paged_prefill: block_tables required");
-    if (block_size <= 0 || block_size % prefill::kTileKV != 0)
-        return fail(NVLLM_B200_EUNSUPPORTED, "paged_prefill: block_size %d (must be a multiple of %d)", block_size,
-                    prefill::kTileKV);
-    if (NB <= 0) return fail(NVLLM_B200_EINVAL, "paged_prefill: NB must be positive");
+    int rc = prefill::check_pages("paged_prefill", NB, block_size);
+    if (rc) return rc;
     return prefill::launch("paged_prefill", q, k_cache, v_cache, (int64_t)NB * block_size, cu_seqlens_q, cu_seqlens_k,
                            block_tables, MB, block_size, cu_seqlens_q_host, out, workspace, workspace_bytes, T, B,
-                           max_seqlen_q, H, KVH, D, scale, stream);
+                           max_seqlen_q, H, KVH, D, scale, nullptr, stream);
+}
+
+extern "C" int nvllm_b200_prefill_step(const void* q, const void* k, const void* v, void* k_cache, void* v_cache,
+                                       const int32_t* slot_mapping, const int32_t* cu_seqlens_q,
+                                       const int32_t* cu_seqlens_k, const int32_t* block_tables,
+                                       const int32_t* cu_seqlens_q_host, void* out, void* workspace,
+                                       size_t workspace_bytes, int64_t T, int B, int max_seqlen_q, int H, int KVH, int D,
+                                       int NB, int block_size, int MB, float scale, void* stream) {
+    using namespace nvllm;
+    const char* who = "prefill_step";
+    if (T < 0 || KVH <= 0 || NB <= 0 || block_size <= 0 || (block_tables && MB <= 0))
+        return fail(NVLLM_B200_EINVAL, "%s: bad size (T=%lld KVH=%d NB=%d block=%d MB=%d)", who, (long long)T, KVH, NB,
+                    block_size, MB);
+    if (D != prefill::kD) return fail(NVLLM_B200_EUNSUPPORTED, "%s: head_dim %d (only 128)", who, D);
+    if (T == 0) return NVLLM_B200_OK;
+    if (!k || !v || !k_cache || !v_cache || !slot_mapping) return fail(NVLLM_B200_EINVAL, "%s: null pointer", who);
+    if (((uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15)
+        return fail(NVLLM_B200_EINVAL, "%s: k/v and caches must be 16-byte aligned", who);
+    int rc = block_tables ? prefill::check_pages(who, NB, block_size) : NVLLM_B200_OK;
+    if (rc) return rc;
+    const int row_chunks = KVH * D / 8;
+    const int64_t num_slots = (int64_t)NB * block_size;
+    const Scatter sc = {(const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache,
+                        slot_mapping, T * row_chunks, row_chunks, num_slots};
+    return prefill::launch(who, q, block_tables ? k_cache : k, block_tables ? v_cache : v, block_tables ? num_slots : T,
+                           cu_seqlens_q, cu_seqlens_k, block_tables, MB, block_size, cu_seqlens_q_host, out, workspace,
+                           workspace_bytes, T, B, max_seqlen_q, H, KVH, D, scale, &sc, stream);
 }

@@ -125,6 +125,14 @@ class Attention:
                                               context.block_tables, context.context_lens, self.scale, self.block_size,
                                               None, True)
         if self.k_cache is not None and self.v_cache is not None:
+            # prefill: one C call too, which lets the scatter run beside the attention of packed keys
+            if context.block_tables is not None or context.max_seqlen_k == context.max_seqlen_q:
+                out = _lib.binding().prefill_step(
+                    q, k, v, self.k_cache, self.v_cache, context.slot_mapping, context.block_tables, context.cu_seqlens_q,
+                    context.cu_seqlens_k, context.max_seqlen_q, self.scale, self.block_size, self.num_heads,
+                    self.num_kv_heads, ops._host_lengths(getattr(context, "cu_seqlens_host", None)))
+                if out is not None:
+                    return out
             num_blocks = self.k_cache.shape[0]
             flat = (num_blocks * self.block_size, self.num_kv_heads, self.head_dim)
             store_kv_to_cache(k, v, self.k_cache.view(flat), self.v_cache.view(flat), context.slot_mapping)
