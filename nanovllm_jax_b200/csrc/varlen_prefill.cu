@@ -259,13 +259,20 @@ constexpr uint32_t kIdescPV = kIdescQK | (1u << 16);  // B operand MN-major
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_t* __restrict__ cu_seqlens,
                                                                     const int32_t* __restrict__ cu_k, int paged, int B,
-                                                                    int4* __restrict__ items, int capacity) {
+                                                                    int4* __restrict__ items, int capacity,
+                                                                    int behind_store) {
     // A row block's weight is its causal span in blocks of 128 keys: level = prefix / 128 + block index.
     __shared__ int hist[kMaxLevels];
     __shared__ int base[kMaxLevels];
     __shared__ int max_level, bad;
-    griddep_wait();
-    griddep_launch_dependents();
+    // Behind this step's own scatter there is nothing to wait for: that kernel has let this one go after everything in front
+    // of it was complete, and writes nothing that is read here.  The wait at the end makes the main kernel's wait cover it.
+    // Only then may the main kernel start: its CTAs dealt to SMs in the order in which the scatter left them, instead of in
+    // order, cost long launches 1 to 3 % (neighbouring CTAs read the same K/V tiles).
+    if (!behind_store) {
+        griddep_wait();
+        griddep_launch_dependents();
+    }
     for (int i = threadIdx.x; i < kMaxLevels; i += blockDim.x) hist[i] = 0;
     if (threadIdx.x == 0) max_level = 0, bad = 0;
     __syncthreads();
@@ -292,6 +299,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
             items[0] = make_int4(0, 0, 0, 0);
             atomicOr(&g_error_flag, 32);
         }
+        if (behind_store) griddep_wait();
         return;
     }
     if (threadIdx.x < 32) {  // base[l] = number of pairs of higher levels: a warp scan from the top, 32 levels at a time
@@ -325,6 +333,10 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
             }
         }
     }
+    if (behind_store) {
+        griddep_wait();
+        griddep_launch_dependents();
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -337,6 +349,8 @@ struct Item {
                                        // larger (0: nothing to do; -1: no more items), sequence
     int dq, dh, ragged, pad;           // Q tile B = rows + dq of head + dh; the last KV tile reaches past the last key
 };
+constexpr int kNoTurnTiles = 2;        // items of so few K/V tiles do without the turns of the two softmax warpgroups: the
+                                       // second tile's wait is not won back there (48 short prompts: 42.4 -> 39.9 us)
 constexpr int kItemRing = 2;
 constexpr int kItemReaders = 3 + 8;    // TMA producer, two MMA issuers, eight softmax warps
 
@@ -776,15 +790,15 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 if (lane == 0) mbar_arrive(&sh->item_empty[k % kItemRing]);
                 continue;
             }
-            const bool both = it.n_b > 0;
+            const bool both = it.n_b > 0 && it.n_kv > kNoTurnTiles;  // the two tiles take turns
             const int q_pos = it.q0 + x * it.dq + row;             // row of the sequence's query block
             const int first_lim = it.prefix + it.q0 + x * it.dq;  // last key visible to the first row of this Q tile
             float m_run = -INFINITY, m_used = -INFINITY, l = 0.f;
             // One KV tile of this Q tile.  Tiles whose last key the tile's first row may still see need no mask; the
             // one or two after them (one when the prefix is a multiple of the tile) are masked per element.  The two
             // kinds run in two separate loops so that each loop body is straight-line code.
-            auto tile_step = [&](const int j, auto diag) -> bool {
-                constexpr bool kDiag = decltype(diag)::value;
+            auto tile_step = [&](const int j, auto kind) -> bool {
+                constexpr bool kDiag = decltype(kind)::value == 1, kDead = decltype(kind)::value == 2;
                 if (!wait_or_abort(sh, &sh->s_full[x], tiles & 1u)) return false;
                 // A(j) starts after B(j-1); B(j) starts after A(j) while A still has tiles.
                 uint64_t* turn_bar = nullptr;
@@ -794,7 +808,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     ++turns_seen;
                 }
                 tc_fence_after();
-                if (kDiag && it.ragged && j == it.n_kv - 1) {
+                if ((kDiag || kDead) && it.ragged && j == it.n_kv - 1) {
                     // The last KV tile of the sequence reaches past its last key: those rows of the V tile hold
                     // whatever follows in memory (the next sequence, padding, recycled cache rows).  Their
                     // probabilities are exactly zero, but 0 * NaN or 0 * Inf in the P.V product would still poison the
@@ -817,6 +831,18 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         fence_proxy_async_smem();  // generic-proxy stores must be visible to the tensor core's reads
                     }
                 }
+                if constexpr (kDead) {  // nothing but the hand-overs: P and O of these rows may hold anything
+                    if (turn_bar != nullptr && !wait_or_abort(sh, turn_bar, turn_parity)) return false;
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (both && (x == 0 || j + 1 < it.n_a)) mbar_arrive(&sh->turn[x]);
+                        mbar_arrive(&sh->p_full[x][0]);
+                        mbar_arrive(&sh->p_full[x][1]);
+                    }
+                    ++tiles;
+                    return true;
+                }
                 if (!softmax_tile<kDiag>(sh, x, t_s, t_o, kDiag ? first_lim - j * kTileKV + row : 0, j == 0,
                                          (tiles - 1) & 1u, p.scale_log2, m_run, m_used, l, turn_bar, turn_parity,
                                          (both && (x == 0 || j + 1 < it.n_a)) ? &sh->turn[x] : nullptr))
@@ -827,8 +853,13 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             };
             const int n_plain = min(n_x, (first_lim + 1) / kTileKV);  // tiles j with j * 128 + 127 <= first_lim
             int j = 0;
-            for (; ok && j < n_plain; ++j) ok = tile_step(j, std::false_type{});
-            for (; ok && j < n_x; ++j) ok = tile_step(j, std::true_type{});
+            const bool dead = q_pos - lane >= it.len;  // the whole warp lies behind the sequence's last row
+            if (dead) {
+                for (; ok && j < n_x; ++j) ok = tile_step(j, std::integral_constant<int, 2>{});
+            } else {
+                for (; ok && j < n_plain; ++j) ok = tile_step(j, std::integral_constant<int, 0>{});
+                for (; ok && j < n_x; ++j) ok = tile_step(j, std::integral_constant<int, 1>{});
+            }
             if (!ok) break;
             // ---- epilogue: O / l -> bf16 -> global, then hand O back to the MMA thread ----
             if (!(ok = wait_or_abort(sh, &sh->o_full[x], (tiles - 1) & 1u))) break;
@@ -837,6 +868,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             __nv_bfloat16* orow = p.out + ((size_t)(it.seq_start + q_pos) * p.H + it.head + x * it.dh) * kD;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
+                if (dead) break;
                 uint32_t ov[32];
                 tmem_ld32(t_o + c * 32, ov);
                 tmem_wait_ld();
@@ -1036,7 +1068,7 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
         cfg.gridDim = dim3(1);
         cfg.blockDim = dim3(kPlanThreads);
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, prefill_plan_kernel, cu_seqlens_q, cu_seqlens_k, block_tables ? 1 : 0, B,
-                                         (int4*)workspace, (int)cap));
+                                         (int4*)workspace, (int)cap, scatter && pdl_enabled() ? 1 : 0));
     }
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(kThreads);
