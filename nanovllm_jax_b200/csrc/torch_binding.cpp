@@ -107,14 +107,20 @@ float to_float(PyObject* o) {
 
 // One scratch buffer per (device, stream), grown on demand: calls on one stream are ordered, so they may share it.  At
 // most kMaxWorkspaces buffers are kept; the one used longest ago goes back to torch's allocator first (it was allocated
-// on its own stream, so the allocator hands it out again only behind that stream's work).  Used under the GIL.
+// on its own stream, so the allocator hands it out again only behind that stream's work).  A buffer that a stream capture
+// has seen is never given back: the graph refers to it for as long as it may be replayed.  Used under the GIL.
 struct Workspace {
     int device;
     cudaStream_t stream;
     uint64_t used;
+    bool captured;
     at::Tensor buf;
 };
 constexpr size_t kMaxWorkspaces = 64;
+std::vector<at::Tensor>& captured_buffers() {
+    static auto* list = new std::vector<at::Tensor>();
+    return *list;
+}
 std::vector<Workspace>& workspaces() {
     static auto* list = new std::vector<Workspace>();  // never destroyed: the allocator may be gone at exit
     return *list;
@@ -134,7 +140,7 @@ const at::Tensor& workspace(int device, cudaStream_t stream, size_t nbytes) {
         at::Tensor buf = at::empty({n}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
         if (!w) {
             if (list.size() < kMaxWorkspaces) {
-                list.push_back({});
+                list.push_back(Workspace{});
                 w = &list.back();
             } else {
                 w = &list[0];
@@ -142,11 +148,18 @@ const at::Tensor& workspace(int device, cudaStream_t stream, size_t nbytes) {
                     if (e.used < w->used) w = &e;
             }
         }
+        if (w->captured) captured_buffers().push_back(w->buf);
         w->device = device;
         w->stream = stream;
+        w->captured = false;
         w->buf = std::move(buf);
     }
     w->used = ++workspace_clock;
+    if (!w->captured) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) (void)cudaGetLastError();
+        w->captured = status != cudaStreamCaptureStatusNone;
+    }
     return w->buf;
 }
 
@@ -564,7 +577,7 @@ int32_t as_i32(PyObject* o) {
     int overflow = 0;
     long v = PyLong_CheckExact(o) ? PyLong_AsLongAndOverflow(o, &overflow) : -1;
     if (!PyLong_CheckExact(o)) {
-        PyObject* i = PyNumber_Index(o);  // numpy integers
+        PyObject* i = PyNumber_Long(o);  // numpy and tensor scalars
         if (!i) throw Raised();
         v = PyLong_AsLongAndOverflow(i, &overflow);
         Py_DECREF(i);
