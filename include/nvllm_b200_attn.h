@@ -168,7 +168,8 @@ int nvllm_b200_paged_decode_static(const void* q, const void* k_cache, const voi
  */
 int nvllm_b200_device_status(int* flags_host);
 
-/* Bytes of scratch nvllm_b200_varlen_prefill needs (may be 0). */
+/* Bytes of scratch nvllm_b200_varlen_prefill, _paged_prefill and _prefill_step need.  256-byte aligned scratch lets them
+ * cut few items with many keys into runs on several SMs (16-byte aligned scratch will do otherwise). */
 size_t nvllm_b200_varlen_prefill_workspace_bytes(int64_t T, int B, int H, int KVH, int D);
 
 /*

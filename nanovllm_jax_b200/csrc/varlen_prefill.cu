@@ -19,7 +19,8 @@
 // that the G heads of a kv head find each other's K/V tiles in L2.  Tensor memory and
 // barriers are set up once per CTA; the loads of the next item are already in flight
 // while the current one drains.  A list of at most one item per SM that the host knows travels with the launch instead
-// (ShortParams), and the step's K/V scatter runs on the SMs it leaves.
+// (ShortParams), and the step's K/V scatter runs on the SMs it leaves.  Few items with many keys are cut into runs of
+// K/V tiles (SplitParams) that a small kernel behind this one combines.
 //
 // Per CTA (12 warps = 3 warpgroups; the first gives registers away with setmaxnreg, the softmax
 // warpgroups take them):
@@ -104,6 +105,23 @@ struct ShortParams : Params {
     int item_ctas;    // CTAs that take items; the others carry the scatter
     Scatter scatter;  // chunks = 0: none
 };
+// Few items with many keys each (a short question behind a long cached conversation): the K/V tiles of an item are cut into
+// up to `splits` contiguous runs, one per CTA, which leave partial results that prefill_combine_kernel puts together.
+struct SplitParams : Params {
+    float* partials;  // [CTA][Q tile][kPartialFloats]
+    int splits;
+};
+constexpr int kPartialFloats = kTileQ * kD + 2 * kTileQ;  // O[128][128] relative to m, then m[128] (log2 units) and l[128]
+constexpr int kMinRun = 4;  // tiles per run: at least one of them is visible to every row (at most two or three are masked)
+// Items of fewer tiles stay whole: they take less time than the partial results and the combining launch (about 6 us).  The
+// rule looks at an item's own tiles, so that packed keys and keys in pages give the same bits.
+// 100 new tokens behind 8000 cached ones: 130 -> 42 us with 32 / 8 heads, 33 with 8 / 1; one prompt of 4000 tokens, 4 / 1
+// heads: 63 -> 50, of 1200 (ten tiles), 8 / 2: 25 -> 28 if it were cut.
+constexpr int kSplitTiles = 12;
+__device__ __forceinline__ int runs_of(const SplitParams& p, int n_a) {
+    return n_a < kSplitTiles ? 1 : min(p.splits, n_a / kMinRun);
+}
+
 __device__ __forceinline__ Record record_of(const Params& p, int pair) {
     return Record{__ldg(p.items + 1 + 2 * pair), __ldg(p.items + 2 + 2 * pair)};
 }
@@ -112,8 +130,10 @@ __device__ __forceinline__ int claim_item(const Params& p) {
     return (int)gridDim.x + atomicAdd(&const_cast<int4*>(p.items)->y, 1);
 }
 __device__ __forceinline__ int claim_item(const ShortParams& p) { return 0x7fffffff; }  // an item per CTA at most
-__device__ __forceinline__ int pairs_of(const Params& p) { return p.items[0].x; }
-__device__ __forceinline__ int pairs_of(const ShortParams& p) { return p.pairs; }
+__device__ __forceinline__ int claim_item(const SplitParams& p) { return 0x7fffffff; }
+__device__ __forceinline__ int items_of(const Params& p) { return p.items[0].x * p.per_pair; }
+__device__ __forceinline__ int items_of(const ShortParams& p) { return p.pairs * p.per_pair; }
+__device__ __forceinline__ int items_of(const SplitParams& p) { return p.items[0].x * p.per_pair * p.splits; }
 
 // ------------------------------------------------------------------------------------------
 // tcgen05 wrappers
@@ -347,7 +367,8 @@ struct Item {
     int k_start, len_k, prefix, kvh;   // first key token (packed keys), key length, len_k - len, kv head
     int n_a, n_b, n_kv, b;             // KV tiles seen by Q tile A, by Q tile B (0: no such rows; else n_a or n_a + 1), the
                                        // larger (0: nothing to do; -1: no more items), sequence
-    int dq, dh, ragged, pad;           // Q tile B = rows + dq of head + dh; the last KV tile reaches past the last key
+    int dq, dh, ragged, kv0;           // Q tile B = rows + dq of head + dh; the last KV tile reaches past the last key; a run
+                                       // of a split item: its first KV tile (len_k and prefix count from there on), else -1
 };
 constexpr int kNoTurnTiles = 2;        // items of so few K/V tiles do without the turns of the two softmax warpgroups: the
                                        // second tile's wait is not won back there (48 short prompts: 42.4 -> 39.9 us)
@@ -406,6 +427,29 @@ __device__ __forceinline__ Item load_item(const P& p, int idx) {
     if (!two && ((it.q0 / kTileQ) & 1)) it.n_a = it.n_b = 0;
     it.n_kv = max(it.n_a, it.n_b);
     it.ragged = it.n_kv * kTileKV > it.len_k;
+    it.kv0 = -1;
+    return it;
+}
+__device__ __forceinline__ Item load_item(const SplitParams& p, int idx) {
+    const int c = idx % p.splits;
+    Item it = load_item<Params>(p, idx / p.splits);
+    const int runs = runs_of(p, it.n_a);
+    if (runs == 1) {
+        if (c > 0) it.n_a = it.n_b = it.n_kv = 0;
+        return it;
+    }
+    if (c >= runs) {
+        it.n_a = it.n_b = it.n_kv = 0;
+        return it;
+    }
+    const int j0 = it.n_a * c / runs, j1 = c + 1 == runs ? it.n_kv : it.n_a * (c + 1) / runs;
+    it.kv0 = j0;
+    it.n_a = min(it.n_a, j1) - j0;
+    it.n_b = it.n_b > 0 ? min(it.n_b, j1) - j0 : 0;
+    it.n_kv = j1 - j0;
+    it.len_k -= j0 * kTileKV;
+    it.prefix -= j0 * kTileKV;
+    it.ragged = it.n_kv * kTileKV > it.len_k;
     return it;
 }
 
@@ -420,7 +464,7 @@ __device__ __forceinline__ bool next_item(Shared* sh, uint32_t k, Item& it) {
 
 // First token (row of the k / v tensor map) of KV tile j of the item's sequence.
 __device__ __forceinline__ int kv_tile_token(const Params& p, const Item& it, int j) {
-    const int off = j * kTileKV;
+    const int off = (max(it.kv0, 0) + j) * kTileKV;
     if (p.block_tables == nullptr) return it.k_start + off;
     int page = __ldg(p.block_tables + (size_t)it.b * p.MB + off / p.block_size);
     if (page < 0) page = 0;  // a padding entry: never reached for keys below len_k
@@ -603,7 +647,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
     // Register budget: the TMA / MMA warpgroup keeps 96 registers per thread, the two softmax warpgroups take 200
     // (96*128 + 200*256 <= 64K), enough to hold a whole 128-column score row.
-    const int total = (tmem != 0xFFFFFFFFu) ? pairs_of(p) * p.per_pair : 0;
+    const int total = (tmem != 0xFFFFFFFFu) ? items_of(p) : 0;
 
     if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
@@ -864,6 +908,32 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             // ---- epilogue: O / l -> bf16 -> global, then hand O back to the MMA thread ----
             if (!(ok = wait_or_abort(sh, &sh->o_full[x], (tiles - 1) & 1u))) break;
             tc_fence_after();
+            if constexpr (std::is_same<P, SplitParams>::value) {
+                if (it.kv0 >= 0) {  // a run of a split item: its O, maximum and sum as they are
+                    float* part = p.partials + ((size_t)blockIdx.x * 2 + x) * kPartialFloats;
+                    if (!dead) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            uint32_t ov[32];
+                            tmem_ld32(t_o + c * 32, ov);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                *reinterpret_cast<uint4*>(part + row * kD + c * 32 + i * 4) =
+                                    make_uint4(ov[4 * i], ov[4 * i + 1], ov[4 * i + 2], ov[4 * i + 3]);
+                        }
+                        part[kTileQ * kD + row] = m_used * p.scale_log2;
+                        part[kTileQ * kD + kTileQ + row] = l;
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&sh->o_empty[x]);
+                        mbar_arrive(&sh->item_empty[k % kItemRing]);
+                    }
+                    continue;
+                }
+            }
             const float inv = 1.0f / l;
             __nv_bfloat16* orow = p.out + ((size_t)(it.seq_start + q_pos) * p.H + it.head + x * it.dh) * kD;
 #pragma unroll
@@ -911,6 +981,41 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
 }
 
+// Puts the runs of split items together: block (item, Q tile, group of 8 rows), thread t owns row t / 16 of the group and
+// dims 8 (t % 16) .. + 7.  Latency-bound (the partials are in L2): the maxima of all runs first, then four runs at a time.
+constexpr int kCombineThreads = 128;
+__global__ void __launch_bounds__(kCombineThreads) prefill_combine_kernel(const __grid_constant__ SplitParams p) {
+    griddep_wait();
+    const int e = blockIdx.x, x = blockIdx.y, row = blockIdx.z * 8 + (threadIdx.x >> 4), c8 = (threadIdx.x & 15) * 8;
+    if (e >= p.items[0].x * p.per_pair) return;
+    const Item it = load_item<Params>(p, e);
+    const int runs = runs_of(p, it.n_a);
+    const int q_pos = it.q0 + x * it.dq + row;
+    if ((x == 0 ? it.n_a : it.n_b) == 0 || runs == 1 || q_pos >= it.len) return;
+    const float* part = p.partials + ((size_t)e * p.splits * 2 + x) * kPartialFloats;
+    constexpr size_t kNext = 2 * kPartialFloats;
+    float m = -INFINITY;
+    for (int c = 0; c < runs; ++c) m = fmaxf(m, __ldcg(part + c * kNext + kTileQ * kD + row));
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, l = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < runs; ++c) {
+        const float* q = part + c * kNext;
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(q + row * kD + c8));
+        const float4 b = __ldcg(reinterpret_cast<const float4*>(q + row * kD + c8) + 1);
+        const float f = fast_exp2(__ldcg(q + kTileQ * kD + row) - m);
+        l += __ldcg(q + kTileQ * kD + kTileQ + row) * f;
+        acc[0] += a.x * f, acc[1] += a.y * f, acc[2] += a.z * f, acc[3] += a.w * f;
+        acc[4] += b.x * f, acc[5] += b.y * f, acc[6] += b.z * f, acc[7] += b.w * f;
+    }
+    const float inv = 1.0f / l;
+    uint4 w;
+    w.x = pack_bf16(acc[0] * inv, acc[1] * inv);
+    w.y = pack_bf16(acc[2] * inv, acc[3] * inv);
+    w.z = pack_bf16(acc[4] * inv, acc[5] * inv);
+    w.w = pack_bf16(acc[6] * inv, acc[7] * inv);
+    *reinterpret_cast<uint4*>(p.out + ((size_t)(it.seq_start + q_pos) * p.H + it.head + x * it.dh) * kD + c8) = w;
+}
+
 // ------------------------------------------------------------------------------------------
 // host
 // ------------------------------------------------------------------------------------------
@@ -938,6 +1043,8 @@ static int ensure_attr() {
     if (dev >= 0 && dev < 64 && !done[dev]) {
         NVLLM_CUDA_OK(cudaFuncSetAttribute(varlen_prefill_kernel<Params>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            kSmemBytes));
+        NVLLM_CUDA_OK(cudaFuncSetAttribute(varlen_prefill_kernel<SplitParams>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         NVLLM_CUDA_OK(cudaFuncSetAttribute(varlen_prefill_kernel<ShortParams>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         done[dev] = true;
@@ -953,6 +1060,15 @@ static int check_pages(const char* who, int NB, int block_size) {
 }
 
 static int64_t item_capacity(int64_t T, int B) { return T / kTileQ + B + 1; }
+static size_t list_bytes(int64_t T, int B) { return ((size_t)(2 * item_capacity(T, B) + 1) * 16 + 255) & ~size_t(255); }
+
+// Runs per item: as many as leave one run per SM; 1 where no item can have enough tiles.
+constexpr int kMaxSplits = 16;
+static int splits_for(int64_t items, int64_t max_tiles, int sms) {
+    if (items <= 0 || 2 * items > sms || max_tiles < kSplitTiles) return 1;
+    return (int)std::min<int64_t>(std::min<int64_t>(sms / items, kMaxSplits), max_tiles / kMinRun);
+}
+static size_t partials_bytes(int sms) { return (size_t)sms * 2 * kPartialFloats * 4; }
 
 // Common launcher.  kv_tokens: extent of the token axis of k / v (T for packed tensors, the slot count of the cache).
 // sc (may be null): the step's K/V scatter.
@@ -979,7 +1095,7 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     if (!q || !k || !v || !cu_seqlens_q || !cu_seqlens_k || !out) return fail(NVLLM_B200_EINVAL, "%s: null pointer", who);
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15)
         return fail(NVLLM_B200_EINVAL, "%s: q/k/v/out must be 16-byte aligned", who);
-    const size_t need = nvllm_b200_varlen_prefill_workspace_bytes(T, B, H, KVH, D);
+    const size_t need = list_bytes(T, B);  // the rest of what is asked for lets items be split
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15))
         return fail(NVLLM_B200_EWORKSPACE, "%s: workspace of %zu bytes required, got %zu", who, need,
                     workspace ? workspace_bytes : (size_t)0);
@@ -987,8 +1103,9 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     ShortParams p;
     // Upper bound of (sequence, row block) pairs: exact from the host copy of cu_seqlens, else from max_seqlen.
     const int64_t cap = item_capacity(T, B);
-    int64_t pairs = 0;
+    int64_t pairs = 0, longest = max_seqlen;
     if (cu_seqlens_host) {
+        longest = 0;
         for (int b = 0; b < B; ++b) {
             const int64_t len = (int64_t)cu_seqlens_host[b + 1] - cu_seqlens_host[b];
             if (len < 0 || cu_seqlens_host[b + 1] > T)
@@ -997,6 +1114,7 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
                 return fail(NVLLM_B200_EUNSUPPORTED, "%s: sequence of %lld tokens (max %d)", who, (long long)len,
                             kMaxLevels * kTileQ);
             pairs += (len + kTileQ - 1) / kTileQ;
+            longest = std::max(longest, len);
         }
     } else {
         if (max_seqlen <= 0) return fail(NVLLM_B200_EINVAL, "%s: max_seqlen must be positive", who);
@@ -1036,7 +1154,12 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     // A short list known to the host (and nothing for the plan kernel to check on the device) travels with the launch, and
     // the scatter, where SMs are left, with it.  Elsewhere the scatter is a launch of its own: on the idle warp of the
     // attention CTAs it slowed them by as much as it took (power and issue slots).
-    const bool brief = cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q && pairs <= kInlineRecords &&
+    const int64_t max_tiles = block_tables ? (int64_t)MB * block_size / kTileKV : (longest + kTileKV - 1) / kTileKV;
+    const size_t lists = list_bytes(T, B);
+    const int splits = workspace_bytes >= lists + partials_bytes(sms) && ((uintptr_t)workspace & 255) == 0
+                           ? splits_for(pairs * p.per_pair, max_tiles, sms)
+                           : 1;
+    const bool brief = splits == 1 && cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q && pairs <= kInlineRecords &&
                        pairs * p.per_pair <= sms;
     if (brief) {
         for (int b = 0; b < B; ++b) {
@@ -1073,7 +1196,18 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
-    if (brief)
+    if (splits > 1) {
+        SplitParams sp;
+        static_cast<Params&>(sp) = p;
+        sp.partials = (float*)((uint8_t*)workspace + lists);
+        sp.splits = splits;
+        cfg.gridDim = dim3((unsigned)(pairs * p.per_pair * splits));
+        NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, varlen_prefill_kernel<SplitParams>, tm_q, tm_k, tm_v, sp));
+        cfg.gridDim = dim3((unsigned)(pairs * p.per_pair), 2, kTileQ / 8);
+        cfg.blockDim = dim3(kCombineThreads);
+        cfg.dynamicSmemBytes = 0;
+        NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, prefill_combine_kernel, sp));
+    } else if (brief)
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, varlen_prefill_kernel<ShortParams>, tm_q, tm_k, tm_v, p));
     else
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, varlen_prefill_kernel<Params>, tm_q, tm_k, tm_v, (const Params&)p));
@@ -1094,12 +1228,17 @@ int clear_prefill_flags() {
 }  // namespace nvllm
 
 extern "C" size_t nvllm_b200_varlen_prefill_workspace_bytes(int64_t T, int B, int H, int KVH, int D) {
-    (void)H;
-    (void)KVH;
+    using namespace nvllm;
+    using namespace nvllm::prefill;
     (void)D;
     if (T < 0 || B < 0) return 256;
-    const size_t n = (size_t)(2 * nvllm::prefill::item_capacity(T, B) + 1) * 16;
-    return (n + 255) & ~size_t(255);
+    size_t n = list_bytes(T, B);
+    if (H > 0 && KVH > 0 && H % KVH == 0) {
+        // room for the partial results of split items where so few items are possible
+        const int64_t blocks = std::max<int64_t>((T + kTileQ - 1) / kTileQ, B), per_pair = (int64_t)KVH * ((H / KVH + 1) / 2);
+        if (2 * blocks * per_pair <= sm_count()) n += partials_bytes(sm_count());
+    }
+    return n;
 }
 
 extern "C" int nvllm_b200_varlen_prefill(const void* q, const void* k, const void* v, const int32_t* cu_seqlens_q,
