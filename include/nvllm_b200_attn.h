@@ -187,7 +187,11 @@ size_t nvllm_b200_varlen_prefill_workspace_bytes(int64_t T, int B, int H, int KV
  *                 device status is raised -- a prompt with a cached prefix goes
  *                 to nvllm_b200_paged_prefill.  cu_seqlens_host, if
  *                 not NULL, is a host copy of cu_seqlens_q that lets the library
- *                 size its grid without reading device memory
+ *                 size its grid without reading device memory.  Only that: the
+ *                 lengths are the device's, so a captured call follows them when
+ *                 they are rewritten between replays (B and T stay), also where
+ *                 that makes more row blocks than the host copy had.  A host copy
+ *                 without any token enqueues no attention
  *   max_seqlen    upper bound of any sequence length (used for grid sizing when
  *                 cu_seqlens_host is NULL)
  *
@@ -225,7 +229,8 @@ int nvllm_b200_varlen_prefill(const void* q, const void* k, const void* v,
  *                 len_k >= len_q for every sequence, else nothing is computed and
  *                 bit 5 (32) of the device status is raised
  *   block_tables  [B, MB] int32, -1 padded
- *   cu_seqlens_q_host  optional host copy of cu_seqlens_q (exact grid sizing)
+ *   cu_seqlens_q_host  optional host copy of cu_seqlens_q: sizes the grid, no more
+ *                 (as in nvllm_b200_varlen_prefill)
  *   workspace     >= nvllm_b200_varlen_prefill_workspace_bytes(T, B, H, KVH, D)
  *
  * Cache rows at positions >= len_k are never used, whatever they hold.

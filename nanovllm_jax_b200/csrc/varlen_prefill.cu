@@ -18,8 +18,8 @@
 // together), and the heads of one (sequence, row block) are neighbours in the list so
 // that the G heads of a kv head find each other's K/V tiles in L2.  Tensor memory and
 // barriers are set up once per CTA; the loads of the next item are already in flight
-// while the current one drains.  A list of at most one item per SM that the host knows travels with the launch instead
-// (ShortParams), and the step's K/V scatter runs on the SMs it leaves.  Few items with many keys are cut into runs of
+// while the current one drains.  Where the host knows that there is at most one item per SM, every CTA finds its own from
+// cu_seqlens instead (ShortParams), and the step's K/V scatter runs on the SMs the items leave.  Few items with many keys are cut into runs of
 // K/V tiles (SplitParams) that a small kernel behind this one combines.
 //
 // Per CTA (12 warps = 3 warpgroups; the first gives registers away with setmaxnreg, the softmax
@@ -78,7 +78,8 @@ constexpr int kMaxLevels = 4096;       // row blocks per sequence the plan kerne
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
-constexpr int kInlineRecords = 32;     // (sequence, row block) pairs that travel as a kernel argument
+constexpr int kShortBlocks = 32;       // a short launch has at most so many row blocks ...
+constexpr int kShortSequences = 32;    // ... of so many sequences: a lane of a warp for each
 
 // A (sequence, row block) pair, longest causal span first: {first query token of the sequence, its query length, first
 // row of the block, sequence index} and {first key token (packed keys), key length, 0, 0}.
@@ -97,11 +98,13 @@ struct Params {
     float scale_log2;
 };
 
-// A short launch (at most one item per SM) carries its records (sorted by the host) and the step's K/V scatter with it: no other kernel runs in front.
-// A kernel of its own, because reading the records from the arguments costs the long launches 3 %.
+// A short launch (at most one item per SM, as far as the host knows) runs without a plan kernel and carries the step's K/V
+// scatter: every CTA finds its item in the device's cu_seqlens (one load latency and a few warp votes; records laid out by the
+// host and passed as arguments were 0.4 us faster, 8.5 against 8.9 us for one prompt of 87 tokens, but a captured launch then
+// kept the lengths of its capture).  Should the lengths make more items than CTAs by then, a CTA takes several.
 struct ShortParams : Params {
-    Record records[kInlineRecords];
-    int pairs;
+    const int32_t* cu_seqlens;
+    int B;
     int item_ctas;    // CTAs that take items; the others carry the scatter
     Scatter scatter;  // chunks = 0: none
 };
@@ -125,14 +128,11 @@ __device__ __forceinline__ int runs_of(const SplitParams& p, int n_a) {
 __device__ __forceinline__ Record record_of(const Params& p, int pair) {
     return Record{__ldg(p.items + 1 + 2 * pair), __ldg(p.items + 2 + 2 * pair)};
 }
-__device__ __forceinline__ Record record_of(const ShortParams& p, int pair) { return p.records[pair]; }
 __device__ __forceinline__ int claim_item(const Params& p) {
     return (int)gridDim.x + atomicAdd(&const_cast<int4*>(p.items)->y, 1);
 }
-__device__ __forceinline__ int claim_item(const ShortParams& p) { return 0x7fffffff; }  // an item per CTA at most
 __device__ __forceinline__ int claim_item(const SplitParams& p) { return 0x7fffffff; }
 __device__ __forceinline__ int items_of(const Params& p) { return p.items[0].x * p.per_pair; }
-__device__ __forceinline__ int items_of(const ShortParams& p) { return p.pairs * p.per_pair; }
 __device__ __forceinline__ int items_of(const SplitParams& p) { return p.items[0].x * p.per_pair * p.splits; }
 
 // ------------------------------------------------------------------------------------------
@@ -397,11 +397,9 @@ __device__ __forceinline__ bool wait_or_abort(Shared* sh, uint64_t* bar, uint32_
     return false;
 }
 
-template <class P>
-__device__ __forceinline__ Item load_item(const P& p, int idx) {
+// Item r (of per_pair) of a (sequence, row block).
+__device__ __forceinline__ Item make_item(const Params& p, const Record& rec, int r) {
     Item it;
-    const int pair = idx / p.per_pair;
-    const int r = idx - pair * p.per_pair;
     const int per_kv = (p.G + 1) >> 1;      // items per kv head
     it.kvh = r / per_kv;
     const int h2 = 2 * (r - it.kvh * per_kv);  // first of the item's heads within the kv head
@@ -409,7 +407,6 @@ __device__ __forceinline__ Item load_item(const P& p, int idx) {
     it.head = it.kvh * p.G + h2;
     it.dq = two ? 0 : kTileQ;
     it.dh = two ? 1 : 0;
-    const Record rec = record_of(p, pair);
     const int4 q = rec.q, k = rec.k;
     it.seq_start = q.x;
     it.len = q.y;
@@ -430,9 +427,13 @@ __device__ __forceinline__ Item load_item(const P& p, int idx) {
     it.kv0 = -1;
     return it;
 }
+__device__ __forceinline__ Item load_item(const Params& p, int idx) {
+    const int pair = idx / p.per_pair;
+    return make_item(p, record_of(p, pair), idx - pair * p.per_pair);
+}
 __device__ __forceinline__ Item load_item(const SplitParams& p, int idx) {
     const int c = idx % p.splits;
-    Item it = load_item<Params>(p, idx / p.splits);
+    Item it = load_item(static_cast<const Params&>(p), idx / p.splits);
     const int runs = runs_of(p, it.n_a);
     if (runs == 1) {
         if (c > 0) it.n_a = it.n_b = it.n_kv = 0;
@@ -594,13 +595,12 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    int item_ctas = gridDim.x;
-    if constexpr (std::is_same<P, ShortParams>::value) {
-        item_ctas = p.item_ctas;
-        if ((int)blockIdx.x >= item_ctas) {  // a CTA that only scatters
+    constexpr bool kShort = std::is_same<P, ShortParams>::value;
+    if constexpr (kShort) {
+        if ((int)blockIdx.x >= p.item_ctas) {  // a CTA that only scatters
             griddep_wait();
             const Scatter& sc = p.scatter;
-            const int first = (blockIdx.x - item_ctas) * (kThreads / kStoreThreads) + tid / kStoreThreads;
+            const int first = (blockIdx.x - p.item_ctas) * (kThreads / kStoreThreads) + tid / kStoreThreads;
             if (tid < kThreads / kStoreThreads * kStoreThreads)
                 store_block<__nv_bfloat16>(first, tid % kStoreThreads, sc.k, sc.v, sc.k_cache, sc.v_cache, sc.slot_mapping,
                                            sc.chunks, sc.row_chunks, sc.num_slots);
@@ -647,7 +647,8 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
     // Register budget: the TMA / MMA warpgroup keeps 96 registers per thread, the two softmax warpgroups take 200
     // (96*128 + 200*256 <= 64K), enough to hold a whole 128-column score row.
-    const int total = (tmem != 0xFFFFFFFFu) ? items_of(p) : 0;
+    int total = 0;
+    if constexpr (!kShort) total = (tmem != 0xFFFFFFFFu) ? items_of(p) : 0;
 
     if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
@@ -692,7 +693,43 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // CTA is fixed, the others are claimed from a counter when the softmax warps start on the item before: with the
         // heaviest items first the CTAs finish together (dealt round-robin, the CTAs with the heaviest items of every round
         // also got the ones left over: 257 us for the last of 148, 209 for the median one).
-        if (lane == 0) {
+        if constexpr (kShort) {
+            // Lane b has sequence b.  Items go by row block, the last ones (the longest spans) first.
+            const int start = lane < p.B ? __ldg(p.cu_seqlens + lane) : 0;
+            const int len = lane < p.B ? __ldg(p.cu_seqlens + lane + 1) - start : 0;
+            const int blocks = len > 0 ? (len + kTileQ - 1) / kTileQ : 0;
+            const int items = tmem != 0xFFFFFFFFu ? __reduce_add_sync(0xffffffffu, blocks) * p.per_pair : 0;
+            const int levels = __reduce_max_sync(0xffffffffu, blocks);
+            uint32_t k = 0;
+            for (int idx = blockIdx.x, more = 1; more; idx += p.item_ctas) {
+                int at = idx / p.per_pair, level = levels - 1;
+                const int r = idx - at * p.per_pair;
+                int4 q = make_int4(0, 0, 0, 0);
+                if (idx < items) {
+                    uint32_t has = __ballot_sync(0xffffffffu, blocks > level);
+                    for (; at >= __popc(has); has = __ballot_sync(0xffffffffu, blocks > level)) at -= __popc(has), --level;
+                    const bool mine = blocks > level && __popc(has & ((1u << lane) - 1)) == at;
+                    const int b = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+                    q = make_int4(__shfl_sync(0xffffffffu, start, b), __shfl_sync(0xffffffffu, len, b), level * kTileQ, b);
+                }
+                if (lane == 0) {
+                    Item it;
+                    it.n_kv = -1;
+                    if (idx < items) it = make_item(p, Record{q, make_int4(q.x, q.y, 0, 0)}, r);
+                    if (it.n_kv != 0) {
+                        const uint32_t slot = k % kItemRing;
+                        more = wait_or_abort(sh, &sh->item_empty[slot], ((k / kItemRing) & 1u) ^ 1u);
+                        if (more) {
+                            sh->items[slot] = it;
+                            mbar_arrive(&sh->item_full[slot]);
+                            ++k;
+                            more = it.n_kv > 0;
+                        }
+                    }
+                }
+                more = __shfl_sync(0xffffffffu, more, 0);
+            }
+        } else if (lane == 0) {
             uint32_t k = 0;
             int idx = blockIdx.x;
             while (true) {
@@ -988,7 +1025,7 @@ __global__ void __launch_bounds__(kCombineThreads) prefill_combine_kernel(const 
     griddep_wait();
     const int e = blockIdx.x, x = blockIdx.y, row = blockIdx.z * 8 + (threadIdx.x >> 4), c8 = (threadIdx.x & 15) * 8;
     if (e >= p.items[0].x * p.per_pair) return;
-    const Item it = load_item<Params>(p, e);
+    const Item it = load_item(static_cast<const Params&>(p), e);
     const int runs = runs_of(p, it.n_a);
     const int q_pos = it.q0 + x * it.dq + row;
     if ((x == 0 ? it.n_a : it.n_b) == 0 || runs == 1 || q_pos >= it.len) return;
@@ -1138,7 +1175,8 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     if ((rc = make_map(&tm_v, v, KVH, kv_tokens))) return rc;
 
     p.items = (const int4*)workspace;
-    p.pairs = 0;
+    p.cu_seqlens = cu_seqlens_q;
+    p.B = B;
     p.block_tables = block_tables;
     p.MB = MB;
     p.block_size = block_size;
@@ -1151,24 +1189,16 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     const int sms = sm_count();
     int ctas = p.item_ctas = (int)std::min<int64_t>(pairs * p.per_pair, sms);
 
-    // A short list known to the host (and nothing for the plan kernel to check on the device) travels with the launch, and
-    // the scatter, where SMs are left, with it.  Elsewhere the scatter is a launch of its own: on the idle warp of the
+    // A short list known to the host (and nothing for the plan kernel to check on the device) needs no plan kernel, and
+    // the scatter, where SMs are left, goes with the launch.  Elsewhere the scatter is a launch of its own: on the idle warp of the
     // attention CTAs it slowed them by as much as it took (power and issue slots).
     const int64_t max_tiles = block_tables ? (int64_t)MB * block_size / kTileKV : (longest + kTileKV - 1) / kTileKV;
     const size_t lists = list_bytes(T, B);
     const int splits = workspace_bytes >= lists + partials_bytes(sms) && ((uintptr_t)workspace & 255) == 0
                            ? splits_for(pairs * p.per_pair, max_tiles, sms)
                            : 1;
-    const bool brief = splits == 1 && cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q && pairs <= kInlineRecords &&
-                       pairs * p.per_pair <= sms;
-    if (brief) {
-        for (int b = 0; b < B; ++b) {
-            const int start = cu_seqlens_host[b], len = cu_seqlens_host[b + 1] - start;
-            for (int l = 0; l < len; l += kTileQ)
-                p.records[p.pairs++] = Record{make_int4(start, len, l, b), make_int4(start, len, 0, 0)};
-        }
-        std::stable_sort(p.records, p.records + p.pairs, [](const Record& a, const Record& b) { return a.q.z > b.q.z; });
-    }
+    const bool brief = splits == 1 && cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q &&
+                       B <= kShortSequences && pairs <= kShortBlocks && pairs * p.per_pair <= sms;
     if (scatter) {
         const int64_t blocks = (store_blocks_for(sc->chunks) + kThreads / kStoreThreads - 1) / (kThreads / kStoreThreads);
         if (brief && ctas + blocks <= sms) {
