@@ -113,6 +113,7 @@ struct ShortParams : Params {
 struct SplitParams : Params {
     float* partials;  // [CTA][Q tile][kPartialFloats]
     int splits;
+    int ctas;  // the launch's
 };
 constexpr int kPartialFloats = kTileQ * kD + 2 * kTileQ;  // O[128][128] relative to m, then m[128] (log2 units) and l[128]
 constexpr int kMinRun = 4;  // tiles per run: at least one of them is visible to every row (at most two or three are masked)
@@ -121,9 +122,12 @@ constexpr int kMinRun = 4;  // tiles per run: at least one of them is visible to
 // 100 new tokens behind 8000 cached ones: 130 -> 42 us with 32 / 8 heads, 33 with 8 / 1; one prompt of 4000 tokens, 4 / 1
 // heads: 63 -> 50, of 1200 (ten tiles), 8 / 2: 25 -> 28 if it were cut.
 constexpr int kSplitTiles = 12;
-__device__ __forceinline__ int runs_of(const SplitParams& p, int n_a) {
-    return n_a < kSplitTiles ? 1 : min(p.splits, n_a / kMinRun);
+// The launch has a CTA for every run that the host could foresee.  Where the device's lengths make more items than that (a
+// captured launch whose lengths were rewritten), the items stay whole and the CTAs claim them one by one.
+__device__ __forceinline__ int splits_of(const SplitParams& p) {
+    return (long long)p.items[0].x * p.per_pair * p.splits <= p.ctas ? p.splits : 1;
 }
+__device__ __forceinline__ int runs_of(int splits, int n_a) { return n_a < kSplitTiles ? 1 : min(splits, n_a / kMinRun); }
 
 __device__ __forceinline__ Record record_of(const Params& p, int pair) {
     return Record{__ldg(p.items + 1 + 2 * pair), __ldg(p.items + 2 + 2 * pair)};
@@ -131,9 +135,8 @@ __device__ __forceinline__ Record record_of(const Params& p, int pair) {
 __device__ __forceinline__ int claim_item(const Params& p) {
     return (int)gridDim.x + atomicAdd(&const_cast<int4*>(p.items)->y, 1);
 }
-__device__ __forceinline__ int claim_item(const SplitParams& p) { return 0x7fffffff; }
 __device__ __forceinline__ int items_of(const Params& p) { return p.items[0].x * p.per_pair; }
-__device__ __forceinline__ int items_of(const SplitParams& p) { return p.items[0].x * p.per_pair * p.splits; }
+__device__ __forceinline__ int items_of(const SplitParams& p) { return p.items[0].x * p.per_pair * splits_of(p); }
 
 // ------------------------------------------------------------------------------------------
 // tcgen05 wrappers
@@ -432,9 +435,9 @@ __device__ __forceinline__ Item load_item(const Params& p, int idx) {
     return make_item(p, record_of(p, pair), idx - pair * p.per_pair);
 }
 __device__ __forceinline__ Item load_item(const SplitParams& p, int idx) {
-    const int c = idx % p.splits;
-    Item it = load_item(static_cast<const Params&>(p), idx / p.splits);
-    const int runs = runs_of(p, it.n_a);
+    const int splits = splits_of(p), c = idx % splits;
+    Item it = load_item(static_cast<const Params&>(p), idx / splits);
+    const int runs = runs_of(splits, it.n_a);
     if (runs == 1) {
         if (c > 0) it.n_a = it.n_b = it.n_kv = 0;
         return it;
@@ -1024,9 +1027,9 @@ constexpr int kCombineThreads = 128;
 __global__ void __launch_bounds__(kCombineThreads) prefill_combine_kernel(const __grid_constant__ SplitParams p) {
     griddep_wait();
     const int e = blockIdx.x, x = blockIdx.y, row = blockIdx.z * 8 + (threadIdx.x >> 4), c8 = (threadIdx.x & 15) * 8;
-    if (e >= p.items[0].x * p.per_pair) return;
+    if (e >= p.items[0].x * p.per_pair || splits_of(p) == 1) return;
     const Item it = load_item(static_cast<const Params&>(p), e);
-    const int runs = runs_of(p, it.n_a);
+    const int runs = runs_of(p.splits, it.n_a);
     const int q_pos = it.q0 + x * it.dq + row;
     if ((x == 0 ? it.n_a : it.n_b) == 0 || runs == 1 || q_pos >= it.len) return;
     const float* part = p.partials + ((size_t)e * p.splits * 2 + x) * kPartialFloats;
@@ -1231,7 +1234,8 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
         static_cast<Params&>(sp) = p;
         sp.partials = (float*)((uint8_t*)workspace + lists);
         sp.splits = splits;
-        cfg.gridDim = dim3((unsigned)(pairs * p.per_pair * splits));
+        sp.ctas = (int)(pairs * p.per_pair * splits);
+        cfg.gridDim = dim3((unsigned)sp.ctas);
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, varlen_prefill_kernel<SplitParams>, tm_q, tm_k, tm_v, sp));
         cfg.gridDim = dim3((unsigned)(pairs * p.per_pair), 2, kTileQ / 8);
         cfg.blockDim = dim3(kCombineThreads);

@@ -12,6 +12,8 @@ pytestmark = pytest.mark.gpu
 CASES = {
     "short": (8, 2, [87, 40, 0, 131], [[1, 128, 129, 0], [0, 0, 0, 258], [100, 100, 58, 0], [64, 64, 65, 65]]),
     "short, odd group": (3, 1, [300, 5], [[5, 300], [130, 129], [0, 1]]),
+    # items cut into runs (twelve K/V tiles or more); then more items than runs were foreseen, which stay whole
+    "split": (4, 1, [1536] + [0] * 23, [[36, 1500] + [0] * 22, [64] * 24, [0] * 23 + [1024], [100] * 14 + [0] * 10]),
     # one row block per 128 tokens at the capture, one per sequence in the replay: several items a CTA
     "short, more items than CTAs": (8, 2, [256] + [0] * 7, [[32] * 8, [1, 3, 250, 2, 0, 0, 0, 0]]),
 }
