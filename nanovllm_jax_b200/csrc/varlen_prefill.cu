@@ -773,12 +773,16 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             uint32_t i = 0;      // items
             bool ok = true;
 
-            auto issue_qk = [&](uint64_t kd) {
+            // behind_pv: o_full(j-1) is committed in front of s_full(j), so that a softmax warp that has seen S(j) finds that
+            // phase of o_full complete.  The other way round a warp that skips the softmax (its rows lie behind the
+            // sequence's end) could be at its wait for o_full(j) a phase too early, where the parity aliases.
+            auto issue_qk = [&](uint64_t kd, bool behind_pv) {
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks) {
                     const uint32_t step = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
                     mma_ss(s_t, q_desc + step, kd + step, kIdescQK, ks > 0);
                 }
+                if (behind_pv) tc_commit(&sh->o_full[x]);
                 tc_commit(&sh->s_full[x]);
             };
             auto issue_pv = [&](int j, uint64_t vd) -> bool {
@@ -808,7 +812,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     if (!(ok = slot_full(kpos))) break;
                     if (n_x > 0) {
                         tc_fence_after();
-                        issue_qk(k_desc0 + (kpos % kSlots) * kSlotStep);
+                        issue_qk(k_desc0 + (kpos % kSlots) * kSlotStep, false);
                         tc_commit(&sh->kv_empty[kpos % kSlots]);
                         if (n_x == 1) tc_commit(&sh->q_empty);
                     } else {
@@ -830,9 +834,8 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     }
                     if (j + 1 < it.n_kv) {
                         if (j + 1 < n_x) {
-                            issue_qk(k_desc0 + (kpos % kSlots) * kSlotStep);
+                            issue_qk(k_desc0 + (kpos % kSlots) * kSlotStep, true);
                             tc_commit(&sh->kv_empty[kpos % kSlots]);
-                            tc_commit(&sh->o_full[x]);
                             tc_commit(&sh->kv_empty[vpos % kSlots]);
                             if (j + 2 == n_x) tc_commit(&sh->q_empty);  // this tile's last Q.K^T has been issued
                         } else {

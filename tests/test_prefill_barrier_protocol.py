@@ -1,26 +1,38 @@
 """Event-driven CPU model of the mbarrier protocol of the prefill kernel (csrc/varlen_prefill.cu).
 
-The kernel's five roles -- TMA producer, two MMA issuers, two softmax warpgroups -- only meet through mbarriers whose
-waits see one parity bit.  The model replays their exact sequence of waits / arrivals / tcgen05.commit for random item
-lists under randomised latencies and checks what the hardware cannot tell us without a hang:
+The kernel's roles -- the warp that writes the item records, TMA producer, two MMA issuers, two softmax warpgroups of four
+warps -- only meet through mbarriers whose waits see one parity bit.  The model replays their exact sequence of waits /
+arrivals / tcgen05.commit for random item lists under randomised latencies and checks what the hardware cannot tell us
+without a hang:
 
   * no deadlock (every role runs to the end of the item list);
+  * every reader of the item ring sees the item it is at;
   * no parity alias: when a wait for phase k passes, exactly k+1 phases have completed (a barrier that got two phases
     ahead of an observer would either release it early or block it forever);
   * no barrier receives more arrivals than its count within a phase;
   * a K/V ring slot is never refilled before both issuers have released it;
   * the softmax warpgroup that zeroes the rows past a sequence's end in its last V tile waits for that slot only
-    at such tiles (skipping every other phase of the slot), and still never sees another tile there.
+    at such tiles (skipping every other phase of the slot), and still never sees another tile there;
+  * warps whose rows all lie behind the sequence's end ("dead": they only pass the hand-overs on, without the softmax's
+    time between them) and items whose two tiles do not take turns, in any mixture, keep all of this.
 
 The tensor pipe is modelled as an in-order queue (a commit arrives when everything its thread issued before has
-finished), TMA loads as delayed arrivals.
+finished, the commits of one thread one after the other), TMA loads as delayed arrivals.
 """
 import heapq
 import random
+from collections import namedtuple
 
 import pytest
 
 SLOTS = 5  # K/V ring slots, filled K0 V0 K1 V1 ...
+ITEM_RING = 2
+ITEM_READERS = 11  # producer, two issuers, eight softmax warps
+
+# n_a, n_b: K/V tiles Q tile A / B visit (n_b = 0: no second tile); ragged: the last V tile reaches past the sequence's end
+# (the softmax warps that use it zero those rows first); live: rows of Q tile A / B in front of the sequence's end; turns: the
+# exponentials of the two tiles alternate
+Item = namedtuple("Item", "n_a n_b ragged live turns")
 
 
 class ProtocolError(Exception):
@@ -35,7 +47,7 @@ class Bar:
 class Sim:
     def __init__(self, seed, jitter):
         self.t, self.q, self.n, self.rng, self.jitter = 0.0, [], 0, random.Random(seed), jitter
-        self.threads, self.pipe_free = {}, 0.0
+        self.threads, self.pipe_free, self.last_commit = {}, 0.0, {}
 
     def lat(self, x):
         return x * (1 + self.jitter * (2 * self.rng.random() - 1)) + self.jitter * 300 * self.rng.random()
@@ -87,8 +99,11 @@ class Sim:
         elif cmd[0] == "mma":  # in-order tensor pipe; commits arrive when the batch (and all before it) is done
             end = max(self.t, self.pipe_free) + cmd[1]
             self.pipe_free = end
+            when = self.last_commit.get(name, 0.0)
             for b in cmd[2]:
-                self.at(end + self.lat(60), lambda b=b: self.arrive(b))
+                when = max(when, end + self.lat(60))
+                self.at(when, lambda b=b: self.arrive(b))
+            self.last_commit[name] = when
             self.at(max(self.t + 20, end - 128), lambda: self.step(name))
         else:
             raise ValueError(cmd)
@@ -101,26 +116,42 @@ class Sim:
             raise ProtocolError(f"deadlock: {sorted(self.threads)} never finished")
 
 
-def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True):
-    """items: per work item (n_a, n_b[, ragged]) = K/V tiles Q tile A / B visit (n_b = 0: no second tile) and whether
-    the last V tile reaches past the sequence's end (the softmax warpgroups that use it zero those rows first)."""
-    items = [it if len(it) == 3 else (it[0], it[1], False) for it in items]
+def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True, o_first=True):
     sim = Sim(seed, jitter)
+    item_full = [Bar(f"item_full{s}", 1) for s in range(ITEM_RING)]
+    item_empty = [Bar(f"item_empty{s}", ITEM_READERS) for s in range(ITEM_RING)]
+    ring = [None] * ITEM_RING  # number of the item whose record the slot holds (len(items): no more)
     q_full, q_empty = Bar("q_full", 1), Bar("q_empty", 2)
     kv_full = [Bar(f"kv_full{s}", 1) for s in range(SLOTS)]
     kv_empty = [Bar(f"kv_empty{s}", empty_count) for s in range(SLOTS)]
     s_full = [Bar(f"s_full{x}", 1) for x in range(2)]
-    p_full = [[Bar(f"p_full{x}{h}", 1) for h in range(2)] for x in range(2)]  # one arrival stands for the 4 warps
+    p_full = [[Bar(f"p_full{x}{h}", 4) for h in range(2)] for x in range(2)]
     o_full = [Bar(f"o_full{x}", 1) for x in range(2)]
-    o_empty = [Bar(f"o_empty{x}", 1) for x in range(2)]
-    turn = [Bar(f"turn{x}", 1) for x in range(2)]
+    o_empty = [Bar(f"o_empty{x}", 4) for x in range(2)]
+    turns = [Bar(f"turn{x}", 4) for x in range(2)]
     slot_tile = [None] * SLOTS  # ring position whose tile the slot holds (or is being filled with)
     slot_state = ["empty"] * SLOTS  # ring-slot invariant: empty -> loading -> full -> (both released) -> empty
     released = [0] * SLOTS
 
+    def records():
+        for k in range(len(items) + 1):
+            if k >= ITEM_RING:
+                yield ("wait", item_empty[k % ITEM_RING], k // ITEM_RING - 1)
+            yield ("delay", 1400)  # claim, record
+            ring[k % ITEM_RING] = k
+            yield ("arrive", item_full[k % ITEM_RING])
+
+    def next_item(k):
+        yield ("wait", item_full[k % ITEM_RING], k // ITEM_RING)
+        if ring[k % ITEM_RING] != k:
+            raise ProtocolError(f"item {ring[k % ITEM_RING]} read for item {k}")
+        return items[k] if k < len(items) else None
+
     def producer():
-        kt = 0
-        for i, (n_a, n_b, _) in enumerate(items):
+        kt = i = 0
+        while (it := (yield from next_item(i))) is not None:
+            yield ("arrive", item_empty[i % ITEM_RING])
+            n_a, n_b = it.n_a, it.n_b
             if i > 0:
                 yield ("wait", q_empty, i - 1)
             yield ("tma", q_full)
@@ -136,6 +167,7 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True):
                     slot_tile[s] = pos
                     yield ("tma", kv_full[s])
                 kt += 1
+            i += 1
 
     def release(s):
         released[s] += 1
@@ -143,13 +175,14 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True):
             released[s], slot_state[s] = 0, "empty"
 
     def issuer(x):
-        kt = tiles = used = 0
+        kt = tiles = used = i = 0
 
         def slot(pos):
             return ("wait", kv_full[pos % SLOTS], pos // SLOTS)
 
-        for i, (n_a, n_b, _) in enumerate(items):
-            n_x, n_kv = (n_a, n_b)[x], max(n_a, n_b)
+        while (it := (yield from next_item(i))) is not None:
+            yield ("arrive", item_empty[i % ITEM_RING])
+            n_x, n_kv = (it.n_a, it.n_b)[x], max(it.n_a, it.n_b)
             yield ("wait", q_full, i)
             if n_x == 0:
                 yield ("arrive", q_empty)
@@ -178,7 +211,8 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True):
                     yield ("arrive", kv_empty[vpos % SLOTS])
                 if j + 1 < n_kv:
                     if j + 1 < n_x:
-                        yield ("mma", 512, [s_full[x], kv_empty[kpos % SLOTS], o_full[x], kv_empty[vpos % SLOTS]]
+                        yield ("mma", 512, ([o_full[x], s_full[x]] if o_first else [s_full[x], o_full[x]])
+                               + [kv_empty[kpos % SLOTS], kv_empty[vpos % SLOTS]]
                                + ([q_empty] if j + 2 == n_x else []))
                     else:
                         yield ("arrive", kv_empty[kpos % SLOTS])
@@ -186,49 +220,72 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True):
                 release(vpos % SLOTS)
             used += 1 if n_x > 0 else 0
             kt += n_kv
+            i += 1
 
-    def softmax(x):
-        tiles = turns_seen = kt = 0
-        for n_a, n_b, ragged in items:
+    def softmax(x, warp):
+        tiles = turns_seen = kt = k = 0
+        while (it := (yield from next_item(k))) is not None:
+            n_a, n_b = it.n_a, it.n_b
             n_x, n_kv = (n_a, n_b)[x], max(n_a, n_b)
-            kt0, kt = kt, kt + n_kv
-            both = n_b > 0
+            kt0, kt, k = kt, kt + n_kv, k + 1
+            if n_x == 0:
+                yield ("arrive", item_empty[(k - 1) % ITEM_RING])
+                continue
+            both = n_b > 0 and it.turns
+            dead = 32 * warp >= it.live[x]
             for j in range(n_x):
                 yield ("wait", s_full[x], tiles)
-                if ragged and j == n_kv - 1:  # zero the rows past the sequence's end in V(last) before P is handed over
+                turn = None
+                if both and (j >= 1 if x == 0 else j < n_a):  # A(j) after B(j-1); B(j) after A(j) while A has tiles
+                    turn = ("wait", turns[x ^ 1], turns_seen)
+                    turns_seen += 1
+                hand = both and (x == 0 or j + 1 < n_a) and (hand_turn_back or x == 0)
+                if it.ragged and j == n_kv - 1:  # zero the rows past the sequence's end in V(last) before P is handed over
                     vpos = 2 * (kt0 + n_kv - 1) + 1
                     yield ("wait", kv_full[vpos % SLOTS], vpos // SLOTS)
                     if slot_tile[vpos % SLOTS] != vpos:
                         raise ProtocolError(f"softmax{x} zeroes rows of ring position {slot_tile[vpos % SLOTS]}, not {vpos}")
                     yield ("delay", 60)
+                if dead:
+                    if turn:
+                        yield turn
+                    if hand:
+                        yield ("arrive", turns[x])
+                    yield ("arrive", p_full[x][0])
+                    yield ("arrive", p_full[x][1])
+                    tiles += 1
+                    continue
                 yield ("delay", 300)  # scores to registers, row max: not exclusive
-                if both and (j >= 1 if x == 0 else j < n_a):  # A(j) after B(j-1); B(j) after A(j) while A has tiles
-                    yield ("wait", turn[x ^ 1], turns_seen)
-                    turns_seen += 1
+                if turn:
+                    yield turn
                 yield ("delay", 800)
                 yield ("arrive", p_full[x][0])
                 yield ("delay", 600)
-                if both and (x == 0 or j + 1 < n_a) and (hand_turn_back or x == 0):
-                    yield ("arrive", turn[x])  # handed over once the last chunk of P is on its way
+                if hand:
+                    yield ("arrive", turns[x])  # handed over once the last chunk of P is on its way
                 yield ("arrive", p_full[x][1])
                 tiles += 1
-            if n_x > 0:
-                yield ("wait", o_full[x], tiles - 1)
+            yield ("wait", o_full[x], tiles - 1)
+            if not dead:
                 yield ("delay", 900)
-                yield ("arrive", o_empty[x])
+            yield ("arrive", o_empty[x])
+            yield ("arrive", item_empty[(k - 1) % ITEM_RING])
 
+    sim.spawn("records", records())
     sim.spawn("producer", producer())
     for x in range(2):
         sim.spawn(f"issuer{x}", issuer(x))
-        sim.spawn(f"softmax{x}", softmax(x))
+        for warp in range(4):
+            sim.spawn(f"softmax{x}{warp}", softmax(x, warp))
     sim.run()
     return sim.t
 
 
-def item_tiles(q0, rows, prefix=0, last=None, pair_heads=False):
-    """What load_item computes for the row block starting at row q0 with `rows` live rows of a sequence with
+def item_tiles(q0, rows, prefix=0, last=None, pair_heads=False, turns=True, run=None):
+    """What make_item computes for the row block starting at row q0 with `rows` live rows of a sequence with
     `prefix` cached tokens; `last` says whether it is the sequence's final block (default: iff the block is not full).
-    pair_heads: the item is 128 rows of two heads (both Q tiles see the same keys) instead of 256 rows of one head."""
+    pair_heads: the item is 128 rows of two heads (both Q tiles see the same keys) instead of 256 rows of one head.
+    run: (c, runs): only the c-th run of its K/V tiles."""
     full = 128 if pair_heads else 256
     rows = min(rows, full)
     last = rows < full if last is None else last
@@ -239,24 +296,47 @@ def item_tiles(q0, rows, prefix=0, last=None, pair_heads=False):
         n_b = n_a
     else:
         n_b = min(nk_total, (prefix + q0 + 255) // 128 + 1) if rows > 128 else 0
-    return n_a, n_b, max(n_a, n_b) * 128 > len_k
+    live = (rows, rows) if pair_heads else (min(rows, 128), rows - 128)
+    n_kv = max(n_a, n_b)
+    if run:
+        c, runs = run
+        j0, j1 = n_a * c // runs, n_kv if c + 1 == runs else n_a * (c + 1) // runs
+        n_a, n_b, len_k = min(n_a, j1) - j0, min(n_b, j1) - j0 if n_b else 0, len_k - j0 * 128
+        n_kv = j1 - j0
+    return Item(n_a, n_b, n_kv * 128 > len_k, live, turns)
+
+
+def random_items(rng, pair_heads, count):
+    return [item_tiles((128 if pair_heads else 256) * rng.randint(0, 7),
+                       rng.choice([1, 20, 64, 100, 128, 129, 200, 256, 256, 256]),
+                       prefix=rng.choice([0, 0, 1, 108, 127, 128, 300]), last=rng.choice([None, None, True]),
+                       pair_heads=pair_heads, turns=rng.random() < 0.6)
+            for _ in range(count)]
 
 
 def test_single_items_of_every_shape():
     for q0 in (0, 256, 1024):
         for rows in (1, 128, 129, 256):
-            assert run_cta([item_tiles(q0, rows)]) > 0
-            assert run_cta([item_tiles(q0, rows, pair_heads=True)]) > 0
+            for turns in (False, True):
+                assert run_cta([item_tiles(q0, rows, turns=turns)]) > 0
+                assert run_cta([item_tiles(q0, rows, pair_heads=True, turns=turns)]) > 0
+
+
+def test_runs_of_split_items():
+    for runs in (2, 3, 5):
+        for c in range(runs):
+            for pair_heads in (False, True):
+                for jitter in (0.0, 0.95):
+                    run_cta([item_tiles(256, 200, prefix=2900, pair_heads=pair_heads, run=(c, runs))], seed=c, jitter=jitter)
 
 
 @pytest.mark.parametrize("seed", range(40))
 def test_random_item_lists_under_random_latencies(seed):
     rng = random.Random(seed)
-    pair_heads = seed % 2 == 1
-    items = [item_tiles((128 if pair_heads else 256) * rng.randint(0, 7), rng.choice([1, 64, 128, 129, 200, 256, 256, 256]),
-                        prefix=rng.choice([0, 0, 1, 127, 128, 300]), last=rng.choice([None, None, True]),
-                        pair_heads=pair_heads)
-             for _ in range(rng.randint(1, 14))]
+    items = random_items(rng, seed % 2 == 1, rng.randint(1, 14))
+    if seed % 4 == 3:  # an odd group: items of two heads and of a lone one
+        items += random_items(rng, False, 4)
+        rng.shuffle(items)
     for jitter in (0.0, 0.4, 0.95):
         run_cta(items, seed=seed, jitter=jitter)
 
@@ -268,3 +348,6 @@ def test_model_catches_broken_protocols():
         run_cta(items, empty_count=1)
     with pytest.raises(ProtocolError, match="deadlock"):  # tile B never hands the softmax turn back
         run_cta(items, hand_turn_back=False)
+    with pytest.raises(ProtocolError, match="o_full"):  # dead warps see S(j) before the commit of P.V(j-1) has arrived
+        for seed in range(40):
+            run_cta([item_tiles(512, 20, prefix=108, pair_heads=True, turns=False)] * 3, seed=seed, jitter=0.95, o_first=False)
