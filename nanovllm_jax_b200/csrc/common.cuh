@@ -92,10 +92,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-// Bounded wait: gives up after `limit` polls (each poll itself blocks for a
-// slice of about 4 us at the hint given here, 1.3 us without one), returns false on timeout so the caller can set an
-// error flag and leave instead of spinning forever.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 22)) {
+// What one poll of a barrier that does not complete blocks for at the hint that mbar_wait gives (1.4 us without one).
+constexpr uint32_t kPollNanoseconds = 4000;
+constexpr uint32_t polls_of_ms(uint32_t ms) { return (uint32_t)((uint64_t)ms * 1000000 / kPollNanoseconds); }
+
+// Bounded wait: gives up after `limit` polls (five seconds unless the caller says otherwise), returns false on timeout so
+// the caller can set an error flag and leave instead of spinning forever.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = polls_of_ms(5000)) {
     for (uint32_t i = 0; i < limit; ++i) {
         uint32_t ok;
         asm volatile(

@@ -496,7 +496,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
             atomicOr(&g_error_flag, 1);
             // Let loads already issued land before the CTA's shared memory is released.
             for (uint32_t j = (it >= stages ? it - stages : 0); j < it; ++j)
-                (void)mbar_wait(full_bar + (j % stages), (j / stages) & 1u, 1u << 16);
+                (void)mbar_wait(full_bar + (j % stages), (j / stages) & 1u, polls_of_ms(90));
         }
         return;
     }
