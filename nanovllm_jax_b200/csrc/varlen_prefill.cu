@@ -100,7 +100,7 @@ struct Params {
 
 // A short launch (at most one item per SM, as far as the host knows) runs without a plan kernel and carries the step's K/V
 // scatter: every CTA finds its item in the device's cu_seqlens (one load latency and a few warp votes; records laid out by the
-// host and passed as arguments were 0.4 us faster, 8.5 against 8.9 us for one prompt of 87 tokens, but a captured launch then
+// host and passed as arguments cost 0.4 us less, 8.5 against 8.9 us for one prompt of 87 tokens, but a captured launch then
 // kept the lengths of its capture).  Should the lengths make more items than CTAs by then, a CTA takes several.
 struct ShortParams : Params {
     const int32_t* cu_seqlens;
@@ -373,8 +373,6 @@ struct Item {
     int dq, dh, ragged, kv0;           // Q tile B = rows + dq of head + dh; the last KV tile reaches past the last key; a run
                                        // of a split item: its first KV tile (len_k and prefix count from there on), else -1
 };
-constexpr int kNoTurnTiles = 2;        // items of so few K/V tiles do without the turns of the two softmax warpgroups: the
-                                       // second tile's wait is not won back there (48 short prompts: 42.4 -> 39.9 us)
 constexpr int kItemRing = 2;
 constexpr int kItemReaders = 3 + 8;    // TMA producer, two MMA issuers, eight softmax warps
 
@@ -877,7 +875,11 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 if (lane == 0) mbar_arrive(&sh->item_empty[k % kItemRing]);
                 continue;
             }
-            const bool both = it.n_b > 0 && it.n_kv > kNoTurnTiles;  // the two tiles take turns
+            // The two tiles take turns, unless tile A has a single K/V tile: then nothing of A could run under B's
+            // exponentials, and B's wait is not won back (64 prompts of 20..128 tokens, 32 / 8 heads: 47.9 us without turns,
+            // 51.3 with).  With two the turns pay: 16 prompts of 256 tokens 35.7 us without, 34.4 with; five of 390..472, 64 / 8
+            // heads, 47.5 and 46.0; 48 of 5..300, 10 / 2 heads, 33.5 and 33.8.
+            const bool both = it.n_b > 0 && it.n_a > 1;
             const int q_pos = it.q0 + x * it.dq + row;             // row of the sequence's query block
             const int first_lim = it.prefix + it.q0 + x * it.dq;  // last key visible to the first row of this Q tile
             float m_run = -INFINITY, m_used = -INFINITY, l = 0.f;
