@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <algorithm>
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -85,19 +86,39 @@ int source_dtype(const at::Tensor& key) {
     raise(PyExc_TypeError, std::string("key must be bf16 or fp32, got ") + dtype_text(key.scalar_type()));
 }
 
-int to_int(PyObject* o) {
-    long v;
-    if (PyLong_Check(o)) {
-        v = PyLong_AsLong(o);
-    } else {
-        PyObject* i = PyNumber_Long(o);  // numpy scalars, whole floats
-        if (!i) throw Raised();
-        v = PyLong_AsLong(i);
-        Py_DECREF(i);
-    }
+// A Python int -> 32 bits; a null pointer stands for an error that is set.
+int narrow(PyObject* i) {
+    if (!i) throw Raised();
+    int overflow = 0;
+    const long v = PyLong_AsLongAndOverflow(i, &overflow);
     if (v == -1 && PyErr_Occurred()) throw Raised();
-    if (v > INT32_MAX || v < INT32_MIN) raise(PyExc_OverflowError, "value does not fit 32 bits");
+    if (overflow || v > INT32_MAX || v < INT32_MIN) raise(PyExc_OverflowError, "value does not fit 32 bits");
     return (int)v;
+}
+struct Owned {
+    PyObject* o;
+    ~Owned() { Py_XDECREF(o); }
+};
+// A size: integers, numpy and tensor scalars, floats without a fraction.
+int to_int(PyObject* o) {
+    if (PyLong_Check(o)) return narrow(o);
+    if (PyIndex_Check(o)) {
+        const Owned i{PyNumber_Index(o)};
+        if (i.o) return narrow(i.o);
+        if (!PyErr_ExceptionMatches(PyExc_TypeError)) throw Raised();
+        PyErr_Clear();  // a tensor of a floating type
+    }
+    const double d = PyFloat_AsDouble(o);
+    if (d == -1.0 && PyErr_Occurred()) throw Raised();
+    if (d > INT32_MAX || d < INT32_MIN) raise(PyExc_OverflowError, "value does not fit 32 bits");
+    if (!(d == std::floor(d))) raise(PyExc_ValueError, "a size must be a whole number, got " + std::to_string(d));
+    return (int)d;
+}
+// An upper bound: whatever int() takes.
+int to_bound(PyObject* o) {
+    if (PyLong_Check(o)) return narrow(o);
+    const Owned i{PyNumber_Long(o)};
+    return narrow(i.o);
 }
 float to_float(PyObject* o) {
     const double v = PyFloat_AsDouble(o);
@@ -379,7 +400,7 @@ PyObject* varlen_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor& k = need(a[1], "k", at::kBFloat16, 3);
         const at::Tensor& v = need(a[2], "v", at::kBFloat16, 3);
         const at::Tensor& cu = need(a[3], "cu_seqlens", at::kInt, 1);
-        const int max_seqlen = to_int(a[4]);
+        const int max_seqlen = to_bound(a[4]);
         const float scale = to_float(a[5]);
         const at::Tensor& cu_k = a[8] == Py_None ? cu : need(a[8], "cu_seqlens_k", at::kInt, 1);
         const int64_t t = q.size(0), h = q.size(1), d = q.size(2);
@@ -409,7 +430,7 @@ PyObject* paged_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor& bt = need(a[3], "block_tables", at::kInt, 2);
         const at::Tensor& cu = need(a[4], "cu_seqlens_q", at::kInt, 1);
         const at::Tensor& cu_k = need(a[5], "cu_seqlens_k", at::kInt, 1);
-        const int max_seqlen_q = to_int(a[6]);
+        const int max_seqlen_q = to_bound(a[6]);
         const float scale = to_float(a[7]);
         const Cache c = paged_cache(kc, vc, q, to_int(a[8]));
         const int64_t t = q.size(0);
@@ -454,7 +475,7 @@ PyObject* prefill_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor& slots = need(a[5], "slot_mapping", at::kInt, 1);
         const at::Tensor& cu = need(a[7], "cu_seqlens_q", at::kInt, 1);
         const at::Tensor& cu_k = need(a[8], "cu_seqlens_k", at::kInt, 1);
-        const int max_seqlen = to_int(a[9]);
+        const int max_seqlen = to_bound(a[9]);
         const float scale = to_float(a[10]);
         const Cache c = paged_cache(kc, vc, q, block_size);
         const int64_t t = q.size(0);
