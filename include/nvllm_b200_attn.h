@@ -193,7 +193,8 @@ size_t nvllm_b200_varlen_prefill_workspace_bytes(int64_t T, int B, int H, int KV
  *                 that makes more row blocks than the host copy had.  A host copy
  *                 without any token enqueues no attention
  *   max_seqlen    upper bound of any sequence length (used for grid sizing when
- *                 cu_seqlens_host is NULL)
+ *                 cu_seqlens_host is NULL; longer sequences are computed all the
+ *                 same, as the attention layer's contexts end at 8192)
  *
  * Unlike the reference, rows beyond the 8192-token bucket (utils/context.py:18-32)
  * are computed rather than returned as zeros.  Rows of `out` at token indices

@@ -1166,6 +1166,8 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
         if (max_seqlen > kMaxLevels * kTileQ)
             return fail(NVLLM_B200_EUNSUPPORTED, "%s: max_seqlen %d (max %d)", who, max_seqlen, kMaxLevels * kTileQ);
         pairs = (int64_t)B * ((max_seqlen + kTileQ - 1) / kTileQ);
+        // The attention layer's contexts round the longest length up to 8192 at most: prompts beyond it show in T.
+        if ((int64_t)B * max_seqlen < T) pairs = cap;
     }
     if (pairs > cap) pairs = cap;
     if (pairs == 0) return scatter_only();

@@ -64,3 +64,28 @@ def test_replay_follows_the_device_lengths(kind, step):
         if step:
             assert np.array_equal(torch_to_bits(attn.k_cache).reshape(-1, kvh, 128)[:w.total_tokens], t["k_bits"])
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("h,kvh,lens", [(2, 1, [9300]), (1, 1, [8200, 3]), (2, 1, [300, 8700])])
+def test_prompts_beyond_the_contexts_length_bucket(h, kvh, lens):
+    """The context's max_seqlen_q ends at 8192, and without a host copy the library sizes its grid from it: prompts beyond it
+    have more row blocks than foreseen (with so few heads the launch cuts its items into runs)."""
+    import torch
+    from nanovllm_jax_b200 import _lib, workloads
+    from nanovllm_jax_b200.layers.attention import Attention
+    from nanovllm_jax_b200.utils.context import create_prefill_context
+    w = workloads.make_prefill_workload("long", seed=9800 + lens[0], batch=len(lens), num_heads=h, num_kv_heads=kvh, len_lo=1,
+                                        len_hi=1, seq_lens=lens)
+    t = workloads.prefill_tensors_numpy(w)
+    q, k, v = (bits_to_torch(t[n + "_bits"]) for n in "qkv")
+    cu = torch.from_numpy(w.cu_seqlens).cuda()
+    attn = Attention(h, 128, w.scale, kvh, 256)
+    ctx = create_prefill_context(cu, cu, max(lens), max(lens), torch.arange(w.total_tokens, dtype=torch.int32, device="cuda"))
+    assert ctx.max_seqlen_q == 8192
+    got = torch_to_f32(attn(q, k, v, ctx))
+    for a, z in zip(w.cu_seqlens[:-1], w.cu_seqlens[1:]):
+        s = (q[a:z].float().transpose(0, 1) @ k[a:z].float().permute(1, 2, 0)) * w.scale
+        s.masked_fill_(torch.ones(z - a, z - a, dtype=torch.bool, device="cuda").triu_(1), float("-inf"))
+        want = (s.softmax(-1) @ v[a:z].float().transpose(0, 1)).transpose(0, 1)
+        assert_attention_close(got[a:z], torch_to_f32(want), f"{lens} rows {a}..{z}")
+    assert _lib.device_status() == 0
