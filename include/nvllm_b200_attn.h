@@ -249,8 +249,8 @@ int nvllm_b200_paged_prefill(const void* q, const void* k_cache, const void* v_c
  * slot_mapping (as nvllm_b200_store_kvcache, bf16 rows), then attend -- over the
  * packed k / v (as nvllm_b200_varlen_prefill, max_seqlen_q >= any length) when
  * block_tables is NULL, over the pages (as nvllm_b200_paged_prefill) otherwise.
- * Same results as the two calls.  One call lets the scatter run beside the
- * attention of packed keys, which does not read the cache.
+ * Same results as the two calls.  The scatter of few packed tokens runs on the
+ * SMs that the attention leaves; elsewhere it is a launch in front of it.
  *
  *   k_cache, v_cache [NB, block_size, KVH, D] bf16;  MB is the width of block_tables
  */

@@ -37,11 +37,12 @@
 //    also scatters the step's new K/V rows into the cache).
 //  * The first tiles are requested before that kernel has finished, unless they hold a slot that it writes.
 //
-// Measured on a B200 (per call, CUDA-graph replay, before -> after the transposed products, the two-stage ring, the
-// early requests and the native walk): one sequence of 300 tokens, 16 / 8 heads, 12.6 -> 7.3 us; Qwen3-8B shapes, batch
-// 64, 1.14 GB: 177 -> 163 us (7.0 TB/s); Qwen3-32B shapes, batch 256, 4.51 GB: 668 -> 621 us (7.26 TB/s).  What bounds it:
-// the stream itself runs at about 7.25 TB/s (a build without the math is not faster); about 3.5 us pass before the first
-// tile is under way and 3.5 us after the last one has landed.
+// Measured on a B200 through the decode step (this kernel and the one in front of it, calls in a row, before -> after the
+// transposed products, the two-stage ring, the early requests and the native walk): one sequence of 300 tokens, 16 / 8
+// heads, 25.0 -> 8.0 us (12.6 -> 7.3 replayed from a graph, where the host's part does not count); Qwen3-8B shapes, batch 64,
+// 1.14 GB: 179 -> 168 us (6.8 TB/s); Qwen3-32B shapes, batch 256, 4.51 GB: 673 -> 640 us (7.05 TB/s; 4.5 to 5 %).  What
+// bounds it: the stream itself runs at about 7.25 TB/s (a build without the math is not faster); about 3.5 us pass before
+// the first tile is under way and 3.5 us after the last one has landed.
 //
 // No spin-wait is unbounded: every mbarrier wait gives up after a poll limit,
 // raises a device error flag (readable through nvllm_b200_device_status) and

@@ -68,7 +68,7 @@ __device__ int g_error_flag = 0;
 constexpr int kD = 128;
 constexpr int kTileQ = 128;            // rows per Q tile
 constexpr int kTileKV = 128;
-constexpr int kThreads = 384;            // 3 warpgroups: {TMA, MMA, 2 idle warps} | softmax A | softmax B
+constexpr int kThreads = 384;            // 3 warpgroups: {TMA, MMA A, MMA B, item records} | softmax A | softmax B
 constexpr int kPanelBytes = 128 * 128;  // 128 rows x 64 dims bf16, 128B-swizzled
 constexpr int kTileBytes = 2 * kPanelBytes;
 constexpr int kSlots = 5;                // one ring for K and V tiles, filled in the order K0 V0 K1 V1 ...
@@ -377,7 +377,7 @@ constexpr int kItemRing = 2;
 constexpr int kItemReaders = 3 + 8;    // TMA producer, two MMA issuers, eight softmax warps
 
 struct Shared {
-    Item items[kItemRing];  // the items of this CTA, written ahead by an otherwise idle warp
+    Item items[kItemRing];  // the items of this CTA, written ahead by warp 3
     uint64_t item_full[kItemRing], item_empty[kItemRing];
     uint64_t q_full, q_empty;
     uint64_t kv_full[kSlots], kv_empty[kSlots];
@@ -1200,7 +1200,7 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     int ctas = p.item_ctas = (int)std::min<int64_t>(pairs * p.per_pair, sms);
 
     // A short list known to the host (and nothing for the plan kernel to check on the device) needs no plan kernel, and
-    // the scatter, where SMs are left, goes with the launch.  Elsewhere the scatter is a launch of its own: on the idle warp of the
+    // the scatter, where SMs are left, goes with the launch.  Elsewhere the scatter is a launch of its own: on a warp of the
     // attention CTAs it slowed them by as much as it took (power and issue slots).
     const int64_t max_tiles = block_tables ? (int64_t)MB * block_size / kTileKV : (longest + kTileKV - 1) / kTileKV;
     const size_t lists = list_bytes(T, B);

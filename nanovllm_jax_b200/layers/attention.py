@@ -125,7 +125,7 @@ class Attention:
                                               context.block_tables, context.context_lens, self.scale, self.block_size,
                                               None, True)
         if self.k_cache is not None and self.v_cache is not None:
-            # prefill: one C call too, which lets the scatter run beside the attention of packed keys
+            # prefill: one C call too (the scatter of few packed tokens runs beside their attention)
             if context.block_tables is not None or context.max_seqlen_k == context.max_seqlen_q:
                 out = _lib.binding().prefill_step(
                     q, k, v, self.k_cache, self.v_cache, context.slot_mapping, context.block_tables, context.cu_seqlens_q,

@@ -1,5 +1,5 @@
 """Attention.__call__ on a prefill step as one C call (nvllm_b200_prefill_step): wherever the K/V scatter runs -- CTAs of
-their own beside a short list of items, the attention kernel's idle warps, the plan kernel, a launch of its own -- the
+its own beside a short list of items, or a launch in front, with the plan kernel working beside it -- the
 caches equal the oracle's bit for bit and the output equals the attention entry points' and, at small sizes, the oracle's.
 The group sizes include odd ones (a lone head per kv head takes 256 rows at a time, the others 128 rows of two heads)."""
 import math
@@ -48,7 +48,8 @@ def test_store_and_attend_in_one_call(lens, host, h, kvh):
     assert _lib.device_status() == 0
 
 
-def test_long_sequences_hide_the_scatter_behind_the_attention():
-    """Eight sequences of 3000 tokens: the scatter runs on the attention kernel's idle warps, twice in a row."""
+def test_long_sequences_store_and_attend_again_and_again():
+    """Eight sequences of 3000 tokens, several calls in a row: the plan of a call runs beside its scatter, and the scatter
+    may start while the call in front of it still attends."""
     test_store_and_attend_in_one_call([3000] * 8, True, 16, 2)
     test_store_and_attend_in_one_call([3000] * 8, False, 16, 2)
