@@ -136,7 +136,17 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* desc, ui
         : "memory");
 }
 
-// 4-D, with an L2 eviction-priority hint (createpolicy result).
+// The same with an L2 eviction-priority hint (createpolicy result).
+__device__ __forceinline__ void tma_load_3d_hint(void* smem_dst, const void* desc, uint64_t* bar, int c0, int c1, int c2,
+                                                 uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], "
+        "[%2], %6;" ::"r"(smem_u32(smem_dst)),
+        "l"(reinterpret_cast<uint64_t>(desc)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "l"(policy)
+        : "memory");
+}
+
+// 4-D, with a hint.
 __device__ __forceinline__ void tma_load_4d_hint(void* smem_dst, const void* desc, uint64_t* bar, int c0, int c1,
                                                  int c2, int c3, uint64_t policy) {
     asm volatile(

@@ -88,7 +88,7 @@ struct Record {
 };
 
 struct Params {
-    const int4* items;  // record 0: {number of pairs, items claimed, 0, 0}; then the two halves of every Record
+    const int4* items;  // record 0: {number of pairs, items claimed, head groups, 0}; then the two halves of every Record
     const int32_t* block_tables;  // [B, MB] page ids, or nullptr for packed keys/values
     int MB, block_size;
     __nv_bfloat16* out;
@@ -124,8 +124,8 @@ constexpr int kMinRun = 4;  // tiles per run: at least one of them is visible to
 constexpr int kSplitTiles = 12;
 // The launch has a CTA for every run that the host could foresee.  Where the device's lengths make more items than that (a
 // captured launch whose lengths were rewritten), the items stay whole and the CTAs claim them one by one.
-__device__ __forceinline__ int splits_of(const SplitParams& p) {
-    return (long long)p.items[0].x * p.per_pair * p.splits <= p.ctas ? p.splits : 1;
+__device__ __forceinline__ int splits_of(const SplitParams& p, int pairs) {
+    return (long long)pairs * p.per_pair * p.splits <= p.ctas ? p.splits : 1;
 }
 __device__ __forceinline__ int runs_of(int splits, int n_a) { return n_a < kSplitTiles ? 1 : min(splits, n_a / kMinRun); }
 
@@ -135,8 +135,18 @@ __device__ __forceinline__ Record record_of(const Params& p, int pair) {
 __device__ __forceinline__ int claim_item(const Params& p) {
     return (int)gridDim.x + atomicAdd(&const_cast<int4*>(p.items)->y, 1);
 }
-__device__ __forceinline__ int items_of(const Params& p) { return p.items[0].x * p.per_pair; }
-__device__ __forceinline__ int items_of(const SplitParams& p) { return p.items[0].x * p.per_pair * splits_of(p); }
+// The item list's header, read once per thread.
+struct List {
+    int pairs, groups;
+};
+__device__ __forceinline__ List list_of(const Params& p) {
+    const int4 h = p.items[0];
+    return List{h.x, h.z};
+}
+__device__ __forceinline__ int items_of(const Params& p, const List& l) { return l.pairs * p.per_pair; }
+__device__ __forceinline__ int items_of(const SplitParams& p, const List& l) {
+    return l.pairs * p.per_pair * splits_of(p, l.pairs);
+}
 
 // ------------------------------------------------------------------------------------------
 // tcgen05 wrappers
@@ -279,15 +289,32 @@ constexpr uint32_t kIdescPV = kIdescQK | (1u << 16);  // B operand MN-major
 // ------------------------------------------------------------------------------------------
 // plan kernel: (sequence, row block) pairs sorted by causal span, largest first
 // ------------------------------------------------------------------------------------------
+// Longest spans first means that all sequences are in flight at once.  Where their keys and values do not fit the L2 the kv
+// heads are taken in groups whose keys and values do, one group after the other, as long as each is long enough for its CTAs to
+// end together.  Together with the streams' eviction hints (Q and the output are touched once), us per call: 16 prompts of
+// 128..4096 tokens, 32 / 8 heads (139 MB of K and V): 931 as one group, 912 with the hints, 880 in two, 884 in four, 916 in
+// eight (4 rounds of items each); 32 of 500..2000, 16 / 8 (164 MB): 398, 384, 366, 367, 386; 8 of 1000..8000, 40 / 8: 2190,
+// 2160, 2104, 2117, 2106; 12 of 17..700 behind 500..5000 cached ones (4 rounds of items in all): 260, 258, 271 in two.
+constexpr long long kGroupRows = (96 << 20) / 512;  // (token, kv head) rows of K and V: 512 bytes
+constexpr int kGroupRounds = 6;                     // items per CTA and group
+__device__ int head_groups(long long keys, int pairs, int per_pair, int KVH, int ctas) {
+    int n = 1;
+    while (KVH % (2 * n) == 0 && keys * KVH > kGroupRows * n &&
+           (long long)pairs * per_pair >= (long long)2 * n * kGroupRounds * ctas)
+        n *= 2;
+    return n;
+}
+
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_t* __restrict__ cu_seqlens,
                                                                     const int32_t* __restrict__ cu_k, int paged, int B,
-                                                                    int4* __restrict__ items, int capacity,
-                                                                    int behind_store) {
+                                                                    int4* __restrict__ items, int capacity, int per_pair,
+                                                                    int KVH, int ctas, int behind_store) {
     // A row block's weight is its causal span in blocks of 128 keys: level = prefix / 128 + block index.
     __shared__ int hist[kMaxLevels];
     __shared__ int base[kMaxLevels];
     __shared__ int max_level, bad;
+    __shared__ unsigned long long keys;
     // Behind this step's own scatter there is nothing to wait for: that kernel has let this one go after everything in front
     // of it was complete, and writes nothing that is read here.  The wait at the end makes the main kernel's wait cover it.
     // Only then may the main kernel start: its CTAs dealt to SMs in the order in which the scatter left them, instead of in
@@ -297,7 +324,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
         griddep_launch_dependents();
     }
     for (int i = threadIdx.x; i < kMaxLevels; i += blockDim.x) hist[i] = 0;
-    if (threadIdx.x == 0) max_level = 0, bad = 0;
+    if (threadIdx.x == 0) max_level = 0, bad = 0, keys = 0;
     __syncthreads();
     // few sequences: a warp each, its lanes take the row blocks; many: a thread each
     const bool by_warp = B <= 256;
@@ -312,6 +339,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
         const int n = len > 0 ? (len + kTileQ - 1) / kTileQ : 0;
         if (n > 0 && l0 == 0) {
             atomicMax(&max_level, min(lvl0 + n, kMaxLevels));
+            atomicAdd(&keys, (unsigned long long)len_k);
             if (lvl0 + n > kMaxLevels) atomicOr(&g_error_flag, 16);
         }
         for (int l = l0; l < n; l += dl) atomicAdd(&hist[min(lvl0 + l, kMaxLevels - 1)], 1);
@@ -319,7 +347,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
     __syncthreads();
     if (bad) {  // uniform: publish an empty list so that the main kernel computes nothing
         if (threadIdx.x == 0) {
-            items[0] = make_int4(0, 0, 0, 0);
+            items[0] = make_int4(0, 0, 1, 0);
             atomicOr(&g_error_flag, 32);
         }
         if (behind_store) griddep_wait();
@@ -339,7 +367,8 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
             if (l >= 0) base[l] = run + incl - h;
             run += __shfl_sync(0xffffffffu, incl, 31);
         }
-        if (threadIdx.x == 0) items[0] = make_int4(run < capacity ? run : capacity, 0, 0, 0);
+        if (threadIdx.x == 0)
+            items[0] = make_int4(min(run, capacity), 0, head_groups((long long)keys, min(run, capacity), per_pair, KVH, ctas), 0);
     }
     __syncthreads();
     for (int b = b0; b < B; b += db) {
@@ -428,13 +457,20 @@ __device__ __forceinline__ Item make_item(const Params& p, const Record& rec, in
     it.kv0 = -1;
     return it;
 }
-__device__ __forceinline__ Item load_item(const Params& p, int idx) {
-    const int pair = idx / p.per_pair;
-    return make_item(p, record_of(p, pair), idx - pair * p.per_pair);
+// Items go by head group (see head_groups), in a group by pair.
+__device__ __forceinline__ Item load_item(const Params& p, const List& l, int idx) {
+    int per = p.per_pair, first = 0;
+    if (l.groups > 1) {
+        per /= l.groups;
+        first = idx / (l.pairs * per) * per;
+        idx -= first * l.pairs;
+    }
+    const int pair = idx / per;
+    return make_item(p, record_of(p, pair), first + idx - pair * per);
 }
-__device__ __forceinline__ Item load_item(const SplitParams& p, int idx) {
-    const int splits = splits_of(p), c = idx % splits;
-    Item it = load_item(static_cast<const Params&>(p), idx / splits);
+__device__ __forceinline__ Item load_item(const SplitParams& p, const List& l, int idx) {
+    const int splits = splits_of(p, l.pairs), c = idx % splits;
+    Item it = load_item(static_cast<const Params&>(p), l, idx / splits);
     const int runs = runs_of(splits, it.n_a);
     if (runs == 1) {
         if (c > 0) it.n_a = it.n_b = it.n_kv = 0;
@@ -474,8 +510,8 @@ __device__ __forceinline__ int kv_tile_token(const Params& p, const Item& it, in
 }
 
 __device__ __forceinline__ void store_32bytes(void* dst, const uint32_t (&w)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+    asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]),
+                 "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
                  : "memory");
 }
 
@@ -648,14 +684,12 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
     // Register budget: the TMA / MMA warpgroup keeps 96 registers per thread, the two softmax warpgroups take 200
     // (96*128 + 200*256 <= 64K), enough to hold a whole 128-column score row.
-    int total = 0;
-    if constexpr (!kShort) total = (tmem != 0xFFFFFFFFu) ? items_of(p) : 0;
-
     if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
     if (warp == 0) {
         // =============================== TMA producer ===============================
         if (lane == 0) {
+            const uint64_t once = policy_evict_first();
             uint32_t kt = 0, i = 0;
             bool ok = true;
             Item it;
@@ -665,11 +699,11 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 const int tok_q = it.seq_start + it.q0;
                 if (i > 0 && !(ok = wait_or_abort(sh, &sh->q_empty, (i - 1) & 1u))) break;
                 mbar_expect_tx(&sh->q_full, (it.n_b > 0 ? 2 : 1) * kTileBytes);
-                tma_load_3d(sQ, &tm_q, &sh->q_full, 0, it.head, tok_q);
-                tma_load_3d(sQ + kPanelBytes, &tm_q, &sh->q_full, 64, it.head, tok_q);
+                tma_load_3d_hint(sQ, &tm_q, &sh->q_full, 0, it.head, tok_q, once);
+                tma_load_3d_hint(sQ + kPanelBytes, &tm_q, &sh->q_full, 64, it.head, tok_q, once);
                 if (it.n_b > 0) {
-                    tma_load_3d(sQ + kTileBytes, &tm_q, &sh->q_full, 0, it.head + it.dh, tok_q + it.dq);
-                    tma_load_3d(sQ + kTileBytes + kPanelBytes, &tm_q, &sh->q_full, 64, it.head + it.dh, tok_q + it.dq);
+                    tma_load_3d_hint(sQ + kTileBytes, &tm_q, &sh->q_full, 0, it.head + it.dh, tok_q + it.dq, once);
+                    tma_load_3d_hint(sQ + kTileBytes + kPanelBytes, &tm_q, &sh->q_full, 64, it.head + it.dh, tok_q + it.dq, once);
                 }
                 for (int j = 0; j < it.n_kv; ++j, ++kt) {
                     const int tok = kv_tile_token(p, it, j);
@@ -731,6 +765,8 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 more = __shfl_sync(0xffffffffu, more, 0);
             }
         } else if (lane == 0) {
+            const List list = list_of(p);
+            const int total = tmem != 0xFFFFFFFFu ? items_of(p, list) : 0;
             uint32_t k = 0;
             int idx = blockIdx.x;
             while (true) {
@@ -740,7 +776,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 do {
                     if (k > 0 || idx != (int)blockIdx.x) idx = claim_item(p);
                     it.n_kv = -1;
-                    if (idx < total) it = load_item(p, idx);
+                    if (idx < total) it = load_item(p, list, idx);
                     if (it.n_kv == 0) idx = total;  // nothing to do there: claim another one
                 } while (it.n_kv == 0);
                 sh->items[slot] = it;
@@ -1032,8 +1068,9 @@ constexpr int kCombineThreads = 128;
 __global__ void __launch_bounds__(kCombineThreads) prefill_combine_kernel(const __grid_constant__ SplitParams p) {
     griddep_wait();
     const int e = blockIdx.x, x = blockIdx.y, row = blockIdx.z * 8 + (threadIdx.x >> 4), c8 = (threadIdx.x & 15) * 8;
-    if (e >= p.items[0].x * p.per_pair || splits_of(p) == 1) return;
-    const Item it = load_item(static_cast<const Params&>(p), e);
+    const List list = list_of(p);
+    if (e >= items_of(static_cast<const Params&>(p), list) || splits_of(p, list.pairs) == 1) return;
+    const Item it = load_item(static_cast<const Params&>(p), list, e);
     const int runs = runs_of(p.splits, it.n_a);
     const int q_pos = it.q0 + x * it.dq + row;
     if ((x == 0 ? it.n_a : it.n_b) == 0 || runs == 1 || q_pos >= it.len) return;
@@ -1231,7 +1268,8 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
         cfg.gridDim = dim3(1);
         cfg.blockDim = dim3(kPlanThreads);
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, prefill_plan_kernel, cu_seqlens_q, cu_seqlens_k, block_tables ? 1 : 0, B,
-                                         (int4*)workspace, (int)cap, scatter && pdl_enabled() ? 1 : 0));
+                                         (int4*)workspace, (int)cap, p.per_pair, KVH, ctas,
+                                         scatter && pdl_enabled() ? 1 : 0));
     }
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(kThreads);

@@ -110,3 +110,17 @@ def test_short_launches_find_every_row_block_once_and_the_long_ones_first(lens, 
     assert sorted(order) == sorted(blocks_of(lens)) and len(set(order)) == len(order)
     levels = [level for _, level in order]
     assert levels == sorted(levels, reverse=True)
+
+
+@pytest.mark.parametrize("pairs,per_pair,groups", [(1, 8, 1), (7, 8, 2), (5, 24, 4), (13, 6, 2), (3, 8, 8)])
+def test_head_groups_take_every_item_once_and_a_groups_heads_together(pairs, per_pair, groups):
+    """load_item: item -> (pair, item of the pair)."""
+    per, found = per_pair // groups, []
+    for idx in range(pairs * per_pair):
+        first = idx // (pairs * per) * per
+        rest = idx - first * pairs
+        found.append((rest // per, first + rest % per))
+    assert sorted(found) == [(p, r) for p in range(pairs) for r in range(per_pair)]
+    for g in range(groups):
+        part = found[g * pairs * per:(g + 1) * pairs * per]
+        assert {r // per for _, r in part} == {g} and [p for p, _ in part] == sorted(p for p, _ in part)
