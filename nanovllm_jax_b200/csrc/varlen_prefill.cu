@@ -9,18 +9,23 @@
 // prefix = len_k - len_q; the model runner attaches the tables on a prefix hit,
 // engine/model_runner.py:311-314).
 //
-// Work item = two 128-row Q tiles (A and B) that share every K/V tile they read: the same 128
-// query rows of two q heads of one kv head -- both see the same keys, run the same number of K/V tiles and finish
-// together -- or, for the last head of an odd group, two consecutive row blocks of it (B then sees one
-// K/V tile more than A).  A tiny plan kernel turns cu_seqlens into the list of
-// (sequence, row block) pairs, longest causal span first; one persistent CTA per SM
+// Work item = two 128-row Q tiles (A and B) that share every K/V tile they read.  A row is a (token, head) pair: the item takes
+// a block of consecutive tokens and all q heads of one kv head, half of the heads in each tile -- both see the same keys, run
+// the same number of K/V tiles and finish together -- or, where their number is odd, all of them in both tiles, which hold
+// one half of the tokens each (B may then see one K/V tile more than A); see Pack.  A tiny plan kernel turns cu_seqlens into
+// the list of (sequence, token block) pairs, longest causal span first; one persistent CTA per SM
 // starts on the item of its number and claims the others one by one (heavy ones first, so the CTAs finish
-// together), and the heads of one (sequence, row block) are neighbours in the list so
-// that the G heads of a kv head find each other's K/V tiles in L2.  Tensor memory and
+// together), and the kv heads go in groups whose keys and values fit the L2 (head_groups).  Tensor memory and
 // barriers are set up once per CTA; the loads of the next item are already in flight
 // while the current one drains.  Where the host knows that there is at most one item per SM, every CTA finds its own from
 // cu_seqlens instead (ShortParams), and the step's K/V scatter runs on the SMs the items leave.  Few items with many keys are cut into runs of
 // K/V tiles (SplitParams) that a small kernel behind this one combines.
+//
+// Rows that are (token, head) pairs leave fewer of them behind the sequences' ends than rows of 128 tokens of one head, and
+// tiles that span few tokens cut the products short at the diagonal.  us per call, before -> after:
+// 48 prompts of 5..300 tokens, 10 / 2 heads, 35.0 -> 28.4; 30 of 65..192, 64 / 8, 64.0 -> 46.7; 32 of 300, 32 / 8, 86.8 -> 74.1;
+// 12 of 17..700 behind 500..5000 cached ones, 32 / 8, 257 -> 238; 16 of 128..4096, 32 / 8, 880 -> 869; one of 8192, 64 / 8,
+// 1059.5 -> 1059.5.
 //
 // Per CTA (12 warps = 3 warpgroups; the first gives registers away with setmaxnreg, the softmax
 // warpgroups take them):
@@ -74,18 +79,43 @@ constexpr int kTileBytes = 2 * kPanelBytes;
 constexpr int kSlots = 5;                // one ring for K and V tiles, filled in the order K0 V0 K1 V1 ...
 constexpr int kSmemTiles = (2 + kSlots) * kTileBytes;  // Q_A Q_B | K/V ring  (224 KB)
 constexpr int kSmemBytes = kSmemTiles + 512 + 1024;  // barriers and item records, alignment slack
-constexpr int kMaxLevels = 4096;       // row blocks per sequence the plan kernel can rank
+constexpr int kMaxLevels = 4096;       // K/V tiles per sequence the plan kernel can rank items by
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 
-constexpr int kShortBlocks = 32;       // a short launch has at most so many row blocks ...
+constexpr int kShortBlocks = 64;       // a short launch has at most so many token blocks ...
 constexpr int kShortSequences = 32;    // ... of so many sequences: a lane of a warp for each
 
-// A (sequence, row block) pair, longest causal span first: {first query token of the sequence, its query length, first
-// row of the block, sequence index} and {first key token (packed keys), key length, 0, 0}.
+// A (sequence, token block) pair, longest causal span first: {first query token of the sequence, its query length, first
+// token of the block, sequence index} and {first key token (packed keys), key length, 0, 0}.
 struct Record {
     int4 q, k;
 };
+
+// What a Q tile holds: `tokens` consecutive tokens of `heads` neighbouring q heads of one kv head, token after token, and what
+// the item's second tile holds beside it.  All heads of a kv head see the same keys, so the narrower the block of tokens, the
+// fewer rows lie behind a sequence's end and the more of a diagonal tile is behind every row (skipped, see key_steps).
+struct Pack {
+    int heads, tokens;  // of a tile
+    int dq, dh;         // tile B: dq tokens further, or dh heads further
+    int span;           // tokens of an item
+    int per_kv;         // items per kv head and token block
+};
+// A kv head's G q heads in one item, half of them per tile: both tiles then see the same keys and finish together.  An odd
+// number goes into both tiles, which take tokens in turn (B may see one K/V tile more).  Groups of more than eight heads are
+// cut into equal parts.
+static Pack make_pack(int G) {
+    int w = std::min(G, 8);
+    while (G % w) --w;
+    Pack k;
+    k.heads = w % 2 ? w : w / 2;
+    k.tokens = kTileQ / k.heads;
+    k.dq = w % 2 ? k.tokens : 0;
+    k.dh = w % 2 ? 0 : k.heads;
+    k.span = w % 2 ? 2 * k.tokens : k.tokens;
+    k.per_kv = G / w;
+    return k;
+}
 
 struct Params {
     const int4* items;  // record 0: {number of pairs, items claimed, head groups, 0}; then the two halves of every Record
@@ -93,7 +123,8 @@ struct Params {
     int MB, block_size;
     __nv_bfloat16* out;
     int H, G;
-    int per_pair;  // items per (sequence, row block): two heads of one kv head each, a lone head where G is odd
+    Pack pack;
+    int per_pair;  // items per (sequence, token block)
     int wide;      // out is aligned to 32 bytes
     float scale_log2;
 };
@@ -116,18 +147,23 @@ struct SplitParams : Params {
     int ctas;  // the launch's
 };
 constexpr int kPartialFloats = kTileQ * kD + 2 * kTileQ;  // O[128][128] relative to m, then m[128] (log2 units) and l[128]
-constexpr int kMinRun = 4;  // tiles per run: at least one of them is visible to every row (at most two or three are masked)
+// K/V tiles per run.  A row that sees none of a run's keys would have no maximum.  An item's first token sees all of its tiles
+// but one (two where the item has more tokens than a tile keys).
+__host__ __device__ __forceinline__ int min_run(int span) { return span > kTileKV ? 3 : 2; }
 // Items of fewer tiles stay whole: they take less time than the partial results and the combining launch (about 6 us).  The
-// rule looks at an item's own tiles, so that packed keys and keys in pages give the same bits.
-// 100 new tokens behind 8000 cached ones: 130 -> 42 us with 32 / 8 heads, 33 with 8 / 1; one prompt of 4000 tokens, 4 / 1
-// heads: 63 -> 50, of 1200 (ten tiles), 8 / 2: 25 -> 28 if it were cut.
-constexpr int kSplitTiles = 12;
+// rule looks at an item's own tiles, so that packed keys and keys in pages give the same bits.  us per call, whole / cut at
+// twelve tiles into runs of four / at eight into runs of two: 100 new tokens behind 8000 cached ones, 32 / 8 heads, 130 / 35 /
+// 35, 8 / 1 heads 32.0 cut at twelve, 29.9 at eight; 20 behind 1200, 16 / 2: 27.6 / 27.6 / 19.6; 8 of 10..40 behind 900..1400, 8 / 1: 31.3 / 31.3
+// / 23.7; one prompt of 1500, 8 / 1: 34.6 / 34.6 / 28.0, of 4000, 4 / 1: 63 / 48.6 / 49.1.
+constexpr int kSplitTiles = 8;
 // The launch has a CTA for every run that the host could foresee.  Where the device's lengths make more items than that (a
 // captured launch whose lengths were rewritten), the items stay whole and the CTAs claim them one by one.
 __device__ __forceinline__ int splits_of(const SplitParams& p, int pairs) {
     return (long long)pairs * p.per_pair * p.splits <= p.ctas ? p.splits : 1;
 }
-__device__ __forceinline__ int runs_of(int splits, int n_a) { return n_a < kSplitTiles ? 1 : min(splits, n_a / kMinRun); }
+__device__ __forceinline__ int runs_of(const Params& p, int splits, int n_a) {
+    return n_a < kSplitTiles ? 1 : min(splits, n_a / min_run(p.pack.span));
+}
 
 __device__ __forceinline__ Record record_of(const Params& p, int pair) {
     return Record{__ldg(p.items + 1 + 2 * pair), __ldg(p.items + 2 + 2 * pair)};
@@ -283,11 +319,12 @@ __device__ __forceinline__ uint64_t mnmajor_desc(uint32_t tile_addr, int ks) {
     return make_desc(tile_addr + ks * 16 * 128, kPanelBytes, 1024);
 }
 
-constexpr uint32_t kIdescQK = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-constexpr uint32_t kIdescPV = kIdescQK | (1u << 16);  // B operand MN-major
+constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 4) << 24);
+constexpr uint32_t idesc_qk(uint32_t keys) { return kIdesc | ((keys >> 3) << 17); }
+constexpr uint32_t kIdescPV = kIdesc | ((128u >> 3) << 17) | (1u << 16);  // B operand MN-major
 
 // ------------------------------------------------------------------------------------------
-// plan kernel: (sequence, row block) pairs sorted by causal span, largest first
+// plan kernel: (sequence, token block) pairs sorted by causal span, largest first
 // ------------------------------------------------------------------------------------------
 // Longest spans first means that all sequences are in flight at once.  Where their keys and values do not fit the L2 the kv
 // heads are taken in groups whose keys and values do, one group after the other, as long as each is long enough for its CTAs to
@@ -305,12 +342,18 @@ __device__ int head_groups(long long keys, int pairs, int per_pair, int KVH, int
     return n;
 }
 
+// K/V tiles in front of the last one that block l of a sequence sees.
+__device__ __forceinline__ int level_of(int len, int len_k, int l, int span) {
+    const int last = min(len, (l + 1) * span) - 1 + max(len_k - len, 0);  // position of the block's last token
+    return min(last / kTileKV, kMaxLevels - 1);
+}
+
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_t* __restrict__ cu_seqlens,
                                                                     const int32_t* __restrict__ cu_k, int paged, int B,
-                                                                    int4* __restrict__ items, int capacity, int per_pair,
-                                                                    int KVH, int ctas, int behind_store) {
-    // A row block's weight is its causal span in blocks of 128 keys: level = prefix / 128 + block index.
+                                                                    int4* __restrict__ items, int capacity, int span,
+                                                                    int per_pair, int KVH, int ctas, int behind_store) {
+    // A token block's level is the number of K/V tiles in front of its last one (level_of).
     __shared__ int hist[kMaxLevels];
     __shared__ int base[kMaxLevels];
     __shared__ int max_level, bad;
@@ -326,7 +369,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
     for (int i = threadIdx.x; i < kMaxLevels; i += blockDim.x) hist[i] = 0;
     if (threadIdx.x == 0) max_level = 0, bad = 0, keys = 0;
     __syncthreads();
-    // few sequences: a warp each, its lanes take the row blocks; many: a thread each
+    // few sequences: a warp each, its lanes take the token blocks; many: a thread each
     const bool by_warp = B <= 256;
     const int b0 = by_warp ? threadIdx.x >> 5 : threadIdx.x, db = by_warp ? kPlanThreads / 32 : kPlanThreads;
     const int l0 = by_warp ? threadIdx.x & 31 : 0, dl = by_warp ? 32 : 1;
@@ -335,14 +378,14 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
         const int len_k = cu_k[b + 1] - cu_k[b];
         // keys can never be fewer than queries; packed keys sit beside the queries, so the counts must be equal
         if (len > 0 && (len_k < len || (!paged && (len_k != len || cu_k[b] != cu_seqlens[b])))) bad = 1;
-        const int lvl0 = len_k > len ? (len_k - len) / kTileQ : 0;
-        const int n = len > 0 ? (len + kTileQ - 1) / kTileQ : 0;
+        const int n = len > 0 ? (len - 1) / span + 1 : 0;
         if (n > 0 && l0 == 0) {
-            atomicMax(&max_level, min(lvl0 + n, kMaxLevels));
+            const int tiles = (max(len, len_k) - 1) / kTileKV + 1;
+            atomicMax(&max_level, min(tiles, kMaxLevels));
             atomicAdd(&keys, (unsigned long long)len_k);
-            if (lvl0 + n > kMaxLevels) atomicOr(&g_error_flag, 16);
+            if (tiles > kMaxLevels) atomicOr(&g_error_flag, 16);
         }
-        for (int l = l0; l < n; l += dl) atomicAdd(&hist[min(lvl0 + l, kMaxLevels - 1)], 1);
+        for (int l = l0; l < n; l += dl) atomicAdd(&hist[level_of(len, len_k, l, span)], 1);
     }
     __syncthreads();
     if (bad) {  // uniform: publish an empty list so that the main kernel computes nothing
@@ -375,12 +418,11 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
         const int start = cu_seqlens[b];
         const int len = cu_seqlens[b + 1] - start;
         const int len_k = cu_k[b + 1] - cu_k[b];
-        const int lvl0 = len_k > len ? (len_k - len) / kTileQ : 0;
-        const int n = len > 0 ? (len + kTileQ - 1) / kTileQ : 0;
+        const int n = len > 0 ? (len - 1) / span + 1 : 0;
         for (int l = l0; l < n; l += dl) {
-            const int slot = atomicAdd(&base[min(lvl0 + l, kMaxLevels - 1)], 1);
+            const int slot = atomicAdd(&base[level_of(len, len_k, l, span)], 1);
             if (slot < capacity) {
-                items[1 + 2 * slot] = make_int4(start, len, l * kTileQ, b);
+                items[1 + 2 * slot] = make_int4(start, len, l * span, b);
                 items[2 + 2 * slot] = make_int4(cu_k[b], len_k, 0, 0);
             }
         }
@@ -395,12 +437,11 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
 // main kernel
 // ------------------------------------------------------------------------------------------
 struct Item {
-    int seq_start, len, q0, head;      // first query token of the sequence, query length, first row of the block, first head
+    int seq_start, len, q0, head;      // first query token of the sequence, query length, first token of the block, first head
     int k_start, len_k, prefix, kvh;   // first key token (packed keys), key length, len_k - len, kv head
     int n_a, n_b, n_kv, b;             // KV tiles seen by Q tile A, by Q tile B (0: no such rows; else n_a or n_a + 1), the
                                        // larger (0: nothing to do; -1: no more items), sequence
-    int dq, dh, ragged, kv0;           // Q tile B = rows + dq of head + dh; the last KV tile reaches past the last key; a run
-                                       // of a split item: its first KV tile (len_k and prefix count from there on), else -1
+    int kv0;                           // a run of a split item: its first KV tile (len_k and prefix count from there on), else -1
 };
 constexpr int kItemRing = 2;
 constexpr int kItemReaders = 3 + 8;    // TMA producer, two MMA issuers, eight softmax warps
@@ -427,16 +468,18 @@ __device__ __forceinline__ bool wait_or_abort(Shared* sh, uint64_t* bar, uint32_
     return false;
 }
 
-// Item r (of per_pair) of a (sequence, row block).
+// Keys up to the last one that a row of Q tile x sees, counted from the item's first K/V tile.
+__device__ __forceinline__ int visible_keys(const Params& p, const Item& it, int x) {
+    return it.prefix + min(it.len, it.q0 + x * p.pack.dq + p.pack.tokens);
+}
+// Steps of 16 keys of the tile's n-th and last K/V tile that hold any of them: what its two products go through.
+__device__ __forceinline__ int key_steps(int keys, int n) { return (min(kTileKV, keys - (n - 1) * kTileKV) + 15) >> 4; }
+
+// Item r (of per_pair) of a (sequence, token block).
 __device__ __forceinline__ Item make_item(const Params& p, const Record& rec, int r) {
     Item it;
-    const int per_kv = (p.G + 1) >> 1;      // items per kv head
-    it.kvh = r / per_kv;
-    const int h2 = 2 * (r - it.kvh * per_kv);  // first of the item's heads within the kv head
-    const bool two = h2 + 1 < p.G;
-    it.head = it.kvh * p.G + h2;
-    it.dq = two ? 0 : kTileQ;
-    it.dh = two ? 1 : 0;
+    it.kvh = r / p.pack.per_kv;
+    it.head = it.kvh * p.G + (r - it.kvh * p.pack.per_kv) * (p.G / p.pack.per_kv);
     const int4 q = rec.q, k = rec.k;
     it.seq_start = q.x;
     it.len = q.y;
@@ -445,15 +488,9 @@ __device__ __forceinline__ Item make_item(const Params& p, const Record& rec, in
     it.k_start = k.x;
     it.len_k = k.y;
     it.prefix = it.len_k - it.len;  // >= 0: the plan kernel publishes no items otherwise
-    const int nk_total = (it.len_k + kTileKV - 1) / kTileKV;
-    // the last row of Q tile x sees keys 0 .. prefix + q0 + 128 x + 127
-    it.n_a = min(nk_total, (it.prefix + it.q0 + kTileQ - 1) / kTileKV + 1);
-    it.n_b = two ? it.n_a
-                 : (it.len - it.q0 > kTileQ ? min(nk_total, (it.prefix + it.q0 + 2 * kTileQ - 1) / kTileKV + 1) : 0);
-    // a lone head takes two row blocks at a time, on the even ones
-    if (!two && ((it.q0 / kTileQ) & 1)) it.n_a = it.n_b = 0;
+    it.n_a = (visible_keys(p, it, 0) - 1) / kTileKV + 1;
+    it.n_b = it.len - it.q0 > p.pack.dq ? (visible_keys(p, it, 1) - 1) / kTileKV + 1 : 0;
     it.n_kv = max(it.n_a, it.n_b);
-    it.ragged = it.n_kv * kTileKV > it.len_k;
     it.kv0 = -1;
     return it;
 }
@@ -471,7 +508,7 @@ __device__ __forceinline__ Item load_item(const Params& p, const List& l, int id
 __device__ __forceinline__ Item load_item(const SplitParams& p, const List& l, int idx) {
     const int splits = splits_of(p, l.pairs), c = idx % splits;
     Item it = load_item(static_cast<const Params&>(p), l, idx / splits);
-    const int runs = runs_of(splits, it.n_a);
+    const int runs = runs_of(p, splits, it.n_a);
     if (runs == 1) {
         if (c > 0) it.n_a = it.n_b = it.n_kv = 0;
         return it;
@@ -487,7 +524,6 @@ __device__ __forceinline__ Item load_item(const SplitParams& p, const List& l, i
     it.n_kv = j1 - j0;
     it.len_k -= j0 * kTileKV;
     it.prefix -= j0 * kTileKV;
-    it.ragged = it.n_kv * kTileKV > it.len_k;
     return it;
 }
 
@@ -516,13 +552,15 @@ __device__ __forceinline__ void store_32bytes(void* dst, const uint32_t (&w)[8])
 }
 
 // One 128-column S row -> running max, optional O rescale, bf16 P in two halves.  DIAG: key column c of this tile is
-// visible iff c <= lim (lim may be negative -- nothing visible in this tile -- or >= 127).  turn_bar (or null): the
+// visible iff c <= lim (lim may be negative -- nothing visible in this tile -- or >= 127), and the limits of the warp's rows
+// lie in warp_lo .. warp_hi; columns behind every limit may hold anything.  turn_bar (or null): the
 // other tile's hand-over this tile's exponentials wait for; turn_out (or null): where this tile hands over.
 // The whole row is held in registers (the softmax warpgroups raise their register budget with setmaxnreg), so
 // tensor memory is read once and its latency is paid once per tile.
 template <bool DIAG>
 __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint32_t t_s, const uint32_t t_o,
-                                             const int lim, const bool first, const uint32_t o_parity_prev,
+                                             const int lim, const int warp_lo, const int warp_hi, const bool first,
+                                             const uint32_t o_parity_prev,
                                              const float scale_log2, float& m_run, float& m_used, float& l,
                                              uint64_t* turn_bar, const uint32_t turn_parity, uint64_t* turn_out) {
     uint32_t v[4][32];
@@ -532,12 +570,11 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
     tmem_ld32(t_s + 96, v[3]);
     tmem_wait_ld();
     float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-    const int warp_lim = lim - (int)(threadIdx.x & 31);  // limit of the warp's first row; the others' follow one by one
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         if (DIAG) {
-            if (32 * c > warp_lim + 31) continue;  // nothing of this chunk is visible to any row of the warp
-            if (32 * c + 31 > warp_lim) {          // mask in place so that the second pass needs no select
+            if (32 * c > warp_hi) continue;  // nothing of this chunk is visible to any row of the warp
+            if (32 * c + 31 > warp_lo) {     // mask in place so that the second pass needs no select
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
                     if (c * 32 + i > lim) v[c][i] = 0xFF800000u;
@@ -583,7 +620,7 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
     uint64_t acc_a = pack2(0.f, 0.f), acc_b = pack2(0.f, 0.f);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        if (DIAG && 32 * c > warp_lim + 31) {
+        if (DIAG && 32 * c > warp_hi) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[c][i] = 0u;
         } else {
@@ -670,6 +707,13 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
     }
+    // Rows of the Q tiles that no load fills (128 is not a multiple of the packed heads): their scores must not vary, since a
+    // warp's rows vote on when to rescale.
+    for (int i = p.pack.heads * p.pack.tokens * 8 + tid; i < kTileQ * 8; i += kThreads) {
+#pragma unroll
+        for (int panel = 0; panel < 4; ++panel) *reinterpret_cast<uint4*>(sQ + panel * kPanelBytes + i * 16) = make_uint4(0, 0, 0, 0);
+        fence_proxy_async_smem();
+    }
     __syncthreads();
     if (warp == 1) {
         tmem_alloc(&sh->tmem_base, kTmemCols);
@@ -698,12 +742,12 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 const int kvh = it.kvh;
                 const int tok_q = it.seq_start + it.q0;
                 if (i > 0 && !(ok = wait_or_abort(sh, &sh->q_empty, (i - 1) & 1u))) break;
-                mbar_expect_tx(&sh->q_full, (it.n_b > 0 ? 2 : 1) * kTileBytes);
+                mbar_expect_tx(&sh->q_full, (it.n_b > 0 ? 4u : 2u) * 128u * (uint32_t)(p.pack.heads * p.pack.tokens));
                 tma_load_3d_hint(sQ, &tm_q, &sh->q_full, 0, it.head, tok_q, once);
                 tma_load_3d_hint(sQ + kPanelBytes, &tm_q, &sh->q_full, 64, it.head, tok_q, once);
                 if (it.n_b > 0) {
-                    tma_load_3d_hint(sQ + kTileBytes, &tm_q, &sh->q_full, 0, it.head + it.dh, tok_q + it.dq, once);
-                    tma_load_3d_hint(sQ + kTileBytes + kPanelBytes, &tm_q, &sh->q_full, 64, it.head + it.dh, tok_q + it.dq, once);
+                    tma_load_3d_hint(sQ + kTileBytes, &tm_q, &sh->q_full, 0, it.head + p.pack.dh, tok_q + p.pack.dq, once);
+                    tma_load_3d_hint(sQ + kTileBytes + kPanelBytes, &tm_q, &sh->q_full, 64, it.head + p.pack.dh, tok_q + p.pack.dq, once);
                 }
                 for (int j = 0; j < it.n_kv; ++j, ++kt) {
                     const int tok = kv_tile_token(p, it, j);
@@ -729,10 +773,10 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // heaviest items first the CTAs finish together (dealt round-robin, the CTAs with the heaviest items of every round
         // also got the ones left over: 257 us for the last of 148, 209 for the median one).
         if constexpr (kShort) {
-            // Lane b has sequence b.  Items go by row block, the last ones (the longest spans) first.
+            // Lane b has sequence b.  Items go by token block, the last ones (the longest spans) first.
             const int start = lane < p.B ? __ldg(p.cu_seqlens + lane) : 0;
             const int len = lane < p.B ? __ldg(p.cu_seqlens + lane + 1) - start : 0;
-            const int blocks = len > 0 ? (len + kTileQ - 1) / kTileQ : 0;
+            const int blocks = len > 0 ? (len - 1) / p.pack.span + 1 : 0;
             const int items = tmem != 0xFFFFFFFFu ? __reduce_add_sync(0xffffffffu, blocks) * p.per_pair : 0;
             const int levels = __reduce_max_sync(0xffffffffu, blocks);
             uint32_t k = 0;
@@ -745,7 +789,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     for (; at >= __popc(has); has = __ballot_sync(0xffffffffu, blocks > level)) at -= __popc(has), --level;
                     const bool mine = blocks > level && __popc(has & ((1u << lane) - 1)) == at;
                     const int b = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
-                    q = make_int4(__shfl_sync(0xffffffffu, start, b), __shfl_sync(0xffffffffu, len, b), level * kTileQ, b);
+                    q = make_int4(__shfl_sync(0xffffffffu, start, b), __shfl_sync(0xffffffffu, len, b), level * p.pack.span, b);
                 }
                 if (lane == 0) {
                     Item it;
@@ -810,16 +854,28 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             // behind_pv: o_full(j-1) is committed in front of s_full(j), so that a softmax warp that has seen S(j) finds that
             // phase of o_full complete.  The other way round a warp that skips the softmax (its rows lie behind the
             // sequence's end) could be at its wait for o_full(j) a phase too early, where the parity aliases.
-            auto issue_qk = [&](uint64_t kd, bool behind_pv) {
+            //
+            // A tile's last products leave out the keys behind every row (key_steps).  They are code of their own: with the key
+            // count as a variable in the others long prompts were 2 % slower (1 of 8192 tokens, 64 / 8 heads: 1049 -> 1074 us).
+            auto issue_qk = [&](uint64_t kd, bool behind_pv, auto last, int steps) {
+                if constexpr (decltype(last)::value) {
+                    const uint32_t idesc = idesc_qk(16 * steps);
+#pragma unroll 1
+                    for (int ks = 0; ks < 8; ++ks) {
+                        const uint32_t step = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
+                        mma_ss(s_t, q_desc + step, kd + step, idesc, ks > 0);
+                    }
+                } else {
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint32_t step = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
-                    mma_ss(s_t, q_desc + step, kd + step, kIdescQK, ks > 0);
+                    for (int ks = 0; ks < 8; ++ks) {
+                        const uint32_t step = (uint32_t)(((ks >> 2) * kPanelBytes + (ks & 3) * 32) >> 4);
+                        mma_ss(s_t, q_desc + step, kd + step, idesc_qk(kTileKV), ks > 0);
+                    }
                 }
                 if (behind_pv) tc_commit(&sh->o_full[x]);
                 tc_commit(&sh->s_full[x]);
             };
-            auto issue_pv = [&](int j, uint64_t vd) -> bool {
+            auto issue_pv = [&](int j, uint64_t vd, auto last, int steps) -> bool {
                 if (j == 0 && used > 0 && !wait_or_abort(sh, &sh->o_empty[x], (used - 1) & 1u)) return false;
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
@@ -827,7 +883,8 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     tc_fence_after();
 #pragma unroll
                     for (int ks = half * 4; ks < half * 4 + 4; ++ks)
-                        mma_ts(o_t, s_t + ks * 8, vd + (uint32_t)((ks * 16 * 128) >> 4), kIdescPV, (j > 0 || ks > 0));
+                        if (!decltype(last)::value || ks < steps)
+                            mma_ts(o_t, s_t + ks * 8, vd + (uint32_t)((ks * 16 * 128) >> 4), kIdescPV, (j > 0 || ks > 0));
                 }
                 ++tiles;
                 return true;
@@ -835,10 +892,13 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             // the slot holding ring position pos: K(j) sits at 2j, V(j) at 2j+1
             auto slot_full = [&](uint32_t pos) { return wait_or_abort(sh, &sh->kv_full[pos % kSlots], (pos / kSlots) & 1u); };
 
+            const std::false_type full;
+            const std::true_type last;
             Item it;
             while (ok && next_item(sh, i, it)) {
                 mbar_arrive(&sh->item_empty[i % kItemRing]);
                 const int n_x = x == 0 ? it.n_a : it.n_b;
+                const int steps = key_steps(visible_keys(p, it, x), n_x);  // of the last tile
                 if (!(ok = wait_or_abort(sh, &sh->q_full, i & 1u))) break;
                 if (n_x == 0) mbar_arrive(&sh->q_empty);  // this tile never reads the Q buffer of this item
                 {
@@ -846,7 +906,11 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     if (!(ok = slot_full(kpos))) break;
                     if (n_x > 0) {
                         tc_fence_after();
-                        issue_qk(k_desc0 + (kpos % kSlots) * kSlotStep, false);
+                        const uint64_t kd = k_desc0 + (kpos % kSlots) * kSlotStep;
+                        if (n_x > 1)
+                            issue_qk(kd, false, full, 8);
+                        else
+                            issue_qk(kd, false, last, steps);
                         tc_commit(&sh->kv_empty[kpos % kSlots]);
                         if (n_x == 1) tc_commit(&sh->q_empty);
                     } else {
@@ -858,8 +922,11 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     if (!(ok = slot_full(vpos))) break;
                     if (j + 1 < it.n_kv && !(ok = slot_full(kpos))) break;
                     if (j < n_x) {
-                        if (!(ok = issue_pv(j, v_desc0 + (vpos % kSlots) * kSlotStep))) break;
-                        if (!(j + 1 < n_x)) {
+                        const uint64_t vd = v_desc0 + (vpos % kSlots) * kSlotStep;
+                        if (j + 1 < n_x) {
+                            if (!(ok = issue_pv(j, vd, full, 8))) break;
+                        } else {
+                            if (!(ok = issue_pv(j, vd, last, steps))) break;
                             tc_commit(&sh->o_full[x]);
                             tc_commit(&sh->kv_empty[vpos % kSlots]);
                         }
@@ -868,7 +935,11 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     }
                     if (j + 1 < it.n_kv) {
                         if (j + 1 < n_x) {
-                            issue_qk(k_desc0 + (kpos % kSlots) * kSlotStep, true);
+                            const uint64_t kd = k_desc0 + (kpos % kSlots) * kSlotStep;
+                            if (j + 2 < n_x)
+                                issue_qk(kd, true, full, 8);
+                            else
+                                issue_qk(kd, true, last, steps);
                             tc_commit(&sh->kv_empty[kpos % kSlots]);
                             tc_commit(&sh->kv_empty[vpos % kSlots]);
                             if (j + 2 == n_x) tc_commit(&sh->q_empty);  // this tile's last Q.K^T has been issued
@@ -888,7 +959,9 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         // ============================ softmax warpgroups ============================
         const int x = (warp - 4) >> 2;              // 0: tile A, 1: tile B
         const int quarter = warp & 3;               // tensor-memory lane quarter this warp may touch
-        const int row = quarter * 32 + lane;        // row within the Q tile
+        const int row = quarter * 32 + lane;        // row within the Q tile: a token and a head
+        const int tok = row / p.pack.heads, tok_head = row - tok * p.pack.heads;
+        const int tok_lo = quarter * 32 / p.pack.heads, tok_hi = (quarter * 32 + 31) / p.pack.heads;  // the warp's tokens
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const uint32_t t_s = tmem + x * 128 + lane_base;
         const uint32_t t_o = tmem + 256 + x * 128 + lane_base;
@@ -916,8 +989,10 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             // 51.3 with).  With two the turns pay: 16 prompts of 256 tokens 35.7 us without, 34.4 with; five of 390..472, 64 / 8
             // heads, 47.5 and 46.0; 48 of 5..300, 10 / 2 heads, 33.5 and 33.8.
             const bool both = it.n_b > 0 && it.n_a > 1;
-            const int q_pos = it.q0 + x * it.dq + row;             // row of the sequence's query block
-            const int first_lim = it.prefix + it.q0 + x * it.dq;  // last key visible to the first row of this Q tile
+            const int q_pos = it.q0 + x * p.pack.dq;      // first token of this Q tile
+            const int first_lim = it.prefix + q_pos;      // last key visible to it
+            const bool ragged = 16 * key_steps(visible_keys(p, it, x), n_x) + (n_x - 1) * kTileKV > it.len_k;
+            const int live = min(p.pack.tokens, it.len - q_pos);  // tokens of the tile in front of the sequence's end
             float m_run = -INFINITY, m_used = -INFINITY, l = 0.f;
             // One KV tile of this Q tile.  Tiles whose last key the tile's first row may still see need no mask; the
             // one or two after them (one when the prefix is a multiple of the tile) are masked per element.  The two
@@ -933,7 +1008,9 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     ++turns_seen;
                 }
                 tc_fence_after();
-                if ((kDiag || kDead) && it.ragged && j == it.n_kv - 1) {
+                // keys of this tile that the products go through, and how many of them are the sequence's
+                if ((kDiag || kDead) && ragged && j == n_x - 1) {
+                    const int through = 16 * key_steps(visible_keys(p, it, x), n_x), own = it.len_k - j * kTileKV;
                     // The last KV tile of the sequence reaches past its last key: those rows of the V tile hold
                     // whatever follows in memory (the next sequence, padding, recycled cache rows).  Their
                     // probabilities are exactly zero, but 0 * NaN or 0 * Inf in the P.V product would still poison the
@@ -943,9 +1020,9 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     // issuer, and the slot cannot be refilled before P.V of this very tile, so the parity wait sees
                     // either "still loading" or "landed", never another tile.  When both Q tiles use the tile both
                     // warpgroups zero it (same bytes, same value).  (Such a tile is always a masked one.)
-                    const uint32_t vpos = 2 * (kt0 + it.n_kv - 1) + 1;
+                    const uint32_t vpos = 2 * (kt0 + j) + 1;
                     if (!wait_or_abort(sh, &sh->kv_full[vpos % kSlots], (vpos / kSlots) & 1u)) return false;
-                    if (row >= it.len_k - (it.n_kv - 1) * kTileKV) {
+                    if (row >= own && row < through) {
                         // a row is 128 contiguous bytes in each 64-dim panel (the swizzle permutes inside a row)
                         uint8_t* vrow = sKV + (vpos % kSlots) * kTileBytes + row * 128;
 #pragma unroll
@@ -968,7 +1045,9 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     ++tiles;
                     return true;
                 }
-                if (!softmax_tile<kDiag>(sh, x, t_s, t_o, kDiag ? first_lim - j * kTileKV + row : 0, j == 0,
+                const int lim = first_lim - j * kTileKV;
+                if (!softmax_tile<kDiag>(sh, x, t_s, t_o, kDiag ? lim + min(tok, live - 1) : 0, kDiag ? lim + min(tok_lo, live - 1) : 0,
+                                         kDiag ? lim + min(tok_hi, live - 1) : 0, j == 0,
                                          (tiles - 1) & 1u, p.scale_log2, m_run, m_used, l, turn_bar, turn_parity,
                                          (both && (x == 0 || j + 1 < it.n_a)) ? &sh->turn[x] : nullptr))
                     return false;
@@ -978,7 +1057,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             };
             const int n_plain = min(n_x, (first_lim + 1) / kTileKV);  // tiles j with j * 128 + 127 <= first_lim
             int j = 0;
-            const bool dead = q_pos - lane >= it.len;  // the whole warp lies behind the sequence's last row
+            const bool dead = tok_lo >= live;  // the whole warp lies behind the sequence's last row
             if (dead) {
                 for (; ok && j < n_x; ++j) ok = tile_step(j, std::integral_constant<int, 2>{});
             } else {
@@ -1016,14 +1095,15 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 }
             }
             const float inv = 1.0f / l;
-            __nv_bfloat16* orow = p.out + ((size_t)(it.seq_start + q_pos) * p.H + it.head + x * it.dh) * kD;
+            const int head = it.head + x * p.pack.dh + tok_head;
+            __nv_bfloat16* orow = p.out + ((size_t)(it.seq_start + q_pos + tok) * p.H + head) * kD;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 if (dead) break;
                 uint32_t ov[32];
                 tmem_ld32(t_o + c * 32, ov);
                 tmem_wait_ld();
-                if (q_pos < it.len && p.wide) {  // whole sectors: half the store instructions
+                if (tok < live && p.wide) {  // whole sectors: half the store instructions
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         uint32_t w[8];
@@ -1032,7 +1112,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                             w[e] = pack_bf16(__uint_as_float(ov[16 * i + 2 * e]) * inv, __uint_as_float(ov[16 * i + 2 * e + 1]) * inv);
                         store_32bytes(orow + c * 32 + i * 16, w);
                     }
-                } else if (q_pos < it.len) {
+                } else if (tok < live) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         uint4 w;
@@ -1071,9 +1151,10 @@ __global__ void __launch_bounds__(kCombineThreads) prefill_combine_kernel(const 
     const List list = list_of(p);
     if (e >= items_of(static_cast<const Params&>(p), list) || splits_of(p, list.pairs) == 1) return;
     const Item it = load_item(static_cast<const Params&>(p), list, e);
-    const int runs = runs_of(p.splits, it.n_a);
-    const int q_pos = it.q0 + x * it.dq + row;
-    if ((x == 0 ? it.n_a : it.n_b) == 0 || runs == 1 || q_pos >= it.len) return;
+    const int runs = runs_of(p, p.splits, it.n_a);
+    const int tok = row / p.pack.heads, q_pos = it.q0 + x * p.pack.dq + tok;
+    if ((x == 0 ? it.n_a : it.n_b) == 0 || runs == 1 || tok >= p.pack.tokens || q_pos >= it.len) return;
+    const int head = it.head + x * p.pack.dh + row - tok * p.pack.heads;
     const float* part = p.partials + ((size_t)e * p.splits * 2 + x) * kPartialFloats;
     constexpr size_t kNext = 2 * kPartialFloats;
     float m = -INFINITY;
@@ -1095,19 +1176,19 @@ __global__ void __launch_bounds__(kCombineThreads) prefill_combine_kernel(const 
     w.y = pack_bf16(acc[2] * inv, acc[3] * inv);
     w.z = pack_bf16(acc[4] * inv, acc[5] * inv);
     w.w = pack_bf16(acc[6] * inv, acc[7] * inv);
-    *reinterpret_cast<uint4*>(p.out + ((size_t)(it.seq_start + q_pos) * p.H + it.head + x * it.dh) * kD + c8) = w;
+    *reinterpret_cast<uint4*>(p.out + ((size_t)(it.seq_start + q_pos) * p.H + head) * kD + c8) = w;
 }
 
 // ------------------------------------------------------------------------------------------
 // host
 // ------------------------------------------------------------------------------------------
-static int make_map(CUtensorMap* map, const void* base, int heads, int64_t tokens) {
+static int make_map(CUtensorMap* map, const void* base, int heads, int64_t tokens, int box_heads = 1, int box_tokens = kTileKV) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return fail(NVLLM_B200_EDRIVER, "cuTensorMapEncodeTiled entry point not available");
     // a panel of 64 dims per load: both panels in one load (the half as a fourth dimension) were 1 % slower
     cuuint64_t dims[3] = {(cuuint64_t)kD, (cuuint64_t)heads, (cuuint64_t)tokens};
     cuuint64_t strides[2] = {(cuuint64_t)kD * 2, (cuuint64_t)heads * kD * 2};
-    cuuint32_t box[3] = {64, 1, 128};
+    cuuint32_t box[3] = {64, (cuuint32_t)box_heads, (cuuint32_t)box_tokens};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1141,14 +1222,14 @@ static int check_pages(const char* who, int NB, int block_size) {
     return NVLLM_B200_OK;
 }
 
-static int64_t item_capacity(int64_t T, int B) { return T / kTileQ + B + 1; }
-static size_t list_bytes(int64_t T, int B) { return ((size_t)(2 * item_capacity(T, B) + 1) * 16 + 255) & ~size_t(255); }
+static int64_t item_capacity(int64_t T, int B, int span) { return T / span + B + 1; }
+static size_t list_bytes(int64_t T, int B, int span) { return ((size_t)(2 * item_capacity(T, B, span) + 1) * 16 + 255) & ~size_t(255); }
 
 // Runs per item: as many as leave one run per SM; 1 where no item can have enough tiles.
 constexpr int kMaxSplits = 16;
-static int splits_for(int64_t items, int64_t max_tiles, int sms) {
+static int splits_for(int64_t items, int64_t max_tiles, int sms, int span) {
     if (items <= 0 || 2 * items > sms || max_tiles < kSplitTiles) return 1;
-    return (int)std::min<int64_t>(std::min<int64_t>(sms / items, kMaxSplits), max_tiles / kMinRun);
+    return (int)std::min<int64_t>(std::min<int64_t>(sms / items, kMaxSplits), max_tiles / min_run(span));
 }
 static size_t partials_bytes(int sms) { return (size_t)sms * 2 * kPartialFloats * 4; }
 
@@ -1177,14 +1258,17 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     if (!q || !k || !v || !cu_seqlens_q || !cu_seqlens_k || !out) return fail(NVLLM_B200_EINVAL, "%s: null pointer", who);
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15)
         return fail(NVLLM_B200_EINVAL, "%s: q/k/v/out must be 16-byte aligned", who);
-    const size_t need = list_bytes(T, B);  // the rest of what is asked for lets items be split
+    const int G = H / KVH;
+    const Pack pack = make_pack(G);
+    const int span = pack.span;
+    const size_t need = list_bytes(T, B, span);  // the rest of what is asked for lets items be split
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15))
         return fail(NVLLM_B200_EWORKSPACE, "%s: workspace of %zu bytes required, got %zu", who, need,
                     workspace ? workspace_bytes : (size_t)0);
 
     ShortParams p;
-    // Upper bound of (sequence, row block) pairs: exact from the host copy of cu_seqlens, else from max_seqlen.
-    const int64_t cap = item_capacity(T, B);
+    // Upper bound of (sequence, token block) pairs: exact from the host copy of cu_seqlens, else from max_seqlen.
+    const int64_t cap = item_capacity(T, B, span);
     int64_t pairs = 0, longest = max_seqlen;
     if (cu_seqlens_host) {
         longest = 0;
@@ -1192,32 +1276,30 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
             const int64_t len = (int64_t)cu_seqlens_host[b + 1] - cu_seqlens_host[b];
             if (len < 0 || cu_seqlens_host[b + 1] > T)
                 return fail(NVLLM_B200_EINVAL, "%s: cu_seqlens_host is not a non-decreasing prefix of T", who);
-            if (len > (int64_t)kMaxLevels * kTileQ)
+            if (len > (int64_t)kMaxLevels * kTileKV)
                 return fail(NVLLM_B200_EUNSUPPORTED, "%s: sequence of %lld tokens (max %d)", who, (long long)len,
-                            kMaxLevels * kTileQ);
-            pairs += (len + kTileQ - 1) / kTileQ;
+                            kMaxLevels * kTileKV);
+            pairs += (len + span - 1) / span;
             longest = std::max(longest, len);
         }
     } else {
         if (max_seqlen <= 0) return fail(NVLLM_B200_EINVAL, "%s: max_seqlen must be positive", who);
-        if (max_seqlen > kMaxLevels * kTileQ)
-            return fail(NVLLM_B200_EUNSUPPORTED, "%s: max_seqlen %d (max %d)", who, max_seqlen, kMaxLevels * kTileQ);
-        pairs = (int64_t)B * ((max_seqlen + kTileQ - 1) / kTileQ);
+        if (max_seqlen > kMaxLevels * kTileKV)
+            return fail(NVLLM_B200_EUNSUPPORTED, "%s: max_seqlen %d (max %d)", who, max_seqlen, kMaxLevels * kTileKV);
+        pairs = (int64_t)B * ((max_seqlen + span - 1) / span);
         // The attention layer's contexts round the longest length up to 8192 at most: prompts beyond it show in T.
         if ((int64_t)B * max_seqlen < T) pairs = cap;
     }
     if (pairs > cap) pairs = cap;
     if (pairs == 0) return scatter_only();
-    const int G = H / KVH;
-    // Two q heads of one kv head make an item: both Q tiles then see the same number of K/V tiles and finish together.  Where
-    // the group size is odd its last head goes alone, 256 rows at a time.
-    p.per_pair = KVH * ((G + 1) / 2);
+    p.pack = pack;
+    p.per_pair = KVH * pack.per_kv;
     if (pairs * p.per_pair > 0x7fffffffLL) return fail(NVLLM_B200_EUNSUPPORTED, "%s: grid too large", who);
 
     int rc = ensure_attr();
     if (rc) return rc;
     CUtensorMap tm_q, tm_k, tm_v;
-    if ((rc = make_map(&tm_q, q, H, T))) return rc;
+    if ((rc = make_map(&tm_q, q, H, T, pack.heads, pack.tokens))) return rc;
     if ((rc = make_map(&tm_k, k, KVH, kv_tokens))) return rc;
     if ((rc = make_map(&tm_v, v, KVH, kv_tokens))) return rc;
 
@@ -1240,9 +1322,9 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     // the scatter, where SMs are left, goes with the launch.  Elsewhere the scatter is a launch of its own: on a warp of the
     // attention CTAs it slowed them by as much as it took (power and issue slots).
     const int64_t max_tiles = block_tables ? (int64_t)MB * block_size / kTileKV : (longest + kTileKV - 1) / kTileKV;
-    const size_t lists = list_bytes(T, B);
+    const size_t lists = need;
     const int splits = workspace_bytes >= lists + partials_bytes(sms) && ((uintptr_t)workspace & 255) == 0
-                           ? splits_for(pairs * p.per_pair, max_tiles, sms)
+                           ? splits_for(pairs * p.per_pair, max_tiles, sms, span)
                            : 1;
     const bool brief = splits == 1 && cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q &&
                        B <= kShortSequences && pairs <= kShortBlocks && pairs * p.per_pair <= sms;
@@ -1268,7 +1350,7 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
         cfg.gridDim = dim3(1);
         cfg.blockDim = dim3(kPlanThreads);
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, prefill_plan_kernel, cu_seqlens_q, cu_seqlens_k, block_tables ? 1 : 0, B,
-                                         (int4*)workspace, (int)cap, p.per_pair, KVH, ctas,
+                                         (int4*)workspace, (int)cap, span, p.per_pair, KVH, ctas,
                                          scatter && pdl_enabled() ? 1 : 0));
     }
     cfg.gridDim = dim3((unsigned)ctas);
@@ -1311,12 +1393,12 @@ extern "C" size_t nvllm_b200_varlen_prefill_workspace_bytes(int64_t T, int B, in
     using namespace nvllm::prefill;
     (void)D;
     if (T < 0 || B < 0) return 256;
-    size_t n = list_bytes(T, B);
-    if (H > 0 && KVH > 0 && H % KVH == 0) {
-        // room for the partial results of split items where so few items are possible
-        const int64_t blocks = std::max<int64_t>((T + kTileQ - 1) / kTileQ, B), per_pair = (int64_t)KVH * ((H / KVH + 1) / 2);
-        if (2 * blocks * per_pair <= sm_count()) n += partials_bytes(sm_count());
-    }
+    if (H <= 0 || KVH <= 0 || H % KVH != 0) return list_bytes(T, B, 1);
+    const Pack pack = make_pack(H / KVH);
+    size_t n = list_bytes(T, B, pack.span);
+    // room for the partial results of split items where so few items are possible
+    const int64_t blocks = std::max<int64_t>((T + pack.span - 1) / pack.span, B), per_pair = (int64_t)KVH * pack.per_kv;
+    if (2 * blocks * per_pair <= sm_count()) n += partials_bytes(sm_count());
     return n;
 }
 

@@ -1,31 +1,38 @@
-"""CPU model of the tile bookkeeping of the prefill kernel (csrc/varlen_prefill.cu): which rows of which head the two Q tiles
-of a work item hold (make_item: 128 rows of two heads, or 256 rows of the last head of an odd group), which 128-key tiles they
-visit and what the element mask leaves of them, whole or cut into runs, must cover exactly the causal region -- key c is used
-for query position p iff c <= p -- of every head once; and the item lists (the plan kernel's, and the one a short launch's CTAs
-find themselves) must contain every (sequence, row block) once, longest causal span first."""
+"""CPU model of the tile bookkeeping of the prefill kernel (csrc/varlen_prefill.cu): which tokens of which heads the two Q tiles
+of a work item hold (make_pack, make_item: (token, head) rows of one kv head), which 128-key tiles they visit, how many keys of
+the last one the products go through and what the element mask leaves of them, whole or cut into runs, must cover exactly the
+causal region -- key c is used for query position p iff c <= p -- of every head once; and the item lists (the plan kernel's, and
+the one a short launch's CTAs find themselves) must contain every (sequence, token block) once, longest causal span first."""
 import numpy as np
 import pytest
 
-TILE, MIN_RUN, SPLIT_TILES = 128, 4, 12
+TILE, SPLIT_TILES = 128, 8
 
 
-def make_item(length, prefix, q0, group, r):
-    """Item r of the row block at q0, for one kv head: [(head, first row, K/V tiles)] of Q tiles A and B, or None."""
-    h2 = 2 * r
-    two = h2 + 1 < group
-    dq, dh = (0, 1) if two else (TILE, 0)
-    nk_total = -(-(prefix + length) // TILE)
-    n_a = min(nk_total, (prefix + q0 + TILE - 1) // TILE + 1)
-    n_b = n_a if two else (min(nk_total, (prefix + q0 + 2 * TILE - 1) // TILE + 1) if length - q0 > TILE else 0)
-    if not two and (q0 // TILE) & 1:
-        return None
-    return [(h2, q0, n_a), (h2 + dh, q0 + dq, n_b)]
+def make_pack(group):
+    w = max(x for x in range(1, 9) if group % x == 0)
+    heads = w if w % 2 else w // 2
+    tokens = TILE // heads
+    return dict(w=w, heads=heads, tokens=tokens, dq=tokens if w % 2 else 0, dh=0 if w % 2 else heads,
+                span=2 * tokens if w % 2 else tokens, per_kv=group // w)
 
 
-def runs(tiles, splits):
+def visible_keys(pack, length, prefix, q0, x):
+    return prefix + min(length, q0 + x * pack["dq"] + pack["tokens"])
+
+
+def make_item(pack, length, prefix, q0, r):
+    """Item r of the token block at q0, for one kv head: [(first head, first token, K/V tiles)] of Q tiles A and B."""
+    n_a = (visible_keys(pack, length, prefix, q0, 0) - 1) // TILE + 1
+    n_b = (visible_keys(pack, length, prefix, q0, 1) - 1) // TILE + 1 if length - q0 > pack["dq"] else 0
+    head = r * pack["w"]
+    return [(head, q0, n_a), (head + pack["dh"], q0 + pack["dq"], n_b)]
+
+
+def runs(pack, tiles, splits):
     """Runs of an item (load_item of SplitParams): per run its first K/V tile and the tiles Q tiles A and B visit there."""
     n_a, n_b = tiles
-    n_kv, count = max(n_a, n_b), 1 if n_a < SPLIT_TILES else min(splits, n_a // MIN_RUN)
+    n_kv, count = max(n_a, n_b), 1 if n_a < SPLIT_TILES else min(splits, n_a // (3 if pack["span"] > TILE else 2))
     out = []
     for c in range(count):
         j0, j1 = n_a * c // count, n_kv if c + 1 == count else n_a * (c + 1) // count
@@ -33,54 +40,69 @@ def runs(tiles, splits):
     return out
 
 
-def seen_keys(prefix, first_row, row, j0, n):
-    """Keys that row `row` of the Q tile at first_row uses in the n tiles from tile j0 on: unmasked tiles whole, of the others
-    the keys up to the row's limit (relative to the run's first tile, as the kernel counts)."""
-    first_lim = prefix - j0 * TILE + first_row
-    n_plain = max(0, min(n, (first_lim + 1) // TILE))
-    keys = [np.arange(n_plain * TILE)]
-    for j in range(n_plain, n):
-        lim = first_lim - j * TILE + row
-        keys.append(j * TILE + np.arange(TILE)[np.arange(TILE) <= lim])
-    return j0 * TILE + np.concatenate(keys)
+def seen_keys(pack, length, prefix, q0, x, row, j0, n):
+    """Keys that row `row` of Q tile x uses in the n tiles from tile j0 on: unmasked tiles whole, of the others the keys up to the
+    row's limit, by chunks of 32 that the warp's rows need (counted from the run's first tile, as the kernel does).  All of them
+    must be keys that the products have gone through."""
+    prefix -= j0 * TILE
+    first = q0 + x * pack["dq"]
+    live = min(pack["tokens"], length - first)
+    tok = lambda r: min(r // pack["heads"], live - 1)
+    warp = row // 32 * 32
+    keys = []
+    for j in range(n):
+        lim, lo, hi = (prefix + first - j * TILE + tok(r) for r in (row, warp, warp + 31))
+        through = 16 * (-(-min(TILE, visible_keys(pack, length, prefix, q0, x) - (n - 1) * TILE) // 16)) if j == n - 1 else TILE
+        if j < (prefix + first + 1) // TILE:
+            seen = np.arange(TILE)  # a plain tile
+        else:
+            seen = [np.arange(32 * c, 32 * c + 32) for c in range(4) if 32 * c <= hi]
+            seen = np.concatenate([c[c <= lim] if c[-1] > lo else c for c in seen] or [np.arange(0)])
+        assert len(seen) == 0 or seen[-1] < through, "a score that was not computed"
+        keys.append(j0 * TILE + j * TILE + seen)
+    return np.concatenate(keys)
 
 
-@pytest.mark.parametrize("group", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("group", [1, 2, 3, 4, 5, 6, 7, 8, 10, 11, 16])
 @pytest.mark.parametrize("prefix", [0, 1, 127, 128, 1500, 2048])
 @pytest.mark.parametrize("length", [1, 5, 127, 128, 129, 255, 256, 257, 300, 512, 513])
 def test_tiles_and_masks_cover_exactly_the_causal_region(length, prefix, group):
+    pack = make_pack(group)
+    assert pack["heads"] * pack["tokens"] <= TILE
     for splits in (1, 3, 16):
         covered = {}
-        for q0 in range(0, length, TILE):
-            for r in range((group + 1) // 2):
-                item = make_item(length, prefix, q0, group, r)
-                if item is None:
+        for q0 in range(0, length, pack["span"]):
+            item = make_item(pack, length, prefix, q0, 0)
+            parts = runs(pack, (item[0][2], item[1][2]), splits)
+            for x, (head, first, n_x) in enumerate(item):
+                if n_x == 0:
+                    assert first >= length
                     continue
-                parts = runs((item[0][2], item[1][2]), splits)
-                for x, (head, first_row, n_x) in enumerate(item):
-                    if n_x == 0:
-                        assert first_row >= length
-                        continue
-                    for row in {0, 1, 31, 32, 100, 127, min(TILE, length - first_row) - 1}:
-                        p = first_row + row
-                        if not 0 <= p < length or row < 0:
-                            continue  # rows past the sequence are computed on whatever the tile holds and never stored
-                        keys = [seen_keys(prefix, first_row, row, j0, (n_a, n_b)[x]) for j0, n_a, n_b in parts]
-                        assert all(len(k) for k in keys), "a run none of whose keys a row sees has no maximum"
-                        assert np.array_equal(np.concatenate(keys), np.arange(prefix + p + 1)), (length, prefix, q0, x, row)
-                    for t in range(first_row, min(first_row + TILE, length)):
-                        covered[head, t] = covered.get((head, t), 0) + 1
+                rows = min(pack["tokens"], length - first) * pack["heads"]
+                for row in {r for r in (0, 1, 31, 32, 100, 127, rows - 1) if r < rows}:
+                    p = first + row // pack["heads"]
+                    keys = [seen_keys(pack, length, prefix, q0, x, row, j0, (n_a, n_b)[x]) for j0, n_a, n_b in parts]
+                    assert all(len(k) for k in keys), "a run none of whose keys a row sees has no maximum"
+                    assert np.array_equal(np.concatenate(keys), np.arange(prefix + p + 1)), (length, prefix, q0, x, row)
+                for r in range(pack["per_kv"]):
+                    h0 = make_item(pack, length, prefix, q0, r)[x][0]
+                    for t in range(first, min(first + pack["tokens"], length)):
+                        for h in range(h0, h0 + pack["heads"]):
+                            covered[h, t] = covered.get((h, t), 0) + 1
         assert covered == {(h, t): 1 for h in range(group) for t in range(length)}, "every row of every head once"
 
 
-def blocks_of(lens):
-    return [(b, level) for b, n in enumerate(lens) for level in range(-(-n // TILE))]
+def blocks_of(lens, span=TILE):
+    return [(b, level) for b, n in enumerate(lens) for level in range(-(-n // span))]
 
 
 def test_plan_orders_items_longest_span_first():
     lens, prefixes = [700, 256, 1, 1300, 0, 257], [0, 3000, 128, 0, 500, 127]
     # the plan kernel: histogram per level, bases assigned from the highest level down, any order inside a level
-    levels = {(b, l): prefixes[b] // TILE + l for b, l in blocks_of(lens)}
+    levels = {(b, l): (prefixes[b] + min(lens[b], (l + 1) * TILE) - 1) // TILE for b, l in blocks_of(lens)}
+    for b, l in levels:  # as many K/V tiles in front of its last one as the item of the block has
+        n_kv = max(n for _, _, n in make_item(make_pack(2), lens[b], prefixes[b], l * TILE, 0))
+        assert levels[b, l] == n_kv - 1
     top = max(levels.values()) + 1
     order = [k for level in range(top - 1, -1, -1) for k, v in levels.items() if v == level]
     assert sorted(order) == sorted(blocks_of(lens)) and len(order) == len(set(order)) == 6 + 2 + 1 + 11 + 0 + 3
