@@ -2,6 +2,8 @@
 // step that folds it into its first kernel lives in paged_decode.cu.
 #include "pre_attention.cuh"
 
+#include <mutex>
+
 namespace nvllm {
 namespace preattn {
 
@@ -14,26 +16,44 @@ __global__ void __launch_bounds__(kThreads) pre_attention_small_kernel(const Par
 
 // Many tokens: a warp works on eight rows of one token at a time (a pass), four lanes per row: first the q rows, then the
 // k and v rows.  A work unit is `span` consecutive passes of a token; the units are dealt round-robin to a persistent grid.
-// The token's cosines and sines are loaded once per unit and stay in registers over its passes, only the eight weight loads
-// of a pass come from shared memory, and the rows of the next pass are requested before the current one is computed.
-// Bound by instruction latency at 16 warps per SM (16 384 tokens, 32 / 8 heads: 87.2 us with a row per four lanes and the
-// rotation loaded for every row, 79.5 us here = 5.6 TB/s; rows staged through shared memory with bulk copies, 142 us).
+// The token's cosines and sines stay in registers over its passes, only the eight weight loads of a pass come from shared
+// memory.  The rows of the next pass, and with a new unit its rotation, are copied (cp.async) into the warp's part of shared
+// memory while the current one is computed: requested into registers, the rows cost sixteen of them, and a unit began with
+// the latencies of its position and of its rotation.
+// Bound by HBM: 16 384 tokens, 32 / 8 heads, 436 MB: 87.2 us with a row per four lanes and the rotation loaded for every row,
+// 81.1 with the next rows in registers, 73.9 here = 5.9 TB/s; 8192 tokens, 64 / 8: 68.2 -> 60.6; 30 000, 28 / 4: 120.7 -> 104.9.
+// One pass ahead is enough and more is slower: two ahead 81.5 us, three 82.4 (reads and writes of the DRAM in each other's
+// way); 12 warps per SM 84.5, 24 (spills) 99.7; bulk copies through shared memory 142.
 constexpr int kPassThreads = 256;
+constexpr int kPassStages = 2;  // the pass that is computed and the next one
+struct PassSmem {  // of a warp
+    uint4 rows[kPassStages][4][32];   // chunk i of each lane's row; every lane copies and reads its own
+    float rotation[kPassStages][kD];  // of the units in flight (a unit has at least one pass)
+};
+constexpr int kPassSmemBytes = kPassThreads / 32 * (int)sizeof(PassSmem);
+
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 __global__ void __launch_bounds__(kPassThreads, 2) pre_attention_pass_kernel(const Params p, const int passes, const int span) {
+    extern __shared__ __align__(16) uint8_t pass_smem[];
     __shared__ __align__(16) float weights[2][kD];
     griddep_wait();  // q, k, v may come from the kernel just before this one (the QKV projection)
     griddep_launch_dependents();
-    weights[threadIdx.x >> 7][threadIdx.x & 127] = (threadIdx.x < kD ? p.q_weight : p.k_weight - kD)[threadIdx.x];
+    for (int i = threadIdx.x; i < 2 * kD; i += kPassThreads) weights[i >> 7][i & 127] = (i < kD ? p.q_weight : p.k_weight - kD)[i];
     __syncthreads();
+    PassSmem& sm = reinterpret_cast<PassSmem*>(pass_smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, q = lane & 3, sub = lane >> 2;
     const int q_passes = (p.H + 7) >> 3;
     const int parts = (passes + span - 1) / span;  // units per token
-    const int64_t units = p.T * parts, stride = (int64_t)gridDim.x * (kPassThreads / 32);
-
-    int64_t unit = (int64_t)blockIdx.x * (kPassThreads / 32) + (threadIdx.x >> 5);
-    if (unit >= units) return;
-    int64_t t = unit / parts;
-    int pass = (int)(unit - t * parts) * span, end = min(pass + span, passes);
+    // a warp's units: the first, and the step to the next one in tokens and parts
+    const int warps = gridDim.x * (kPassThreads / 32), step_t = warps / parts, step_part = warps - step_t * parts;
 
     auto source = [&](int64_t tok, int ps) -> const __nv_bfloat16* {  // this lane's row in a pass (null: none)
         if (ps < q_passes) {
@@ -43,47 +63,87 @@ __global__ void __launch_bounds__(kPassThreads, 2) pre_attention_pass_kernel(con
         const int r = (ps - q_passes) * 8 + sub;
         return r < p.KVH ? p.k + (tok * p.KVH + r) * kD : (r < 2 * p.KVH ? p.v + (tok * p.KVH + r - p.KVH) * kD : nullptr);
     };
-    auto load = [&](const __nv_bfloat16* src, uint4 (&w)[4]) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            w[i] = src ? *reinterpret_cast<const uint4*>(src + (q + 4 * i) * 8) : make_uint4(0, 0, 0, 0);
-    };
-
     auto store = [&](__nv_bfloat16* dst, const uint4 (&w)[4]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(dst + (q + 4 * i) * 8) = w[i];
     };
+    struct Cursor {  // a pass of a unit
+        int64_t t;
+        int part, pass, end;
+    };
+    auto enter = [&](Cursor& c) {  // the first pass of its unit
+        c.pass = c.part * span;
+        c.end = min(c.pass + span, passes);
+    };
+    auto step = [&](Cursor& c) {  // to the next unit
+        c.t += step_t;
+        c.part += step_part;
+        if (c.part >= parts) c.part -= parts, ++c.t;
+        enter(c);
+    };
 
-    const __nv_bfloat16* src = source(t, pass);
-    uint4 w[4];
-    load(src, w);
+    Cursor at, ahead;
+    {
+        const int unit = blockIdx.x * (kPassThreads / 32) + (threadIdx.x >> 5);
+        at.t = unit / parts;
+        at.part = unit - (int)at.t * parts;
+    }
+    if (at.t >= p.T) return;
+    enter(at);
+    ahead = at;
+    uint32_t filled = 0, entered = 0;  // passes and units copied so far
+    int pos = __ldg(p.positions + ahead.t);
+    bool fresh_ahead = true;  // ahead's rotation is not on its way yet
+    auto fetch = [&]() {  // copies the pass at `ahead` and moves on; one group per call
+        if (ahead.t < p.T) {
+            if (fresh_ahead) {
+                const int64_t row = pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
+                copy16_async(sm.rotation[entered] + lane * 4, p.cos_sin + row * kD + lane * 4);
+                if (++entered == kPassStages) entered = 0;
+                Cursor next = ahead;
+                step(next);
+                if (next.t < p.T) pos = __ldg(p.positions + next.t);
+            }
+            const __nv_bfloat16* src = source(ahead.t, ahead.pass);
+            if (src) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) copy16_async(&sm.rows[filled][i][lane], src + (q + 4 * i) * 8);
+            }
+            if (++filled == kPassStages) filled = 0;
+            fresh_ahead = ++ahead.pass == ahead.end;
+            if (fresh_ahead) step(ahead);
+        }
+        copy_commit();
+    };
+#pragma unroll 1
+    for (int i = 0; i + 1 < kPassStages; ++i) fetch();
+
     uint64_t c[2][4], s[2][4];
     int64_t slot = -1;
-    bool fresh = true;  // t's metadata and rotation are not loaded yet
+    bool fresh = true;  // at's slot and rotation are not loaded yet
+    uint32_t done = 0, unit_no = 0;
+#pragma unroll 1
     while (true) {
+        copy_wait<kPassStages - 2>();
+        __syncwarp();  // the other lanes' parts of the rotation; and all have read the buffers that fetch() fills next
         if (fresh) {
-            const int pos = __ldg(p.positions + t);
-            slot = __ldg(p.slot_mapping + t);
-            load_rotation(p, pos, q, c, s);
-            fresh = false;
-        }
-        int64_t next_t = t;
-        int next_pass = pass + 1;
-        bool more = true;
-        const bool new_unit = next_pass == end;
-        if (new_unit) {
-            unit += stride;
-            more = unit < units;
-            if (more) {
-                next_t = unit / parts;
-                next_pass = (int)(unit - next_t * parts) * span;
+            slot = __ldg(p.slot_mapping + at.t);
+            const float* cs = sm.rotation[unit_no] + q * 8;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                load_pairs(cs + 32 * i, c[i]);
+                load_pairs(cs + 32 * i + 64, s[i]);
             }
+            if (++unit_no == kPassStages) unit_no = 0;
         }
-        const __nv_bfloat16* next_src = more ? source(next_t, next_pass) : nullptr;
-        uint4 next_w[4];
-        load(next_src, next_w);
+        uint4 w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = sm.rows[done][i][lane];
+        if (++done == kPassStages) done = 0;
+        fetch();
 
-        const int r = (pass - q_passes) * 8 + sub;  // row among the k and v rows (negative: a q row)
+        const __nv_bfloat16* src = source(at.t, at.pass);
+        const int r = (at.pass - q_passes) * 8 + sub;  // row among the k and v rows (negative: a q row)
         const bool is_v = r >= p.KVH;
         const bool cached = src && r >= 0 && slot >= 0 && slot < p.num_slots;
         if (is_v && cached) store(p.v_cache + (slot * p.KVH + r - p.KVH) * kD, w);
@@ -92,15 +152,13 @@ __global__ void __launch_bounds__(kPassThreads, 2) pre_attention_pass_kernel(con
             if (src && !is_v) store(const_cast<__nv_bfloat16*>(src), w);  // q and k are updated in place
             if (!is_v && cached) store(p.k_cache + (slot * p.KVH + r) * kD, w);
         }
-        if (!more) break;
-        fresh = next_t != t;
-        if (new_unit) end = min(next_pass + span, passes);
-        t = next_t;
-        pass = next_pass;
-        src = next_src;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = next_w[i];
+        fresh = ++at.pass == at.end;
+        if (fresh) {
+            step(at);
+            if (at.t >= p.T) break;
+        }
     }
+    copy_wait<0>();
 }
 
 int check_args(const char* who, const void* q, const void* k, const void* v, const float* q_weight, const float* k_weight,
@@ -141,10 +199,16 @@ extern "C" int nvllm_b200_qk_norm_rope_store(void* q, void* k, const void* v, co
     cfg.stream = reinterpret_cast<cudaStream_t>(stream);
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    // The pass kernel pays where its passes are full and every resident warp (two CTAs per SM) gets ten of them or more.
+    // The pass kernel pays where its passes are full and every resident warp (two CTAs per SM) gets 4.5 of them or more, or eight
+    // with passes three quarters full.  us, small kernel / this one, 2368 warps: 32 / 8 heads (full), 4.1 passes a warp
+    // 9.0 / 9.8, 4.4 10.9 / 10.6, 5.1 12.7 / 11.5, 8.1 20.4 / 17.9; 28 / 4 (0.9), 4.6 9.4 / 8.9; 14 / 2 (0.75), 5.0
+    // 8.7 / 10.6, 7.6 16.1 / 16.4, 20.8 39.2 / 36.0; 12 / 4 (0.83), 5.1 11.1 / 11.5, 7.6 17.4 / 17.0, 11.4 24.9 / 22.4; 18 / 2
+    // (0.69), 13.5 24.8 / 25.2; 8 / 1 (0.62), 16.9 28.7 / 32.1.
     const int passes = (H + 7) / 8 + (2 * KVH + 7) / 8;
     const int64_t ctas = 2 * (int64_t)sm_count(), warps = ctas * (preattn::kPassThreads / 32);
-    if (T * passes < 10 * warps || 10 * (H + 2 * KVH) < 9 * 8 * passes) {
+    const int rows = H + 2 * KVH, room = 8 * passes;
+    const bool many = 10 * rows >= 9 * room ? 2 * T * passes >= 9 * warps : 4 * rows >= 3 * room && T * passes >= 8 * warps;
+    if (!many) {
         cfg.gridDim = dim3((unsigned)preattn::blocks_for(T, H, KVH));
         cfg.blockDim = dim3(preattn::kThreads);
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, preattn::pre_attention_small_kernel, p));
@@ -160,6 +224,19 @@ extern "C" int nvllm_b200_qk_norm_rope_store(void* q, void* k, const void* v, co
     }
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(preattn::kPassThreads);
+    cfg.dynamicSmemBytes = preattn::kPassSmemBytes;
+    {
+        static std::mutex mu;
+        static bool done[64];
+        int dev = 0;
+        NVLLM_CUDA_OK(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev < 0 || dev >= 64 || !done[dev]) {
+            NVLLM_CUDA_OK(cudaFuncSetAttribute(preattn::pre_attention_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               preattn::kPassSmemBytes));
+            if (dev >= 0 && dev < 64) done[dev] = true;
+        }
+    }
     NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, preattn::pre_attention_pass_kernel, p, passes, span));
     return NVLLM_B200_OK;
 }
