@@ -1038,7 +1038,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        if (both && (x == 0 || j + 1 < it.n_a)) mbar_arrive(&sh->turn[x]);
+                        if (both && (x == 0 || j < it.n_a)) mbar_arrive(&sh->turn[x]);
                         mbar_arrive(&sh->p_full[x][0]);
                         mbar_arrive(&sh->p_full[x][1]);
                     }
@@ -1049,9 +1049,9 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 if (!softmax_tile<kDiag>(sh, x, t_s, t_o, kDiag ? lim + min(tok, live - 1) : 0, kDiag ? lim + min(tok_lo, live - 1) : 0,
                                          kDiag ? lim + min(tok_hi, live - 1) : 0, j == 0,
                                          (tiles - 1) & 1u, p.scale_log2, m_run, m_used, l, turn_bar, turn_parity,
-                                         (both && (x == 0 || j + 1 < it.n_a)) ? &sh->turn[x] : nullptr))
+                                         (both && (x == 0 || j < it.n_a)) ? &sh->turn[x] : nullptr))
                     return false;
-                // hand the turn over: A after each of its tiles, B while A still has a tile that will wait for it
+                // the turn is handed over by A after each of its tiles, by B after those that followed one of A's
                 ++tiles;
                 return true;
             };
@@ -1091,6 +1091,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                         mbar_arrive(&sh->o_empty[x]);
                         mbar_arrive(&sh->item_empty[k % kItemRing]);
                     }
+                    if (x == 0 && both) ok = wait_or_abort(sh, &sh->turn[1], turns_seen++ & 1u);
                     continue;
                 }
             }
@@ -1130,6 +1131,9 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 mbar_arrive(&sh->o_empty[x]);
                 mbar_arrive(&sh->item_empty[k % kItemRing]);  // only now: the next claim waits for it
             }
+            // B's last turn.  Else A, two hand-overs further with the next item's first tile, could lap a warp of B that was
+            // held up in front of its last wait (2.7 us would do), and the parity would alias.
+            if (x == 0 && both) ok = wait_or_abort(sh, &sh->turn[1], turns_seen++ & 1u);
         }
     }
 

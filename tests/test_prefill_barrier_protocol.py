@@ -116,7 +116,7 @@ class Sim:
             raise ProtocolError(f"deadlock: {sorted(self.threads)} never finished")
 
 
-def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True, o_first=True):
+def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True, o_first=True, last_turn=True, slow=0):
     sim = Sim(seed, jitter)
     item_full = [Bar(f"item_full{s}", 1) for s in range(ITEM_RING)]
     item_empty = [Bar(f"item_empty{s}", ITEM_READERS) for s in range(ITEM_RING)]
@@ -239,7 +239,7 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True, o_fir
                 if both and (j >= 1 if x == 0 else j < n_a):  # A(j) after B(j-1); B(j) after A(j) while A has tiles
                     turn = ("wait", turns[x ^ 1], turns_seen)
                     turns_seen += 1
-                hand = both and (x == 0 or j + 1 < n_a) and (hand_turn_back or x == 0)
+                hand = both and (x == 0 or j < (n_a if last_turn else n_a - 1)) and (hand_turn_back or x == 0)
                 if it.ragged and j == n_kv - 1:  # zero the rows past the sequence's end in V(last) before P is handed over
                     vpos = 2 * (kt0 + n_kv - 1) + 1
                     yield ("wait", kv_full[vpos % SLOTS], vpos // SLOTS)
@@ -255,7 +255,7 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True, o_fir
                     yield ("arrive", p_full[x][1])
                     tiles += 1
                     continue
-                yield ("delay", 300)  # scores to registers, row max: not exclusive
+                yield ("delay", 300 + (slow if (x, warp) == (1, 3) else 0))  # scores to registers, row max: not exclusive
                 if turn:
                     yield turn
                 yield ("delay", 800)
@@ -270,6 +270,9 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True, o_fir
                 yield ("delay", 900)
             yield ("arrive", o_empty[x])
             yield ("arrive", item_empty[(k - 1) % ITEM_RING])
+            if x == 0 and both and last_turn:
+                yield ("wait", turns[1], turns_seen)
+                turns_seen += 1
 
     sim.spawn("records", records())
     sim.spawn("producer", producer())
@@ -351,3 +354,8 @@ def test_model_catches_broken_protocols():
     with pytest.raises(ProtocolError, match="o_full"):  # dead warps see S(j) before the commit of P.V(j-1) has arrived
         for seed in range(40):
             run_cta([item_tiles(512, 20, prefix=108, pair_heads=True, turns=False)] * 3, seed=seed, jitter=0.95, o_first=False)
+    # tile A, done with its next item's first tile, laps a warp of B that is held up in front of its last turn
+    heads = [item_tiles(128, 128, pair_heads=True)] * 6
+    run_cta(heads, slow=20000)
+    with pytest.raises(ProtocolError, match="turn"):
+        run_cta(heads, slow=20000, last_turn=False)
