@@ -14,14 +14,14 @@ __global__ void __launch_bounds__(kThreads) pre_attention_small_kernel(const Par
     pre_attention_block(blockIdx.x, p);
 }
 
-// Many tokens: a warp works on eight rows of one token at a time (a pass), four lanes per row: first the q rows, then the
-// k and v rows.  A work unit is `span` consecutive passes of a token; the units are dealt round-robin to a persistent grid.
+// Many tokens: a warp works on eight rows of one token at a time (a pass), four lanes per row: the q rows, the k rows, the v
+// rows.  A work unit is `span` consecutive passes of a token; the units are dealt round-robin to a persistent grid.
 // The token's cosines and sines stay in registers over its passes, only the eight weight loads of a pass come from shared
 // memory.  The rows of the next pass, and with a new unit its rotation, are copied (cp.async) into the warp's part of shared
 // memory while the current one is computed: requested into registers, the rows cost sixteen of them, and a unit began with
 // the latencies of its position and of its rotation.
 // Bound by HBM: 16 384 tokens, 32 / 8 heads, 436 MB: 87.2 us with a row per four lanes and the rotation loaded for every row,
-// 81.1 with the next rows in registers, 73.9 here = 5.9 TB/s; 8192 tokens, 64 / 8: 68.2 -> 60.6; 30 000, 28 / 4: 120.7 -> 104.9.
+// 81.1 with the next rows in registers, 72.8 here = 6.0 TB/s; 8192 tokens, 64 / 8: 68.2 -> 60.6; 30 000, 28 / 4: 120.7 -> 103.2.
 // One pass ahead is enough and more is slower: two ahead 81.5 us, three 82.4 (reads and writes of the DRAM in each other's
 // way); 12 warps per SM 84.5, 24 (spills) 99.7; bulk copies through shared memory 142.
 constexpr int kPassThreads = 256;
@@ -50,17 +50,13 @@ __global__ void __launch_bounds__(kPassThreads, 2) pre_attention_pass_kernel(con
     __syncthreads();
     PassSmem& sm = reinterpret_cast<PassSmem*>(pass_smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, q = lane & 3, sub = lane >> 2;
-    const int q_passes = (p.H + 7) >> 3;
     const int parts = (passes + span - 1) / span;  // units per token
     // a warp's units: the first, and the step to the next one in tokens and parts
     const int warps = gridDim.x * (kPassThreads / 32), step_t = warps / parts, step_part = warps - step_t * parts;
 
     auto source = [&](int64_t tok, int ps) -> const __nv_bfloat16* {  // this lane's row in a pass (null: none)
-        if (ps < q_passes) {
-            const int r = ps * 8 + sub;
-            return r < p.H ? p.q + (tok * p.H + r) * kD : nullptr;
-        }
-        const int r = (ps - q_passes) * 8 + sub;
+        const int r = ps * 8 + sub - p.H;
+        if (r < 0) return p.q + (tok * p.H + r + p.H) * kD;
         return r < p.KVH ? p.k + (tok * p.KVH + r) * kD : (r < 2 * p.KVH ? p.v + (tok * p.KVH + r - p.KVH) * kD : nullptr);
     };
     auto store = [&](__nv_bfloat16* dst, const uint4 (&w)[4]) {
@@ -143,7 +139,7 @@ __global__ void __launch_bounds__(kPassThreads, 2) pre_attention_pass_kernel(con
         fetch();
 
         const __nv_bfloat16* src = source(at.t, at.pass);
-        const int r = (at.pass - q_passes) * 8 + sub;  // row among the k and v rows (negative: a q row)
+        const int r = at.pass * 8 + sub - p.H;  // row among the k and v rows (negative: a q row)
         const bool is_v = r >= p.KVH;
         const bool cached = src && r >= 0 && slot >= 0 && slot < p.num_slots;
         if (is_v && cached) store(p.v_cache + (slot * p.KVH + r - p.KVH) * kD, w);
@@ -200,14 +196,16 @@ extern "C" int nvllm_b200_qk_norm_rope_store(void* q, void* k, const void* v, co
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
     // The pass kernel pays where its passes are full and every resident warp (two CTAs per SM) gets 4.5 of them or more, or eight
-    // with passes three quarters full.  us, small kernel / this one, 2368 warps: 32 / 8 heads (full), 4.1 passes a warp
-    // 9.0 / 9.8, 4.4 10.9 / 10.6, 5.1 12.7 / 11.5, 8.1 20.4 / 17.9; 28 / 4 (0.9), 4.6 9.4 / 8.9; 14 / 2 (0.75), 5.0
-    // 8.7 / 10.6, 7.6 16.1 / 16.4, 20.8 39.2 / 36.0; 12 / 4 (0.83), 5.1 11.1 / 11.5, 7.6 17.4 / 17.0, 11.4 24.9 / 22.4; 18 / 2
-    // (0.69), 13.5 24.8 / 25.2; 8 / 1 (0.62), 16.9 28.7 / 32.1.
-    const int passes = (H + 7) / 8 + (2 * KVH + 7) / 8;
+    // with passes three quarters full (but not where that is a token's only pass, which loads a rotation every time).  us,
+    // small kernel / this one, 2368 warps: 32 / 8 heads (full), 4.1 passes a warp 9.0 / 9.8, 4.4 10.9 / 10.6, 5.1 12.7 / 11.5, 8.1
+    // 20.4 / 17.9; 6 / 1, 6.9 20.5 / 18.1; 28 / 4 (0.9), 4.6 9.4 / 8.9; 18 / 2 (0.92), 6.3 15.6 / 14.4; 10 / 2 (0.88), 4.2
+    // 9.2 / 11.4, 13.8 31.6 / 28.6; 12 / 4 (0.83), 5.1 11.1 / 11.5, 7.6 17.4 / 17.0; 14 / 2 (0.75), 5.0 8.7 / 10.6, 20.8 39.4 / 35.0;
+    // one pass a token: 5 / 1 (0.88), 6.9 18.2 / 19.3, 4 / 1 (0.75), 8.4 18.8 / 22.8; 8 / 1 (0.62), 16.9 28.4 / 32.1.
+    const int passes = (H + 2 * KVH + 7) / 8;
     const int64_t ctas = 2 * (int64_t)sm_count(), warps = ctas * (preattn::kPassThreads / 32);
     const int rows = H + 2 * KVH, room = 8 * passes;
-    const bool many = 10 * rows >= 9 * room ? 2 * T * passes >= 9 * warps : 4 * rows >= 3 * room && T * passes >= 8 * warps;
+    const bool many = 10 * rows >= 9 * room ? 2 * T * passes >= 9 * warps
+                                            : passes > 1 && 4 * rows >= 3 * room && T * passes >= 8 * warps;
     if (!many) {
         cfg.gridDim = dim3((unsigned)preattn::blocks_for(T, H, KVH));
         cfg.blockDim = dim3(preattn::kThreads);

@@ -8,6 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("t,h,kvh", [(1775, 32, 8), (1776, 32, 8), (1065, 64, 8), (1066, 64, 8), (2132, 28, 4), (6314, 14, 2),
-                                     (6315, 14, 2), (6317, 12, 4), (8191, 9, 8)])
+                                     (6315, 14, 2), (6317, 12, 4), (8191, 9, 8), (8190, 18, 2), (8190, 10, 2),
+                                     (8191, 6, 1), (8191, 5, 1)])
 def test_lines_and_ragged_units(t, h, kvh):
     check(t, h, kvh)
