@@ -58,7 +58,7 @@ PREFILL_METRIC, PREFILL_UNIT = "varlen_prefill_tflops", "TFLOP/s"
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel (mean of two launches), from the ncu
 # captures summarised under profiles/ (a property of the launch, independent of the page-pool size the capture used);
 # None where no capture exists.
-NCU_TRAFFIC_BYTES = {"cfg2": 1_020_566_784, "cfg4": 2_147_142_016}
+NCU_TRAFFIC_BYTES = {"cfg2": 1_020_566_784, "cfg4": 844_928_128}
 
 
 def load_peaks():
