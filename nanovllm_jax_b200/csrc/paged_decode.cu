@@ -438,8 +438,13 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 }
             }
             if (!waited) {
+                // With q in flight only the first tile goes ahead of the wait: nothing can be done with it before q is here,
+                // and while the tiles behind it were walked and requested q's request waited.  us per layer of a fused step,
+                // a ring of tiles ahead -> one: one sequence of 300 tokens, 16 / 8 heads 9.0 -> 8.3, four of 100..600, 32 / 8
+                // 10.8 -> 10.2, eight of 64..1024, 16 / 8 11.7 -> 11.4, 12 of 64..2000, 5 / 1 12.0 -> 11.3, 32 of 512..2000, 32 / 8
+                // 33.2 -> 32.8, 64 of 512..8192 169.1 -> 168.8, 256 of 20..300 42.1 -> 42.3.
                 const int first_slot = __shfl_sync(0xffffffffu, slot, 0);
-                bool stop = !early || first_slot < 0 || it == (p.q_in_flight ? stages : 2 * stages);
+                bool stop = !early || first_slot < 0 || it == (p.q_in_flight ? 1u : 2 * stages);
                 if (p.slot_mapping != nullptr) {
 #pragma unroll
                     for (int i = 0; i < kEarlySlots; ++i) {
