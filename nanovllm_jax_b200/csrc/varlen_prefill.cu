@@ -156,13 +156,18 @@ __host__ __device__ __forceinline__ int min_run(int span) { return span > kTileK
 // 35, 8 / 1 heads 32.0 cut at twelve, 29.9 at eight; 20 behind 1200, 16 / 2: 27.6 / 27.6 / 19.6; 8 of 10..40 behind 900..1400, 8 / 1: 31.3 / 31.3
 // / 23.7; one prompt of 1500, 8 / 1: 34.6 / 34.6 / 28.0, of 4000, 4 / 1: 63 / 48.6 / 49.1.
 constexpr int kSplitTiles = 8;
+constexpr int kMaxSplits = 16;  // runs per item
+// A sequence without a cached prefix is cut only if it has more keys: below, whole items leave the launch short (no plan kernel, the
+// scatter in it).  One prompt of 1000, 16 / 2 heads, whole 22.3 us, cut 27.7; of 1200, 8 / 2, 25.2 / 27.5; of 1500, 5 / 1, only
+// the items of twelve tiles cut 34.9, all of eight or more 28.7.
+constexpr int kWholeKeys = 11 * kTileKV;
 // The launch has a CTA for every run that the host could foresee.  Where the device's lengths make more items than that (a
 // captured launch whose lengths were rewritten), the items stay whole and the CTAs claim them one by one.
 __device__ __forceinline__ int splits_of(const SplitParams& p, int pairs) {
     return (long long)pairs * p.per_pair * p.splits <= p.ctas ? p.splits : 1;
 }
-__device__ __forceinline__ int runs_of(const Params& p, int splits, int n_a) {
-    return n_a < kSplitTiles ? 1 : min(splits, n_a / min_run(p.pack.span));
+__device__ __forceinline__ int runs_of(const Params& p, int splits, int n_a, int prefix, int len_k) {
+    return n_a < kSplitTiles || (prefix == 0 && len_k <= kWholeKeys) ? 1 : min(splits, n_a / min_run(p.pack.span));
 }
 
 __device__ __forceinline__ Record record_of(const Params& p, int pair) {
@@ -530,7 +535,7 @@ __device__ __forceinline__ Item load_item(const Params& p, const List& l, int id
 __device__ __forceinline__ Item load_item(const SplitParams& p, const List& l, int idx) {
     const int splits = splits_of(p, l.pairs), c = idx % splits;
     Item it = load_item(static_cast<const Params&>(p), l, idx / splits);
-    const int runs = runs_of(p, splits, it.n_a);
+    const int runs = runs_of(p, splits, it.n_a, it.prefix, it.len_k);
     if (runs == 1) {
         if (c > 0) it.n_a = it.n_b = it.n_kv = 0;
         return it;
@@ -1169,32 +1174,48 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 }
 
 // Puts the runs of split items together: block (item, Q tile, group of 8 rows), thread t owns row t / 16 of the group and
-// dims 8 (t % 16) .. + 7.  Latency-bound (the partials are in L2): the maxima of all runs first, then four runs at a time.
+// dims 8 (t % 16) .. + 7.  Latency-bound (the partials are in L2): the maxima of all runs first, then eight runs at a
+// time, the ones that are not there included (a loop over the runs, unrolled by four, took the remainder one by one).
 constexpr int kCombineThreads = 128;
+constexpr int kCombineBatch = 8;
 __global__ void __launch_bounds__(kCombineThreads) prefill_combine_kernel(const __grid_constant__ SplitParams p) {
     griddep_wait();
     const int e = blockIdx.x, x = blockIdx.y, row = blockIdx.z * 8 + (threadIdx.x >> 4), c8 = (threadIdx.x & 15) * 8;
     const List list = list_of(p);
     if (e >= items_of(static_cast<const Params&>(p), list) || splits_of(p, list.pairs) == 1) return;
     const Item it = load_item(static_cast<const Params&>(p), list, e);
-    const int runs = runs_of(p, p.splits, it.n_a);
+    const int runs = runs_of(p, p.splits, it.n_a, it.prefix, it.len_k);
     const int tok = row / p.pack.heads, q_pos = it.q0 + x * p.pack.dq + tok;
     if ((x == 0 ? it.n_a : it.n_b) == 0 || runs == 1 || tok >= p.pack.tokens || q_pos >= it.len) return;
     const int head = it.head + x * p.pack.dh + row - tok * p.pack.heads;
     const float* part = p.partials + ((size_t)e * p.splits * 2 + x) * kPartialFloats;
     constexpr size_t kNext = 2 * kPartialFloats;
-    float m = -INFINITY;
-    for (int c = 0; c < runs; ++c) m = fmaxf(m, __ldcg(part + c * kNext + kTileQ * kD + row));
+    float mv[kMaxSplits], m = -INFINITY;
+#pragma unroll
+    for (int c = 0; c < kMaxSplits; ++c) mv[c] = c < runs ? __ldcg(part + c * kNext + kTileQ * kD + row) : -INFINITY;
+#pragma unroll
+    for (int c = 0; c < kMaxSplits; ++c) m = fmaxf(m, mv[c]);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, l = 0.f;
-#pragma unroll 4
-    for (int c = 0; c < runs; ++c) {
-        const float* q = part + c * kNext;
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(q + row * kD + c8));
-        const float4 b = __ldcg(reinterpret_cast<const float4*>(q + row * kD + c8) + 1);
-        const float f = fast_exp2(__ldcg(q + kTileQ * kD + row) - m);
-        l += __ldcg(q + kTileQ * kD + kTileQ + row) * f;
-        acc[0] += a.x * f, acc[1] += a.y * f, acc[2] += a.z * f, acc[3] += a.w * f;
-        acc[4] += b.x * f, acc[5] += b.y * f, acc[6] += b.z * f, acc[7] += b.w * f;
+#pragma unroll
+    for (int c0 = 0; c0 < kMaxSplits; c0 += kCombineBatch) {
+        if (c0 >= runs) break;
+        float4 a[kCombineBatch], b[kCombineBatch];
+        float lv[kCombineBatch];
+#pragma unroll
+        for (int u = 0; u < kCombineBatch; ++u) {
+            const float* q = part + (c0 + u < runs ? c0 + u : 0) * kNext;
+            a[u] = __ldcg(reinterpret_cast<const float4*>(q + row * kD + c8));
+            b[u] = __ldcg(reinterpret_cast<const float4*>(q + row * kD + c8) + 1);
+            lv[u] = __ldcg(q + kTileQ * kD + kTileQ + row);
+        }
+#pragma unroll
+        for (int u = 0; u < kCombineBatch; ++u) {
+            if (c0 + u >= runs) break;
+            const float f = fast_exp2(mv[c0 + u] - m);
+            l += lv[u] * f;
+            acc[0] += a[u].x * f, acc[1] += a[u].y * f, acc[2] += a[u].z * f, acc[3] += a[u].w * f;
+            acc[4] += b[u].x * f, acc[5] += b[u].y * f, acc[6] += b[u].z * f, acc[7] += b[u].w * f;
+        }
     }
     const float inv = 1.0f / l;
     uint4 w;
@@ -1252,7 +1273,6 @@ static int64_t item_capacity(int64_t T, int B, int span) { return T / span + B +
 static size_t list_bytes(int64_t T, int B, int span) { return ((size_t)(2 * item_capacity(T, B, span) + 1) * 16 + 255) & ~size_t(255); }
 
 // Runs per item: as many as leave one run per SM; 1 where no item can have enough tiles.
-constexpr int kMaxSplits = 16;
 static int splits_for(int64_t items, int64_t max_tiles, int sms, int span) {
     if (items <= 0 || 2 * items > sms || max_tiles < kSplitTiles) return 1;
     return (int)std::min<int64_t>(std::min<int64_t>(sms / items, kMaxSplits), max_tiles / min_run(span));
@@ -1349,11 +1369,13 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     // attention CTAs it slowed them by as much as it took (power and issue slots).
     const int64_t max_tiles = block_tables ? (int64_t)MB * block_size / kTileKV : (longest + kTileKV - 1) / kTileKV;
     const size_t lists = need;
-    const int splits = workspace_bytes >= lists + partials_bytes(sms) && ((uintptr_t)workspace & 255) == 0
+    const bool may_be_brief = cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q && B <= kShortSequences &&
+                              pairs <= kShortBlocks && pairs * p.per_pair <= sms;
+    const int splits = workspace_bytes >= lists + partials_bytes(sms) && ((uintptr_t)workspace & 255) == 0 &&
+                               (block_tables || longest > kWholeKeys)
                            ? splits_for(pairs * p.per_pair, max_tiles, sms, span)
                            : 1;
-    const bool brief = splits == 1 && cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q &&
-                       B <= kShortSequences && pairs <= kShortBlocks && pairs * p.per_pair <= sms;
+    const bool brief = splits == 1 && may_be_brief;
     if (scatter) {
         const int64_t blocks = (store_blocks_for(sc->chunks) + kThreads / kStoreThreads - 1) / (kThreads / kStoreThreads);
         if (brief && ctas + blocks <= sms) {

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 TILE, SPLIT_TILES = 128, 8
+WHOLE_KEYS = 11 * TILE  # sequences without a cached prefix are cut if they have more keys
 
 
 def make_pack(group):
@@ -29,10 +30,12 @@ def make_item(pack, length, prefix, q0, r):
     return [(head, q0, n_a), (head + pack["dh"], q0 + pack["dq"], n_b)]
 
 
-def runs(pack, tiles, splits):
+def runs(pack, tiles, splits, prefix, len_k):
     """Runs of an item (load_item of SplitParams): per run its first K/V tile and the tiles Q tiles A and B visit there."""
     n_a, n_b = tiles
-    n_kv, count = max(n_a, n_b), 1 if n_a < SPLIT_TILES else min(splits, n_a // (3 if pack["span"] > TILE else 2))
+    n_kv, count = max(n_a, n_b), 1
+    if n_a >= SPLIT_TILES and (prefix > 0 or len_k > WHOLE_KEYS):
+        count = min(splits, n_a // (3 if pack["span"] > TILE else 2))
     out = []
     for c in range(count):
         j0, j1 = n_a * c // count, n_kv if c + 1 == count else n_a * (c + 1) // count
@@ -73,7 +76,7 @@ def test_tiles_and_masks_cover_exactly_the_causal_region(length, prefix, group):
         covered = {}
         for q0 in range(0, length, pack["span"]):
             item = make_item(pack, length, prefix, q0, 0)
-            parts = runs(pack, (item[0][2], item[1][2]), splits)
+            parts = runs(pack, (item[0][2], item[1][2]), splits, prefix, prefix + length)
             for x, (head, first, n_x) in enumerate(item):
                 if n_x == 0:
                     assert first >= length
