@@ -618,7 +618,7 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
     m_run = fmaxf(m_run, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)));
     if (turn_bar != nullptr && !wait_or_abort(sh, turn_bar, turn_parity)) return false;
     if (first) {
-        m_used = m_run;  // finite: key 0 of the sequence is visible to every row and sits in the first tile
+        m_used = m_run;  // finite for live rows: key 0 of the sequence is visible to every row and sits in the first tile
     } else {
         const bool grow = (m_run - m_used) * scale_log2 > kRescaleThreshold;
         if (__any_sync(0xffffffffu, grow)) {
@@ -733,13 +733,6 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         prefetch_tensormap(&tm_q);
         prefetch_tensormap(&tm_k);
         prefetch_tensormap(&tm_v);
-    }
-    // Rows of the Q tiles that no load fills (128 is not a multiple of the packed heads): their scores must not vary, since a
-    // warp's rows vote on when to rescale.
-    for (int i = p.pack.heads * p.pack.tokens * 8 + tid; i < kTileQ * 8; i += kThreads) {
-#pragma unroll
-        for (int panel = 0; panel < 4; ++panel) *reinterpret_cast<uint4*>(sQ + panel * kPanelBytes + i * 16) = make_uint4(0, 0, 0, 0);
-        fence_proxy_async_smem();
     }
     __syncthreads();
     if (warp == 1) {
@@ -1020,7 +1013,10 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             const int first_lim = it.prefix + q_pos;      // last key visible to it
             const bool ragged = 16 * key_steps(visible_keys(p, it, x), n_x) + (n_x - 1) * kTileKV > it.len_k;
             const int live = min(p.pack.tokens, it.len - q_pos);  // tokens of the tile in front of the sequence's end
-            float m_run = -INFINITY, m_used = -INFINITY, l = 0.f;
+            // Rows behind the sequence's end (the next sequence's queries, or rows of the tile that no load fills) must not vote
+            // on when to rescale: from a maximum of +inf nothing grows, their P is 0 (NaN for scores of inf or NaN), and what
+            // O holds of them is never stored.
+            float m_run = tok < live ? -INFINITY : INFINITY, m_used = -INFINITY, l = 0.f;
             // One KV tile of this Q tile.  Tiles whose last key the tile's first row may still see need no mask; the
             // one or two after them (one when the prefix is a multiple of the tile) are masked per element.  The two
             // kinds run in two separate loops so that each loop body is straight-line code.
