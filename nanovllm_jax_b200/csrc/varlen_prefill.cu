@@ -103,8 +103,8 @@ struct Pack {
 };
 // A kv head's G q heads in one item, half of them per tile: both tiles then see the same keys and finish together.  An odd
 // number goes into both tiles, which take tokens in turn (B may see one K/V tile more).  Groups of more than eight heads are
-// cut into equal parts.
-static Pack make_pack(int G) {
+// cut into equal parts.  `lone`: items of tile A alone, twice as many (see lone_tiles).
+static Pack make_pack(int G, bool lone = false) {
     int w = std::min(G, 8);
     while (G % w) --w;
     Pack k;
@@ -114,6 +114,7 @@ static Pack make_pack(int G) {
     k.dh = w % 2 ? 0 : k.heads;
     k.span = w % 2 ? 2 * k.tokens : k.tokens;
     k.per_kv = G / w;
+    if (lone) k.dq = 1 << 28, k.dh = 0, k.span = k.tokens, k.per_kv = G / k.heads;  // no tokens behind dq: no tile B
     return k;
 }
 
@@ -1273,6 +1274,14 @@ static int splits_for(int64_t items, int64_t max_tiles, int sms, int span) {
     if (items <= 0 || 2 * items > sms || max_tiles < kSplitTiles) return 1;
     return (int)std::min<int64_t>(std::min<int64_t>(sms / items, kMaxSplits), max_tiles / min_run(span));
 }
+// Whether split items are of one Q tile, which has its SM's exponentials to itself and takes no turns, rather than of two.  They are
+// twice as many, so where the SMs do not suffice a run has more K/V tiles: worth up to three more where a tile's live rows fill more
+// than a warp, none where they do not.  60 new tokens, 32 / 8 heads, behind 3000 cached ones (two / three tiles a run) 24.0 -> 21.3 us,
+// behind 6500 (four / six) 29.5 -> 26.0, behind 12 000 (six / eleven, so still of two) 36.0, else 36.3; 16 / 8 heads there 32.7, else 35.6.
+static bool lone_tiles(int64_t max_tiles, int splits, int lone_splits, int64_t live_rows) {
+    const int more = live_rows > 32 ? 3 : 0;
+    return (max_tiles + lone_splits - 1) / lone_splits <= (max_tiles + splits - 1) / splits + more;
+}
 static size_t partials_bytes(int sms) { return (size_t)sms * 2 * kPartialFloats * 4; }
 
 // Common launcher.  kv_tokens: extent of the token axis of k / v (T for packed tensors, the slot count of the cache).
@@ -1301,17 +1310,14 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15)
         return fail(NVLLM_B200_EINVAL, "%s: q/k/v/out must be 16-byte aligned", who);
     const int G = H / KVH;
-    const Pack pack = make_pack(G);
-    const int span = pack.span;
-    const size_t need = list_bytes(T, B, span);  // the rest of what is asked for lets items be split
+    Pack pack = make_pack(G);
+    const size_t need = list_bytes(T, B, pack.span);  // the rest of what is asked for lets items be split
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15))
         return fail(NVLLM_B200_EWORKSPACE, "%s: workspace of %zu bytes required, got %zu", who, need,
                     workspace ? workspace_bytes : (size_t)0);
 
     ShortParams p;
-    // Upper bound of (sequence, token block) pairs: exact from the host copy of cu_seqlens, else from max_seqlen.
-    const int64_t cap = item_capacity(T, B, span);
-    int64_t pairs = 0, longest = max_seqlen;
+    int64_t longest = max_seqlen;
     if (cu_seqlens_host) {
         longest = 0;
         for (int b = 0; b < B; ++b) {
@@ -1321,22 +1327,46 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
             if (len > (int64_t)kMaxLevels * kTileKV)
                 return fail(NVLLM_B200_EUNSUPPORTED, "%s: sequence of %lld tokens (max %d)", who, (long long)len,
                             kMaxLevels * kTileKV);
-            pairs += (len + span - 1) / span;
             longest = std::max(longest, len);
         }
     } else {
         if (max_seqlen <= 0) return fail(NVLLM_B200_EINVAL, "%s: max_seqlen must be positive", who);
         if (max_seqlen > kMaxLevels * kTileKV)
             return fail(NVLLM_B200_EUNSUPPORTED, "%s: max_seqlen %d (max %d)", who, max_seqlen, kMaxLevels * kTileKV);
-        pairs = (int64_t)B * ((max_seqlen + span - 1) / span);
-        // The attention layer's contexts round the longest length up to 8192 at most: prompts beyond it show in T.
-        if ((int64_t)B * max_seqlen < T) pairs = cap;
     }
-    if (pairs > cap) pairs = cap;
+    // Upper bound of (sequence, token block) pairs: exact from the host copy of cu_seqlens, else from max_seqlen.
+    auto pairs_of = [&](int span) {
+        const int64_t cap = item_capacity(T, B, span);
+        int64_t n = 0;
+        if (cu_seqlens_host) {
+            for (int b = 0; b < B; ++b) n += ((int64_t)cu_seqlens_host[b + 1] - cu_seqlens_host[b] + span - 1) / span;
+        } else {
+            n = (int64_t)B * ((max_seqlen + span - 1) / span);
+            // The attention layer's contexts round the longest length up to 8192 at most: prompts beyond it show in T.
+            if ((int64_t)B * max_seqlen < T) n = cap;
+        }
+        return std::min(n, cap);
+    };
+    int64_t pairs = pairs_of(pack.span);
     if (pairs == 0) return scatter_only();
+    if (pairs * KVH * pack.per_kv > 0x7fffffffLL) return fail(NVLLM_B200_EUNSUPPORTED, "%s: grid too large", who);
+    const int sms = sm_count();
+    const int64_t max_tiles = block_tables ? (int64_t)MB * block_size / kTileKV : (longest + kTileKV - 1) / kTileKV;
+    auto splits_with = [&](const Pack& k, int64_t n) {
+        const bool room = workspace_bytes >= list_bytes(T, B, k.span) + partials_bytes(sms) && ((uintptr_t)workspace & 255) == 0;
+        return room && (block_tables || longest > kWholeKeys) ? splits_for(n * KVH * k.per_kv, max_tiles, sms, k.span) : 1;
+    };
+    int splits = splits_with(pack, pairs);
+    // Longer queries could be split without a prefix, too, and packed keys and keys in pages are to give the same bits.  With queries
+    // of at most dq tokens the items have no tile B as it is.
+    if (splits > 1 && block_tables && longest < kSplitTiles * kTileKV && longest > pack.dq) {
+        const Pack lone = make_pack(G, true);
+        const int64_t n = pairs_of(lone.span);
+        const int s = splits_with(lone, n);
+        if (s > 1 && lone_tiles(max_tiles, splits, s, longest * pack.heads)) pack = lone, pairs = n, splits = s;
+    }
     p.pack = pack;
     p.per_pair = KVH * pack.per_kv;
-    if (pairs * p.per_pair > 0x7fffffffLL) return fail(NVLLM_B200_EUNSUPPORTED, "%s: grid too large", who);
 
     int rc = ensure_attr();
     if (rc) return rc;
@@ -1357,21 +1387,13 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     p.wide = ((uintptr_t)out & 31) == 0;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.scatter = Scatter{};
-    const int sms = sm_count();
     int ctas = p.item_ctas = (int)std::min<int64_t>(pairs * p.per_pair, sms);
 
     // A short list known to the host (and nothing for the plan kernel to check on the device) needs no plan kernel, and
     // the scatter, where SMs are left, goes with the launch.  Elsewhere the scatter is a launch of its own: on a warp of the
     // attention CTAs it slowed them by as much as it took (power and issue slots).
-    const int64_t max_tiles = block_tables ? (int64_t)MB * block_size / kTileKV : (longest + kTileKV - 1) / kTileKV;
-    const size_t lists = need;
-    const bool may_be_brief = cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q && B <= kShortSequences &&
-                              pairs <= kShortBlocks && pairs * p.per_pair <= sms;
-    const int splits = workspace_bytes >= lists + partials_bytes(sms) && ((uintptr_t)workspace & 255) == 0 &&
-                               (block_tables || longest > kWholeKeys)
-                           ? splits_for(pairs * p.per_pair, max_tiles, sms, span)
-                           : 1;
-    const bool brief = splits == 1 && may_be_brief;
+    const bool brief = splits == 1 && cu_seqlens_host && !block_tables && cu_seqlens_k == cu_seqlens_q &&
+                       B <= kShortSequences && pairs <= kShortBlocks && pairs * p.per_pair <= sms;
     if (scatter) {
         const int64_t blocks = (store_blocks_for(sc->chunks) + kThreads / kStoreThreads - 1) / (kThreads / kStoreThreads);
         if (brief && ctas + blocks <= sms) {
@@ -1394,7 +1416,7 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
         cfg.gridDim = dim3(1);
         cfg.blockDim = dim3(kPlanThreads);
         NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, prefill_plan_kernel, cu_seqlens_q, cu_seqlens_k, block_tables ? 1 : 0, B,
-                                         (int4*)workspace, (int)cap, span, p.per_pair, KVH, ctas,
+                                         (int4*)workspace, (int)item_capacity(T, B, pack.span), pack.span, p.per_pair, KVH, ctas,
                                          scatter && pdl_enabled() ? 1 : 0));
     }
     cfg.gridDim = dim3((unsigned)ctas);
@@ -1403,7 +1425,7 @@ static int launch(const char* who, const void* q, const void* k, const void* v, 
     if (splits > 1) {
         SplitParams sp;
         static_cast<Params&>(sp) = p;
-        sp.partials = (float*)((uint8_t*)workspace + lists);
+        sp.partials = (float*)((uint8_t*)workspace + list_bytes(T, B, pack.span));
         sp.splits = splits;
         sp.ctas = (int)(pairs * p.per_pair * splits);
         cfg.gridDim = dim3((unsigned)sp.ctas);
@@ -1442,7 +1464,8 @@ extern "C" size_t nvllm_b200_varlen_prefill_workspace_bytes(int64_t T, int B, in
     size_t n = list_bytes(T, B, pack.span);
     // room for the partial results of split items where so few items are possible
     const int64_t blocks = std::max<int64_t>((T + pack.span - 1) / pack.span, B), per_pair = (int64_t)KVH * pack.per_kv;
-    if (2 * blocks * per_pair <= sm_count()) n += partials_bytes(sm_count());
+    if (2 * blocks * per_pair <= sm_count())
+        n = list_bytes(T, B, make_pack(H / KVH, true).span) + partials_bytes(sm_count());
     return n;
 }
 

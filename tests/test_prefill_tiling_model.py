@@ -10,10 +10,13 @@ TILE, SPLIT_TILES = 128, 8
 WHOLE_KEYS = 11 * TILE  # sequences without a cached prefix are cut if they have more keys
 
 
-def make_pack(group):
+def make_pack(group, lone=False):
+    """`lone`: items of tile A alone (no sequence has tokens as far behind a block's first as dq)."""
     w = max(x for x in range(1, 9) if group % x == 0)
     heads = w if w % 2 else w // 2
     tokens = TILE // heads
+    if lone:
+        return dict(w=heads, heads=heads, tokens=tokens, dq=1 << 28, dh=0, span=tokens, per_kv=group // heads)
     return dict(w=w, heads=heads, tokens=tokens, dq=tokens if w % 2 else 0, dh=0 if w % 2 else heads,
                 span=2 * tokens if w % 2 else tokens, per_kv=group // w)
 
@@ -66,11 +69,12 @@ def seen_keys(pack, length, prefix, q0, x, row, j0, n):
     return np.concatenate(keys)
 
 
+@pytest.mark.parametrize("lone", [False, True])
 @pytest.mark.parametrize("group", [1, 2, 3, 4, 5, 6, 7, 8, 10, 11, 16])
 @pytest.mark.parametrize("prefix", [0, 1, 127, 128, 1500, 2048])
 @pytest.mark.parametrize("length", [1, 5, 127, 128, 129, 255, 256, 257, 300, 512, 513])
-def test_tiles_and_masks_cover_exactly_the_causal_region(length, prefix, group):
-    pack = make_pack(group)
+def test_tiles_and_masks_cover_exactly_the_causal_region(length, prefix, group, lone):
+    pack = make_pack(group, lone)
     assert pack["heads"] * pack["tokens"] <= TILE
     for splits in (1, 3, 16):
         covered = {}
