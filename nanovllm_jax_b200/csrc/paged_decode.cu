@@ -89,7 +89,7 @@ struct Params {
     const int32_t* block_tables;
     const int32_t* context_lens;
     const int32_t* slot_mapping;  // [B] slots that the kernel just before this one writes, or null: it writes none
-    int q_in_flight;              // that kernel writes q too
+    int q_in_flight;              // that kernel writes q too: tiles requested ahead of the wait for it (0: it does not)
     __nv_bfloat16* out;
     float* partials;        // [chunks][KVH][2][partial_floats]
     unsigned int* tickets;  // [B*KVH] partials delivered so far per (sequence, kv head); zero when the kernel starts
@@ -438,13 +438,8 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                 }
             }
             if (!waited) {
-                // With q in flight only the first tile goes ahead of the wait: nothing can be done with it before q is here,
-                // and while the tiles behind it were walked and requested q's request waited.  us per layer of a fused step,
-                // a ring of tiles ahead -> one: one sequence of 300 tokens, 16 / 8 heads 9.0 -> 8.3, four of 100..600, 32 / 8
-                // 10.8 -> 10.2, eight of 64..1024, 16 / 8 11.7 -> 11.4, 12 of 64..2000, 5 / 1 12.0 -> 11.3, 32 of 512..2000, 32 / 8
-                // 33.2 -> 32.8, 64 of 512..8192 169.1 -> 168.8, 256 of 20..300 42.1 -> 42.3.
                 const int first_slot = __shfl_sync(0xffffffffu, slot, 0);
-                bool stop = !early || first_slot < 0 || it == (p.q_in_flight ? 1u : 2 * stages);
+                bool stop = !early || first_slot < 0 || it == (p.q_in_flight ? min((uint32_t)p.q_in_flight, stages) : 2 * stages);
                 if (p.slot_mapping != nullptr) {
 #pragma unroll
                     for (int i = 0; i < kEarlySlots; ++i) {
@@ -887,7 +882,6 @@ static int launch_decode(const char* who, const DecodeArgs& a, const StepArgs* s
     p.q = (const __nv_bfloat16*)a.q;
     p.block_tables = a.block_tables;
     p.context_lens = a.context_lens;
-    p.q_in_flight = pre != nullptr;
     p.slot_mapping = pre ? pre->slot_mapping : (step ? step->slot_mapping : nullptr);
     p.out = (__nv_bfloat16*)a.out;
     p.tickets = tickets;
@@ -900,6 +894,11 @@ static int launch_decode(const char* who, const DecodeArgs& a, const StepArgs* s
     p.block_size = a.block_size;
     p.MB = a.MB;
     p.num_groups = main_grid() / a.KVH;
+    // q is requested when the tiles ahead of the wait for it have been walked.  One tile where a chunk is part of a sequence: nothing
+    // can be done with more before q is here (12 sequences of 64..2000 tokens, 5 / 1 heads, 11.3 us per layer, a ring of tiles 12.0).
+    // A ring where a chunk holds several: their boundaries and page lookups are then behind it (96 of 20..300, 32 / 8, 22.8 us, one
+    // tile 23.4).
+    p.q_in_flight = pre == nullptr ? 0 : (a.B >= p.num_groups ? kStages : 1);
     p.item_cost = item_cost();
     p.scale_log2 = a.scale * 1.4426950408889634f;
 
