@@ -2,8 +2,6 @@
 // step that folds it into its first kernel lives in paged_decode.cu.
 #include "pre_attention.cuh"
 
-#include <mutex>
-
 namespace nvllm {
 namespace preattn {
 
@@ -31,6 +29,7 @@ struct PassSmem {  // of a warp
     float rotation[kPassStages][kD];  // of the units in flight (a unit has at least one pass)
 };
 constexpr int kPassSmemBytes = kPassThreads / 32 * (int)sizeof(PassSmem);
+static_assert(kPassSmemBytes + 2 * kD * 4 <= 48 * 1024, "more than a launch gets without asking");
 
 __device__ __forceinline__ void copy16_async(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -223,18 +222,6 @@ extern "C" int nvllm_b200_qk_norm_rope_store(void* q, void* k, const void* v, co
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(preattn::kPassThreads);
     cfg.dynamicSmemBytes = preattn::kPassSmemBytes;
-    {
-        static std::mutex mu;
-        static bool done[64];
-        int dev = 0;
-        NVLLM_CUDA_OK(cudaGetDevice(&dev));
-        std::lock_guard<std::mutex> lock(mu);
-        if (dev < 0 || dev >= 64 || !done[dev]) {
-            NVLLM_CUDA_OK(cudaFuncSetAttribute(preattn::pre_attention_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               preattn::kPassSmemBytes));
-            if (dev >= 0 && dev < 64) done[dev] = true;
-        }
-    }
     NVLLM_CUDA_OK(cudaLaunchKernelEx(&cfg, preattn::pre_attention_pass_kernel, p, passes, span));
     return NVLLM_B200_OK;
 }
