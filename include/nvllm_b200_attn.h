@@ -190,7 +190,7 @@ size_t nvllm_b200_varlen_prefill_workspace_bytes(int64_t T, int B, int H, int KV
  *                 size its grid without reading device memory.  Only that: the
  *                 lengths are the device's, so a captured call follows them when
  *                 they are rewritten between replays (B and T stay), also where
- *                 that makes more row blocks than the host copy had.  A host copy
+ *                 that makes more token blocks than the host copy had.  A host copy
  *                 without any token enqueues no attention
  *   max_seqlen    upper bound of any sequence length (used for grid sizing when
  *                 cu_seqlens_host is NULL; longer sequences are computed all the

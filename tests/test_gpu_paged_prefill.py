@@ -68,7 +68,8 @@ def _status_clean():
 @pytest.mark.parametrize("prefix", [0, 1, 255, 256, 257, 3 * 256 + 17])
 def test_prefix_lengths_with_ragged_new_lengths(prefix, h, kvh):
     """Every sequence of the batch has the same cached prefix; the new lengths straddle the 128 / 256 row tiles.
-    (8, 2): an item is 128 rows of two heads; (3, 1): the group size is odd, an item is 256 rows of one head."""
+    (8, 2): both Q tiles of an item hold two heads of its 64 tokens; (3, 1): the group size is odd, each holds all heads of 42 of its
+    84 tokens."""
     new_lens = [1, 5, 127, 128, 129, 255, 256, 257, 300, 700]
     c = _case([prefix] * len(new_lens), new_lens, h=h, kvh=kvh, block_size=256, seed=600 + prefix + h)
     assert_attention_close(torch_to_f32(_run(c)), _want(c), f"prefix {prefix} H={h} KVH={kvh}")

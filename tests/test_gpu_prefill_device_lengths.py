@@ -1,6 +1,6 @@
 """A prefill follows the lengths in the device's cu_seqlens: the host copy only sizes the grid.  A captured call is replayed
-with other lengths than it was captured with (the same number of sequences and packed tokens), among them more row blocks
-than the host copy had."""
+with other lengths than it was captured with (the same number of sequences and packed tokens), among them more token
+blocks than the host copy had."""
 import numpy as np
 import pytest
 
@@ -12,9 +12,9 @@ pytestmark = pytest.mark.gpu
 CASES = {
     "short": (8, 2, [87, 40, 0, 131], [[1, 128, 129, 0], [0, 0, 0, 258], [100, 100, 58, 0], [64, 64, 65, 65]]),
     "short, odd group": (3, 1, [300, 5], [[5, 300], [130, 129], [0, 1]]),
-    # items cut into runs (twelve K/V tiles or more); then more items than runs were foreseen, which stay whole
+    # items cut into runs (eight K/V tiles or more); then more items than runs were foreseen, which stay whole
     "split": (4, 1, [1536] + [0] * 23, [[36, 1500] + [0] * 22, [64] * 24, [0] * 23 + [1024], [100] * 14 + [0] * 10]),
-    # one row block per 128 tokens at the capture, one per sequence in the replay: several items a CTA
+    # four token blocks of 64 at the capture, eight sequences in a replay: several items a CTA
     "short, more items than CTAs": (8, 2, [256] + [0] * 7, [[32] * 8, [1, 3, 250, 2, 0, 0, 0, 0]]),
 }
 
@@ -69,7 +69,7 @@ def test_replay_follows_the_device_lengths(kind, step):
 @pytest.mark.parametrize("h,kvh,lens", [(2, 1, [9300]), (1, 1, [8200, 3]), (2, 1, [300, 8700])])
 def test_prompts_beyond_the_contexts_length_bucket(h, kvh, lens):
     """The context's max_seqlen_q ends at 8192, and without a host copy the library sizes its grid from it: prompts beyond it
-    have more row blocks than foreseen (with so few heads the launch cuts its items into runs)."""
+    have more token blocks than foreseen (with so few heads the launch cuts its items into runs)."""
     import torch
     from nanovllm_jax_b200 import _lib, workloads
     from nanovllm_jax_b200.layers.attention import Attention

@@ -1,5 +1,5 @@
 """Prefill of few items with many keys: the K/V tiles of an item are cut into runs on several CTAs and the partial results
-combined.  Around the sizes where items start to be cut (twelve K/V tiles, half as many items as SMs), with prefixes that are
+combined.  Around the sizes where items start to be cut (eight K/V tiles, half as many items as SMs), with prefixes that are
 and are not multiples of the tile, even and odd head groups, ragged ends, a sequence too short to be cut beside one that is."""
 import numpy as np
 import pytest

@@ -1,7 +1,7 @@
 """Attention.__call__ on a prefill step as one C call (nvllm_b200_prefill_step): wherever the K/V scatter runs -- CTAs of
 its own beside a short list of items, or a launch in front, with the plan kernel working beside it -- the
 caches equal the oracle's bit for bit and the output equals the attention entry points' and, at small sizes, the oracle's.
-The group sizes include odd ones (a lone head per kv head takes 256 rows at a time, the others 128 rows of two heads)."""
+The group sizes include odd ones (a Q tile holds all heads and half of an item's tokens; in the others half of the heads)."""
 import math
 
 import numpy as np

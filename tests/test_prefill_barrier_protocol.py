@@ -285,9 +285,10 @@ def run_cta(items, seed=0, jitter=0.0, empty_count=2, hand_turn_back=True, o_fir
 
 
 def item_tiles(q0, rows, prefix=0, last=None, pair_heads=False, turns=True, run=None):
-    """What make_item computes for the row block starting at row q0 with `rows` live rows of a sequence with
-    `prefix` cached tokens; `last` says whether it is the sequence's final block (default: iff the block is not full).
-    pair_heads: the item is 128 rows of two heads (both Q tiles see the same keys) instead of 256 rows of one head.
+    """What make_item computes for the token block starting at token q0 with `rows` live tokens of a sequence with
+    `prefix` cached ones; `last` says whether it is the sequence's final block (default: iff the block is not full).
+    pair_heads: both Q tiles hold the same 128 tokens (two q heads per kv head) and see the same keys; else each holds 128 of the
+    item's 256 (a single one), and tile B has nothing to do in blocks of at most 128, as in items of one tile.
     run: (c, runs): only the c-th run of its K/V tiles."""
     full = 128 if pair_heads else 256
     rows = min(rows, full)
@@ -337,7 +338,7 @@ def test_runs_of_split_items():
 def test_random_item_lists_under_random_latencies(seed):
     rng = random.Random(seed)
     items = random_items(rng, seed % 2 == 1, rng.randint(1, 14))
-    if seed % 4 == 3:  # an odd group: items of two heads and of a lone one
+    if seed % 4 == 3:  # both kinds in one list
         items += random_items(rng, False, 4)
         rng.shuffle(items)
     for jitter in (0.0, 0.4, 0.95):
