@@ -18,10 +18,8 @@ __global__ void __launch_bounds__(kThreads) pre_attention_small_kernel(const Par
 // memory.  The rows of the next pass, and with a new unit its rotation, are copied (cp.async) into the warp's part of shared
 // memory while the current one is computed: requested into registers, the rows cost sixteen of them, and a unit began with
 // the latencies of its position and of its rotation.
-// Bound by HBM: 16 384 tokens, 32 / 8 heads, 436 MB: 87.2 us with a row per four lanes and the rotation loaded for every row,
-// 81.1 with the next rows in registers, 72.8 here = 6.0 TB/s; 8192 tokens, 64 / 8: 68.2 -> 60.6; 30 000, 28 / 4: 120.7 -> 103.2.
-// One pass ahead is enough and more is slower: two ahead 81.5 us, three 82.4 (reads and writes of the DRAM in each other's
-// way); 12 warps per SM 84.5, 24 (spills) 99.7; bulk copies through shared memory 142.
+// Bound by HBM: 16 384 tokens, 32 / 8 heads, 445 MB: 81.1 us with the next rows in registers, 73.4 here = 6.1 TB/s.  One pass ahead is
+// enough: with two (81.5 us) reads and writes of the DRAM are in each other's way.
 constexpr int kPassThreads = 256;
 constexpr int kPassStages = 2;  // the pass that is computed and the next one
 struct PassSmem {  // of a warp
@@ -194,12 +192,10 @@ extern "C" int nvllm_b200_qk_norm_rope_store(void* q, void* k, const void* v, co
     cfg.stream = reinterpret_cast<cudaStream_t>(stream);
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    // The pass kernel pays where its passes are full and every resident warp (two CTAs per SM) gets 4.5 of them or more, or eight
-    // with passes three quarters full (but not where that is a token's only pass, which loads a rotation every time).  us,
-    // small kernel / this one, 2368 warps: 32 / 8 heads (full), 4.1 passes a warp 9.0 / 9.8, 4.4 10.9 / 10.6, 5.1 12.7 / 11.5, 8.1
-    // 20.4 / 17.9; 6 / 1, 6.9 20.5 / 18.1; 28 / 4 (0.9), 4.6 9.4 / 8.9; 18 / 2 (0.92), 6.3 15.6 / 14.4; 10 / 2 (0.88), 4.2
-    // 9.2 / 11.4, 13.8 31.6 / 28.6; 12 / 4 (0.83), 5.1 11.1 / 11.5, 7.6 17.4 / 17.0; 14 / 2 (0.75), 5.0 8.7 / 10.6, 20.8 39.4 / 35.0;
-    // one pass a token: 5 / 1 (0.88), 6.9 18.2 / 19.3, 4 / 1 (0.75), 8.4 18.8 / 22.8; 8 / 1 (0.62), 16.9 28.4 / 32.1.
+    // The pass kernel pays where its passes are full and every resident warp (two CTAs per SM) gets 4.5 of them or more (32 / 8 heads,
+    // small kernel / this one: 4.1 passes a warp 9.0 / 9.8 us, 5.1 12.7 / 11.5), or eight with passes three quarters full (12 / 4:
+    // 5.1 11.1 / 11.5, 7.6 17.4 / 17.0), but not where that is a token's only pass, which loads a rotation every time (4 / 1: 8.4
+    // 18.8 / 22.8).
     const int passes = (H + 2 * KVH + 7) / 8;
     const int64_t ctas = 2 * (int64_t)sm_count(), warps = ctas * (preattn::kPassThreads / 32);
     const int rows = H + 2 * KVH, room = 8 * passes;

@@ -18,14 +18,13 @@
 // together), and the kv heads go in groups whose keys and values fit the L2 (head_groups).  Tensor memory and
 // barriers are set up once per CTA; the loads of the next item are already in flight
 // while the current one drains.  Where the host knows that there is at most one item per SM, every CTA finds its own from
-// cu_seqlens instead (ShortParams), and the step's K/V scatter runs on the SMs the items leave.  Few items with many keys are cut into runs of
-// K/V tiles (SplitParams) that a small kernel behind this one combines.
+// cu_seqlens instead (ShortParams), and the step's K/V scatter runs on the SMs the items leave.  Few items with many keys are cut
+// into runs of K/V tiles (SplitParams), of tile A alone where SMs would idle otherwise (lone_tiles), that a small kernel behind this
+// one combines.
 //
 // Rows that are (token, head) pairs leave fewer of them behind the sequences' ends than rows of 128 tokens of one head, and
-// tiles that span few tokens cut the products short at the diagonal.  us per call, before -> after:
-// 48 prompts of 5..300 tokens, 10 / 2 heads, 35.0 -> 28.4; 30 of 65..192, 64 / 8, 64.0 -> 46.7; 32 of 300, 32 / 8, 86.8 -> 74.1;
-// 12 of 17..700 behind 500..5000 cached ones, 32 / 8, 257 -> 238; 16 of 128..4096, 32 / 8, 880 -> 869; one of 8192, 64 / 8,
-// 1059.5 -> 1059.5.
+// tiles that span few tokens cut the products short at the diagonal: 30 prompts of 65..192 tokens, 64 / 8 heads, 64.0 -> 46.7 us,
+// 16 of 128..4096, 32 / 8, 880 -> 869.
 //
 // Per CTA (12 warps = 3 warpgroups; the first gives registers away with setmaxnreg, the softmax
 // warpgroups take them):
@@ -48,7 +47,8 @@
 //               releases four P.V k-steps) and rescales O only when the max grew by more
 //               than 2^8 (exact: the stale max is carried into the final normalisation).
 //               Tiles strictly above the diagonal are skipped; of a diagonal tile each warp
-//               masks the one chunk of 32 keys that its rows' limits fall into and skips the chunks behind it.  The exponentials of the two tiles take turns
+//               masks the one chunk of 32 keys that its rows' limits fall into and skips
+//               the chunks behind it.  The exponentials of the two tiles take turns
 //               (A(0) B(0) A(1) ...): they share the four MUFU pipes, which bound the
 //               kernel, and alternating keeps one tile's MMAs, score loads and row max
 //               running under the other tile's exponentials.
@@ -152,15 +152,12 @@ constexpr int kPartialFloats = kTileQ * kD + 2 * kTileQ;  // O[128][128] relativ
 // but one (two where the item has more tokens than a tile keys).
 __host__ __device__ __forceinline__ int min_run(int span) { return span > kTileKV ? 3 : 2; }
 // Items of fewer tiles stay whole: they take less time than the partial results and the combining launch (about 6 us).  The
-// rule looks at an item's own tiles, so that packed keys and keys in pages give the same bits.  us per call, whole / cut at
-// twelve tiles into runs of four / at eight into runs of two: 100 new tokens behind 8000 cached ones, 32 / 8 heads, 130 / 35 /
-// 35, 8 / 1 heads 32.0 cut at twelve, 29.9 at eight; 20 behind 1200, 16 / 2: 27.6 / 27.6 / 19.6; 8 of 10..40 behind 900..1400, 8 / 1: 31.3 / 31.3
-// / 23.7; one prompt of 1500, 8 / 1: 34.6 / 34.6 / 28.0, of 4000, 4 / 1: 63 / 48.6 / 49.1.
+// rule looks at an item's own tiles, so that packed keys and keys in pages give the same bits.  20 new tokens behind 1200 cached
+// ones, 16 / 2 heads: whole 27.6 us, cut 19.6; 100 behind 8000, 32 / 8: 130 and 35.
 constexpr int kSplitTiles = 8;
 constexpr int kMaxSplits = 16;  // runs per item
 // A sequence without a cached prefix is cut only if it has more keys: below, whole items leave the launch short (no plan kernel, the
-// scatter in it).  One prompt of 1000, 16 / 2 heads, whole 22.3 us, cut 27.7; of 1200, 8 / 2, 25.2 / 27.5; of 1500, 5 / 1, only
-// the items of twelve tiles cut 34.9, all of eight or more 28.7.
+// scatter in it).  One prompt of 1200, 8 / 2 heads, whole 25.2 us, cut 27.5; of 1500, 8 / 1, whole 34.6, cut 28.0.
 constexpr int kWholeKeys = 11 * kTileKV;
 // The launch has a CTA for every run that the host could foresee.  Where the device's lengths make more items than that (a
 // captured launch whose lengths were rewritten), the items stay whole and the CTAs claim them one by one.
@@ -334,10 +331,8 @@ constexpr uint32_t kIdescPV = kIdesc | ((128u >> 3) << 17) | (1u << 16);  // B o
 // ------------------------------------------------------------------------------------------
 // Longest spans first means that all sequences are in flight at once.  Where their keys and values do not fit the L2 the kv
 // heads are taken in groups whose keys and values do, one group after the other, as long as each is long enough for its CTAs to
-// end together.  Together with the streams' eviction hints (Q and the output are touched once), us per call: 16 prompts of
-// 128..4096 tokens, 32 / 8 heads (139 MB of K and V): 931 as one group, 912 with the hints, 880 in two, 884 in four, 916 in
-// eight (4 rounds of items each); 32 of 500..2000, 16 / 8 (164 MB): 398, 384, 366, 367, 386; 8 of 1000..8000, 40 / 8: 2190,
-// 2160, 2104, 2117, 2106; 12 of 17..700 behind 500..5000 cached ones (4 rounds of items in all): 260, 258, 271 in two.
+// end together.  16 prompts of 128..4096 tokens, 32 / 8 heads (139 MB of K and V): 912 us as one group, 880 in two, 916 in eight (four
+// rounds of items each); 12 of 17..700 behind 500..5000 cached ones (four rounds in all): 258, in two 271.
 constexpr long long kGroupRows = (96 << 20) / 512;  // (token, kv head) rows of K and V: 512 bytes
 constexpr int kGroupRounds = 6;                     // items per CTA and group
 __device__ int head_groups(long long keys, int pairs, int per_pair, int KVH, int ctas) {
@@ -405,7 +400,7 @@ __global__ void __launch_bounds__(kPlanThreads) prefill_plan_kernel(const int32_
         for (int l = l0; l < n; l += dl) atomicAdd(&hist[level_of(len, len_k, l, span)], 1);
     }
     // One update per warp (a 64-bit atomic of shared memory and a load latency per sequence cost 100 sequences of 10..100 tokens
-    // 2.1 us of 43.3, 48 of 5..300 1.1 of 29.9).
+    // 2.1 us of 43.3).
     my_level = __reduce_max_sync(0xffffffffu, my_level);
     my_keys = __reduce_add_sync(0xffffffffu, my_keys);
     if ((threadIdx.x & 31) == 0) {
@@ -573,6 +568,9 @@ __device__ __forceinline__ int kv_tile_token(const Params& p, const Item& it, in
     return page * p.block_size + off % p.block_size;  // block_size is a multiple of the tile: a tile never straddles pages
 }
 
+// The output is marked as evicted first, so that it does not push keys and values out of the L2 (16 prompts of 128..4096 tokens, 32 / 8
+// heads, with Q's loads marked too: 931 -> 912 us as one head group).  The GEMM that reads it next does not notice: attention and an
+// o_proj-shaped GEMM together, outputs of 4 to 268 MB, take 0 to 0.4 % less with the mark.
 __device__ __forceinline__ void store_32bytes(void* dst, const uint32_t (&w)[8]) {
     asm volatile("st.global.L1::no_allocate.L2::evict_first.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]),
                  "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
@@ -1007,8 +1005,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             }
             // The two tiles take turns, unless tile A has a single K/V tile: then nothing of A could run under B's
             // exponentials, and B's wait is not won back (64 prompts of 20..128 tokens, 32 / 8 heads: 47.9 us without turns,
-            // 51.3 with).  With two the turns pay: 16 prompts of 256 tokens 35.7 us without, 34.4 with; five of 390..472, 64 / 8
-            // heads, 47.5 and 46.0; 48 of 5..300, 10 / 2 heads, 33.5 and 33.8.
+            // 51.3 with).  With two the turns pay (16 prompts of 256 tokens: 35.7 us without, 34.4 with).
             const bool both = it.n_b > 0 && it.n_a > 1;
             const int q_pos = it.q0 + x * p.pack.dq;      // first token of this Q tile
             const int first_lim = it.prefix + q_pos;      // last key visible to it
