@@ -579,15 +579,17 @@ __device__ __forceinline__ void store_32bytes(void* dst, const uint32_t (&w)[8])
 
 // One 128-column S row -> running max, optional O rescale, bf16 P in two halves.  DIAG: key column c of this tile is
 // visible iff c <= lim (lim may be negative -- nothing visible in this tile -- or >= 127), and the limits of the warp's rows
-// lie in warp_lo .. warp_hi; columns behind every limit may hold anything.  turn_bar (or null): the
-// other tile's hand-over this tile's exponentials wait for; turn_out (or null): where this tile hands over.
+// lie in warp_lo .. warp_hi; columns behind every limit may hold anything.  alive: the warp's rows in front of the
+// sequence's end; the others (the next sequence's queries, rows that no load fills) have no vote on when to rescale, or the
+// live rows' bits would depend on them.  turn_bar (or null): the other tile's hand-over this tile's exponentials wait for;
+// turn_out (or null): where this tile hands over.
 // The whole row is held in registers (the softmax warpgroups raise their register budget with setmaxnreg), so
 // tensor memory is read once and its latency is paid once per tile.
 template <bool DIAG>
 __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint32_t t_s, const uint32_t t_o,
                                              const int lim, const int warp_lo, const int warp_hi, const bool first,
                                              const uint32_t o_parity_prev,
-                                             const float scale_log2, float& m_run, float& m_used, float& l,
+                                             const float scale_log2, const uint32_t alive, float& m_run, float& m_used, float& l,
                                              uint64_t* turn_bar, const uint32_t turn_parity, uint64_t* turn_out) {
     uint32_t v[4][32];
     tmem_ld32(t_s, v[0]);
@@ -620,7 +622,7 @@ __device__ __forceinline__ bool softmax_tile(Shared* sh, const int x, const uint
         m_used = m_run;  // finite for live rows: key 0 of the sequence is visible to every row and sits in the first tile
     } else {
         const bool grow = (m_run - m_used) * scale_log2 > kRescaleThreshold;
-        if (__any_sync(0xffffffffu, grow)) {
+        if (__ballot_sync(0xffffffffu, grow) & alive) {
             // O holds sums relative to m_used: bring it to m_run before this tile's P.V is added.
             if (!wait_or_abort(sh, &sh->o_full[x], o_parity_prev)) return false;
             tc_fence_after();
@@ -1011,10 +1013,8 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             const int first_lim = it.prefix + q_pos;      // last key visible to it
             const bool ragged = 16 * key_steps(visible_keys(p, it, x), n_x) + (n_x - 1) * kTileKV > it.len_k;
             const int live = min(p.pack.tokens, it.len - q_pos);  // tokens of the tile in front of the sequence's end
-            // Rows behind the sequence's end (the next sequence's queries, or rows of the tile that no load fills) must not vote
-            // on when to rescale: from a maximum of +inf nothing grows, their P is 0 (NaN for scores of inf or NaN), and what
-            // O holds of them is never stored.
-            float m_run = tok < live ? -INFINITY : INFINITY, m_used = -INFINITY, l = 0.f;
+            float m_run = -INFINITY, m_used = -INFINITY, l = 0.f;
+            const uint32_t alive = __ballot_sync(0xffffffffu, tok < live);
             // One KV tile of this Q tile.  Tiles whose last key the tile's first row may still see need no mask; the
             // one or two after them (one when the prefix is a multiple of the tile) are masked per element.  The two
             // kinds run in two separate loops so that each loop body is straight-line code.
@@ -1069,7 +1069,7 @@ varlen_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                 const int lim = first_lim - j * kTileKV;
                 if (!softmax_tile<kDiag>(sh, x, t_s, t_o, kDiag ? lim + min(tok, live - 1) : 0, kDiag ? lim + min(tok_lo, live - 1) : 0,
                                          kDiag ? lim + min(tok_hi, live - 1) : 0, j == 0,
-                                         (tiles - 1) & 1u, p.scale_log2, m_run, m_used, l, turn_bar, turn_parity,
+                                         (tiles - 1) & 1u, p.scale_log2, alive, m_run, m_used, l, turn_bar, turn_parity,
                                          (both && (x == 0 || j < it.n_a)) ? &sh->turn[x] : nullptr))
                     return false;
                 // the turn is handed over by A after each of its tiles, by B after those that followed one of A's
